@@ -147,7 +147,9 @@ def _service(case):
                 old["stream"].close()
             old["index"].close()
         n = case["rows"]
-        centers = _centers(case["dim"], 256 if n > 1_000_000 else 64)
+        # (tables searched through a graph: clusters of about 2000 rows, so that
+        # no row is a hub whose surplus links the builder keeps in any order)
+        centers = _centers(case["dim"], max(64, n // 2000) if graph else 256 if n > 1_000_000 else 64)
         rows = _mixture(_gen(datagen.SEED + 1), centers, n, case["values"])
         rng = np.random.default_rng(datagen.SEED + 3)
         cols = np.stack([rng.integers(0, 10, n).astype(np.float64),
