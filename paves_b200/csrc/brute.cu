@@ -76,6 +76,11 @@ int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &
         }
         db.one_range = ok;
     }
+    // many range-form programs: the position form (up to eight take one turn
+    // of the general kernel, which has no tables to make first)
+    db.rank_ok = P >= PV_RANK_MIN_PROGS && P <= PV_RANK_MAX_PROGS && rank_batch_ok(g, pb);
+    if (db.rank_ok)
+        PV_CUDA_OK(g->scan.rank_tab.ensure(rank_tab_bytes(P)), errbuf, errlen);
     // sparse route: one filter shared by the whole batch whose matches are
     // bounded by a small count (the scan then reads only those rows)
     db.sparse_bound = 0;
@@ -100,6 +105,51 @@ int brute_upload(FvGpuIndex *g, DevBatch &db, char *errbuf, size_t errlen) {
     return 0;
 }
 
+int brute_bitmaps(FvGpuIndex *g, const DevBatch &db, char *errbuf, size_t errlen) {
+    char *d = db.stage_d->as<char>();
+    const PredProg *d_progs = (const PredProg *)(d + db.off_progs);
+    const PredInsn *d_insns = (const PredInsn *)(d + db.off_insns);
+    const double *d_consts = (const double *)(d + db.off_consts);
+    const int *d_counts = (const int *)(d + db.off_counts);
+    const uint64_t bm_words = (g->count + 31) / 32;
+    const int P = db.P;
+    ScanScratch &s = g->scan;
+    PV_CUDA_OK(s.bitmaps.ensure((size_t)P * bm_words * 4), errbuf, errlen);
+    PV_CUDA_OK(s.popcnt.ensure((size_t)P * 8), errbuf, errlen);
+    uint32_t *bm = s.bitmaps.as<uint32_t>();
+    unsigned long long *pop = s.popcnt.as<unsigned long long>();
+    if (db.counts_on_device) {
+        // one launch shape for any batch: the staged counts give each of the
+        // two forms its programs, and the other finds none
+        g->launches++;
+        PV_CUDA_OK(launch_bitmaps_capped(g->d_cols, g->count, d_insns, d_progs, d_consts,
+                                         d_counts, P, db.ninsns, db.nconsts, bm, bm_words, pop,
+                                         g->sm_count, g->stream, g->ncols),
+                   errbuf, errlen);
+        if (!g->rank_cols || P > PV_RANK_MAX_PROGS) return 0;
+        PV_CUDA_OK(s.rank_tab.ensure(rank_tab_bytes(P)), errbuf, errlen);
+        g->launches += 3;
+        PV_CUDA_OK(launch_bitmaps_rank(g, d_insns, d_progs, d_consts, P, d_counts + 4,
+                                       s.rank_tab.p, bm, bm_words, pop, g->stream),
+                   errbuf, errlen);
+        return 0;
+    }
+    if (db.rank_ok) {
+        PV_CUDA_OK(s.rank_tab.ensure(rank_tab_bytes(P)), errbuf, errlen);
+        g->launches += 3;
+        PV_CUDA_OK(launch_bitmaps_rank(g, d_insns, d_progs, d_consts, P, nullptr, s.rank_tab.p,
+                                       bm, bm_words, pop, g->stream),
+                   errbuf, errlen);
+        return 0;
+    }
+    g->launches++;
+    PV_CUDA_OK(launch_bitmaps(g->d_cols, g->count, d_insns, d_progs, d_consts, P, bm, bm_words,
+                              pop, g->sm_count, g->stream, db.ninsns, db.nconsts, g->ncols,
+                              db.one_range),
+               errbuf, errlen);
+    return 0;
+}
+
 // Device-side work of one batch: inputs already resident in db.stage_d.
 int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_out,
                  uint32_t *d_cnt, uint8_t *d_trunc, char *errbuf, size_t errlen,
@@ -117,25 +167,8 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     if (ev) cudaEventRecord(ev[0], g->stream);
     if (bitmaps_ready) {
         // the caller launched the bitmaps of this batch
-    } else if (db.counts_on_device && P > 0) {
-        PV_CUDA_OK(s.bitmaps.ensure((size_t)P * bm_words * 4), errbuf, errlen);
-        PV_CUDA_OK(s.popcnt.ensure((size_t)P * 8), errbuf, errlen);
-        g->launches++;
-        PV_CUDA_OK(launch_bitmaps_capped(g->d_cols, g->count, d_insns, d_progs, d_consts,
-                                         (const int *)(d + db.off_counts), P, db.ninsns,
-                                         db.nconsts, s.bitmaps.as<uint32_t>(), bm_words,
-                                         s.popcnt.as<unsigned long long>(), g->sm_count,
-                                         g->stream, g->ncols),
-                   errbuf, errlen);
     } else if (P > 0) {
-        PV_CUDA_OK(s.bitmaps.ensure((size_t)P * bm_words * 4), errbuf, errlen);
-        PV_CUDA_OK(s.popcnt.ensure((size_t)P * 8), errbuf, errlen);
-        g->launches++;
-        PV_CUDA_OK(launch_bitmaps(g->d_cols, g->count, d_insns, d_progs, d_consts, P,
-                                  s.bitmaps.as<uint32_t>(), bm_words,
-                                  s.popcnt.as<unsigned long long>(), g->sm_count, g->stream,
-                                  db.ninsns, db.nconsts, g->ncols, db.one_range),
-                   errbuf, errlen);
+        if (brute_bitmaps(g, db, errbuf, errlen)) return -1;
     } else {
         PV_CUDA_OK(s.popcnt.ensure(8), errbuf, errlen);
     }

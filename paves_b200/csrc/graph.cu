@@ -662,21 +662,11 @@ int graph_run_host(FvGpuIndex *g, int nq, const float *queries, const uint32_t *
     memcpy(db.stage_h->as<char>() + off_ent, entries, (size_t)nq * 4);
     if (brute_upload(g, db, errbuf, errlen)) return -1;
     char *d = db.stage_d->as<char>();
-    const uint64_t bm_words = (g->count + 31) / 32;
     ScanScratch &s = g->scan;
     const int P = db.P;
     cudaEventRecord(g->ev0, g->stream);
     if (P > 0) {
-        PV_CUDA_OK(s.bitmaps.ensure((size_t)P * bm_words * 4), errbuf, errlen);
-        PV_CUDA_OK(s.popcnt.ensure((size_t)P * 8), errbuf, errlen);
-        g->launches++;
-        PV_CUDA_OK(launch_bitmaps(g->d_cols, g->count, (const PredInsn *)(d + db.off_insns),
-                                  (const PredProg *)(d + db.off_progs),
-                                  (const double *)(d + db.off_consts), P,
-                                  s.bitmaps.as<uint32_t>(), bm_words,
-                                  s.popcnt.as<unsigned long long>(), g->sm_count, g->stream,
-                                  db.ninsns, db.nconsts, g->ncols, db.one_range),
-                   errbuf, errlen);
+        if (brute_bitmaps(g, db, errbuf, errlen)) return -1;
     }
     const GraphOut lo = graph_out_layout(nq, ef);
     const size_t off_cnt = lo.off_cnt, off_exh = lo.off_exh, off_st = lo.off_st;

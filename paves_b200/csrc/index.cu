@@ -212,6 +212,9 @@ extern "C" void fv_gpu_index_free(FvGpuIndex *g) {
         cudaFree(g->d_vecs);
         cudaFree(g->d_cols);
         cudaFree(g->d_prows);
+        cudaFree(g->d_rank);
+        cudaFree(g->d_code);
+        cudaFree(g->d_sorted);
         cudaFree(g->d_adj);
         cudaFree(g->d_deg);
         cudaFree(g->d_vlow);
@@ -220,6 +223,7 @@ extern "C" void fv_gpu_index_free(FvGpuIndex *g) {
         cudaFree(g->d_norm32);
     }
     Buf *bufs[] = {&g->scan.stage_h, &g->scan.stage_d, &g->scan.bitmaps, &g->scan.popcnt,
+                   &g->scan.rank_tab,
                    &g->scan.tau, &g->scan.part, &g->scan.part_cnt, &g->scan.cand,
                    &g->scan.out_d, &g->scan.out_h, &g->scan.sparse, &g->graph.visited, &g->graph.res,
                    &g->graph.stats, &g->graph.route, &g->graph.route_h, &g->graph.gout};
@@ -325,6 +329,7 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         if ((e = cudaMemcpyAsync(g->d_prows, post_rows, count * (size_t)ncols * 4,
                                  cudaMemcpyHostToDevice, g->stream)) != cudaSuccess)
             return bail("postings copy", e);
+        if ((e = pv::build_rank_cols(g)) != cudaSuccess) return bail("column positions", e);
         pv::build_sorted_cols(g, cols, post_rows);
     }
 
@@ -498,6 +503,12 @@ FvGpuIndex *index_view(const FvGpuIndex *g) {
     v->d_vecs = g->d_vecs;
     v->d_cols = g->d_cols;
     v->d_prows = g->d_prows;
+    v->d_rank = g->d_rank;
+    v->d_code = g->d_code;
+    v->d_sorted = g->d_sorted;
+    memcpy(v->rank_nv, g->rank_nv, sizeof(v->rank_nv));
+    v->rank_cols = g->rank_cols;
+    v->code_cols = g->code_cols;
     v->d_adj = g->d_adj;
     v->d_deg = g->d_deg;
     v->deg_cap = g->deg_cap;

@@ -38,6 +38,8 @@ struct Buf {
     template <typename T> T *as() const { return (T *)p; }
 };
 
+constexpr int PV_RANK_COLS = 4;
+
 // Host-compiled predicates of one batch (see pred.cpp).
 struct PredBatch {
     std::vector<PredInsn> insns;
@@ -53,6 +55,7 @@ struct ScanScratch {
     Buf stage_d;         // device copy of the packed inputs
     Buf bitmaps;         // [P][bm_words] u32
     Buf popcnt;          // [P] u64
+    Buf rank_tab;        // [P] programs as position intervals (bitmap_rank.cu)
     Buf tau;             // [nq] u64
     Buf part;            // [nq][grow][K] u64 keys
     Buf part_cnt;        // [nq][grow] u32
@@ -86,6 +89,15 @@ struct FvGpuIndex {
     float *d_vecs = nullptr; // [count][dpad] exact rows (always resident)
     double *d_cols = nullptr;     // [ncols][count]
     uint32_t *d_prows = nullptr;  // [ncols][count]
+    // filters as positions in a column's value order (bitmap_rank.cu; tables
+    // of at most PV_RANK_COLS columns): per row its position and the code of
+    // its small integer, per column the values in order and how many are
+    // numbers; rank_cols / code_cols: the columns each serves
+    uint32_t *d_rank = nullptr;   // [ncols][count]
+    uint8_t *d_code = nullptr;    // [ncols][count]
+    double *d_sorted = nullptr;   // [ncols][count]
+    uint32_t rank_nv[pv::PV_RANK_COLS] = {};
+    int rank_cols = 0, code_cols = 0;
 
     // level-0 graph as fixed-degree device adjacency ("device CSR"):
     // d_adj[node*deg_cap + i], padded with UINT32_MAX; d_deg[node]

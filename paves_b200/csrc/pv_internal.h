@@ -31,6 +31,17 @@ cudaError_t launch_bitmaps_capped(const double *cols, uint64_t nrows, const Pred
                                   unsigned long long *popcnt, int sm_count, cudaStream_t st,
                                   int ncols = 1 << 30);
 
+// many range-form programs at once (bitmap_rank.cu)
+constexpr int PV_RANK_MIN_PROGS = 9;
+constexpr int PV_RANK_MAX_PROGS = 1024;  // its tables of four columns fit a block
+size_t rank_tab_bytes(int P);
+cudaError_t build_rank_cols(FvGpuIndex *g);
+bool rank_batch_ok(const FvGpuIndex *g, const PredBatch &pb);
+cudaError_t launch_bitmaps_rank(const FvGpuIndex *g, const PredInsn *insns, const PredProg *progs,
+                                const double *consts, int P, const int *dP, void *tab,
+                                uint32_t *bitmaps, uint64_t bm_words, unsigned long long *popcnt,
+                                cudaStream_t st);
+
 // ---- per-query top-KO of dense key runs (scan_tc.cu): keys of query q are
 // dense[q][0 .. dcnt[q]) (<= dcap), at most the bound tau[q] (tau null: no
 // bound); KO <= 1024. Writes out [nq][KO] ascending, out_cnt, trunc (from
@@ -105,11 +116,16 @@ struct DevBatch {
     // one program in range form whose terms are all well formed (constants
     // in the pool, columns in the table): the lean bitmap kernel
     bool one_range = false;
+    // many programs, all of the form bitmap_rank.cu takes
+    bool rank_ok = false;
 };
 
 int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &pb,
                   DevBatch &db, size_t extra_bytes, char *errbuf, size_t errlen);
 int brute_upload(FvGpuIndex *g, DevBatch &db, char *errbuf, size_t errlen);
+// The bitmaps and counts of a staged batch's db.P > 0 programs into g->scan,
+// by the kernel its programs allow.
+int brute_bitmaps(FvGpuIndex *g, const DevBatch &db, char *errbuf, size_t errlen);
 // ev (optional): 5 events recorded before bitmaps, before scan, after scan,
 // after re-rank and after merge. bm_done (with bitmaps_ready: the caller's
 // bitmap kernel is the last launch on the stream): recorded once the

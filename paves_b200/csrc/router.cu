@@ -589,18 +589,11 @@ extern "C" int pv_router_features(PvRouter *r, FvGpuIndex *g, int nq, const floa
     }
     if (brute_upload(g, db, errbuf, errlen)) return -1;
     char *d = db.stage_d->as<char>();
-    const uint64_t bm_words = (g->count + 31) / 32;
     ScanScratch &s = g->scan;
     const int P = db.P;
     RT_OK(s.popcnt.ensure((size_t)(P > 0 ? P : 1) * 8));
     if (P > 0) {
-        RT_OK(s.bitmaps.ensure((size_t)P * bm_words * 4));
-        g->launches++;
-        RT_OK(launch_bitmaps(g->d_cols, g->count, (const PredInsn *)(d + db.off_insns),
-                             (const PredProg *)(d + db.off_progs),
-                             (const double *)(d + db.off_consts), P, s.bitmaps.as<uint32_t>(),
-                             bm_words, s.popcnt.as<unsigned long long>(), g->sm_count, g->stream,
-                             db.ninsns, db.nconsts, g->ncols, db.one_range));
+        if (brute_bitmaps(g, db, errbuf, errlen)) return -1;
     }
     const size_t fbytes = (size_t)nq * NI * 4;
     RT_OK(s.out_d.ensure(fbytes));
@@ -1121,12 +1114,7 @@ extern "C" int pv_routed_batch(FvGpuIndex *g, PvRouter *r, int nq, const float *
                              side>>>((const float *)(d + db.off_q), nq, g->dpad, r->d_cent,
                                      r->ncent, dpart);
     if (P > 0) {
-        g->launches++;
-        RT_OK(launch_bitmaps(g->d_cols, g->count, (const PredInsn *)(d + db.off_insns),
-                             (const PredProg *)(d + db.off_progs),
-                             (const double *)(d + db.off_consts), P, s.bitmaps.as<uint32_t>(),
-                             bm_words, s.popcnt.as<unsigned long long>(), g->sm_count, g->stream,
-                             db.ninsns, db.nconsts, g->ncols, db.one_range));
+        if (brute_bitmaps(g, db, errbuf, errlen)) return -1;
     }
     // Speculative scan on the main stream meanwhile: a scan costs about the
     // same for one query as for the batch and is exact, so it runs unless

@@ -91,7 +91,7 @@ void layout(Bucket &b, const FvGpuIndex *g) {
     db.off_insns = db.off_progs + al((size_t)B * sizeof(PredProg) + 8);
     db.off_consts = db.off_insns + al((size_t)b.insn_cap * sizeof(PredInsn));
     db.off_counts = db.off_consts + al((size_t)b.const_cap * 8);
-    db.off_extra = db.off_counts + al(16);
+    db.off_extra = db.off_counts + al(32);
     db.bytes = db.off_extra;
     db.stage_h = &b.stage_h;
     db.stage_d = &b.stage_d;
@@ -141,7 +141,11 @@ int stage(Bucket &b, const FvGpuIndex *g, int nq, const float *queries, const Pr
                                   pb.consts.data()) >= PV_LAZY_MIN_PASS;
     }
     int32_t *cnt = (int32_t *)(h + b.db.off_counts);
-    cnt[0] = lazy ? 0 : P;
+    // all programs in the position form: the rank kernels take them (cnt[4]),
+    // else the general one does (cnt[0])
+    const bool rank = !lazy && P >= PV_RANK_MIN_PROGS && b.db.P <= PV_RANK_MAX_PROGS && rank_batch_ok(g, pb);
+    cnt[0] = lazy || rank ? 0 : P;
+    cnt[4] = rank ? P : 0;
     cnt[1] = (int)pb.insns.size();
     cnt[2] = (int)pb.consts.size();
     cnt[3] = lazy ? 1 : 0;
