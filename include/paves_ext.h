@@ -31,6 +31,10 @@ int pv_pred_check(int nq, const FvGpuQueryDesc *qd, const FvGpuPredNode *nodes, 
                   const int32_t *children, int nchildren, const double *invals, int ninvals,
                   int ncols, int *nprog, char *errbuf, size_t errlen);
 
+/* Largest |v| of n host values when every one is an integer of magnitude at
+ * most 256 (rows whose BF16 distances can be certified exact), else -1. */
+float pv_rows_integral_amax(const float *v, uint64_t n);
+
 typedef struct PvBatch PvBatch;
 
 /* Compiles the batch's predicates and copies queries + predicate programs

@@ -144,20 +144,6 @@ static int pick_device(size_t need) {
 
 }  // namespace pv
 
-// Largest |value| of an array if every value is an integer of magnitude
-// <= 256 (exactly representable in bf16), else -1.
-float pv_integral_amax(const float *v, uint64_t n) {
-    float amax = 0.f;
-    for (uint64_t i = 0; i < n; i++) {
-        const float x = v[i];
-        if (x != floorf(x)) return -1.f;
-        const float a = fabsf(x);
-        if (a > amax) amax = a;
-        if (amax > 256.f) return -1.f;
-    }
-    return amax;
-}
-
 // True when bf16 tensor-core distances are exact for rows with integral
 // max row_amax and queries with integral max q_amax: the norm form's
 // largest intermediate, ||x||^2 + ||q||^2 <= dim * (row_amax^2 + q_amax^2),

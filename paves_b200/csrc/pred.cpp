@@ -7,6 +7,7 @@
 // re-serialized in post-order with n-ary AND/OR folded into binary steps so
 // the device evaluates it with a 64-bit bit stack. Identical predicates in a
 // batch share one program (and therefore one bitmap).
+#include <immintrin.h>
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -440,3 +441,46 @@ int compile_predicates(int nq, const int32_t *proot, size_t proot_stride,
 }
 
 }  // namespace pv
+
+// Largest |value| of an array if every value is an integer of magnitude
+// <= 256 (exactly representable in bf16), else -1. Eight values at a time,
+// with one test per block (3.7 ms for 7.7M values on one core; a test per
+// value took 24 ms): a value that is its own floor is an integer (NaN is
+// not), and magnitudes compare as their bits.
+float pv_integral_amax(const float *v, uint64_t n) {
+    constexpr uint64_t BLOCK = 4096;
+    uint32_t top = 0;
+    for (uint64_t b = 0; b < n; b += BLOCK) {
+        const uint64_t e = b + BLOCK < n ? b + BLOCK : n;
+        uint32_t bad = 0, m = 0;
+        uint64_t i = b;
+        __m256 vbad = _mm256_setzero_ps();
+        __m256i vm = _mm256_setzero_si256();
+        for (; i + 8 <= e; i += 8) {
+            const __m256 x = _mm256_loadu_ps(v + i);
+            vbad = _mm256_or_ps(vbad, _mm256_cmp_ps(x, _mm256_floor_ps(x), _CMP_NEQ_UQ));
+            vm = _mm256_max_epu32(vm, _mm256_and_si256(_mm256_castps_si256(x),
+                                                       _mm256_set1_epi32(0x7FFFFFFF)));
+        }
+        alignas(32) uint32_t lane[8];
+        _mm256_store_si256((__m256i *)lane, vm);
+        for (uint32_t u : lane) m = u > m ? u : m;
+        bad = (uint32_t)_mm256_movemask_ps(vbad);
+        for (; i < e; i++) {
+            uint32_t u;
+            memcpy(&u, v + i, 4);
+            u &= 0x7FFFFFFFu;
+            m = u > m ? u : m;
+            bad |= (uint32_t)(v[i] != floorf(v[i]));
+        }
+        top = m > top ? m : top;
+        if (bad || top > 0x43800000u) return -1.f;  // 256.f
+    }
+    float amax;
+    memcpy(&amax, &top, 4);
+    return amax;
+}
+
+extern "C" float pv_rows_integral_amax(const float *v, uint64_t n) {
+    return v ? pv_integral_amax(v, n) : -1.f;
+}

@@ -33,7 +33,7 @@ class Hnsw:
         err = C.create_string_buffer(256)
         if builder == "gpu":
             v = self.vectors
-            integral = bool(np.all(np.abs(v) <= 256.0) and np.array_equal(v, np.rint(v)))
+            integral = L.pv_rows_integral_amax(ptr(v), v.size) >= 0.0
             prec = _lib.FV_GPU_PREC_BF16 if integral else _lib.FV_GPU_PREC_FP32
             cand = candidates or min(1023, 4 * M - 1)
             h = L.pv_hnsw_build_gpu(ptr(v), n, d, M, cand, device, prec, err, 256)
