@@ -269,7 +269,6 @@ pserve_kernel(const __grid_constant__ CUtensorMap tmX, SvArgs p) {
             sa.tile_step = pl.seed_step;
             sa.tiles_per_cta = pl.seed_tiles;
             sa.KP = pl.seed_kwrite;
-            sa.kwrite = pl.seed_kwrite;
             sa.push_tau = pl.seed_kwrite == pl.S ? 1 : 0;
             sa.fullmin = nullptr;
             // shared memory the merges wrote is refilled by TMA (async proxy)
@@ -299,7 +298,6 @@ pserve_kernel(const __grid_constant__ CUtensorMap tmX, SvArgs p) {
         a.tile_step = 1;
         a.tiles_per_cta = pl.tpc;
         a.KP = pl.KP;
-        a.kwrite = pl.KP;
         a.push_tau = pl.push_tau;
         a.fullmin = pl.certify ? p.fullmin : nullptr;
         fence_proxy_async();

@@ -46,13 +46,15 @@ cudaError_t launch_bitmaps_rank(const FvGpuIndex *g, const PredInsn *insns, cons
 // dense[q][0 .. dcnt[q]) (<= dcap), at most the bound tau[q] (tau null: no
 // bound); KO <= 1024. Writes out [nq][KO] ascending, out_cnt, trunc (from
 // popcnt[qprog[q]] or nrows), tau_out[q] = min(tau_out[q], KO-th key) and
-// unc[q] (a full list's last key, fullmin[q], at or below the answer's end).
+// unc[q] (a full list's last key, fullmin[q], at or below the answer's end;
+// or, with an estimated bound, KO > 32, fewer than KO keys at or below it).
 cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *dcnt,
                                bool reset_cnt, const unsigned long long *fullmin,
                                const unsigned long long *tau, int KO, const int32_t *qprog,
                                const unsigned long long *popcnt, uint64_t nrows, int nq,
                                FvHit *out, uint32_t *out_cnt, uint8_t *trunc,
-                               unsigned long long *tau_out, uint8_t *unc, cudaStream_t st);
+                               unsigned long long *tau_out, uint8_t *unc, cudaStream_t st,
+                               bool estimated = false);
 
 // ---- exact FP32 scan (scan_f32.cu)
 struct ScanF32Args {

@@ -30,6 +30,8 @@
 // warp shrinks by the replication factor and all four SM sub-partitions
 // work (without it the warps of the padding lanes idle).
 // All waits are bounded by a deadline and unwind through an abort flag.
+#include <math.h>
+
 #include <algorithm>
 
 #include <cuda.h>
@@ -53,7 +55,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte alignment for the swizzled operand tiles
     unsigned char *base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const TcSmem sm = tc_carve(base, a.kblocks, a.NS, a.KP, EPI, KIND != TCK_TF32);
+    const TcSmem sm = tc_carve(base, a.kblocks, a.NS, a.KP, EPI);
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int warp = threadIdx.x >> 5;
@@ -149,12 +151,13 @@ dense_merge_kernel(const uint64_t *__restrict__ dense, uint64_t dcap, int stage_
                    const unsigned long long *__restrict__ popcnt, uint64_t nrows,
                    FvHit *__restrict__ out, uint32_t *__restrict__ out_cnt,
                    uint8_t *__restrict__ trunc, unsigned long long *tau_out,
-                   uint8_t *__restrict__ unc) {
+                   uint8_t *__restrict__ unc, int estimated) {
     extern __shared__ __align__(16) unsigned char dm_smem[];
     pdl_wait();
     pdl_trigger();
     dense_merge_query(blockIdx.x, (uint64_t *)dm_smem, dense, dcap, stage_cap, dcnt, reset_cnt,
-                      fullmin, tau, KO, qprog, popcnt, nrows, out, out_cnt, trunc, tau_out, unc);
+                      fullmin, tau, KO, qprog, popcnt, nrows, out, out_cnt, trunc, tau_out, unc,
+                      estimated != 0);
 }
 
 __global__ void __launch_bounds__(DM_THREADS)
@@ -185,7 +188,8 @@ cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *d
                                const unsigned long long *tau, int KO, const int32_t *qprog,
                                const unsigned long long *popcnt, uint64_t nrows, int nq,
                                FvHit *out, uint32_t *out_cnt, uint8_t *trunc,
-                               unsigned long long *tau_out, uint8_t *unc, cudaStream_t st) {
+                               unsigned long long *tau_out, uint8_t *unc, cudaStream_t st,
+                               bool estimated) {
     if (KO < 1 || KO > DM_OUT) return cudaErrorInvalidValue;
     if (KO <= 32) {
         return launch_pdl(dense_top32_kernel, dim3(nq), dim3(DM_THREADS), 0, st, dense, dcap,
@@ -199,7 +203,7 @@ cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *d
     if (e != cudaSuccess) return e;
     return launch_pdl(dense_merge_kernel, dim3(nq), dim3(DM_THREADS), smem, st, dense, dcap,
                       stage_cap, dcnt, reset_cnt ? 1 : 0, fullmin, tau, KO, qprog, popcnt, nrows,
-                      out, out_cnt, trunc, tau_out, unc);
+                      out, out_cnt, trunc, tau_out, unc, estimated ? 1 : 0);
 }
 
 // ---------------------------------------------------------------- host side
@@ -272,15 +276,15 @@ bool tc_supported(const FvGpuIndex *g) {
     return row_bytes <= 512;  // query tile <= 64 KB of shared memory
 }
 
-static size_t tc_smem(int kblocks, int NS, int KP, int EPI, bool staged = true) {
-    return tc_smem_bytes(kblocks, NS, KP, EPI, staged);
+static size_t tc_smem(int kblocks, int NS, int KP, int EPI) {
+    return tc_smem_bytes(kblocks, NS, KP, EPI);
 }
 
 bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns) {
     if (!tc_supported(g) || epi < 1 || epi > 3 || ns < 2 || ns > TC_MAX_STAGES) return false;
     const int S = tc_superset(g, topb, -1.f);
     if (!S) return false;
-    const int KP = S < TC_MAX_LIST ? S : TC_MAX_LIST;
+    const int KP = std::min(S, tc_list_cap(epi));
     const int esz = g->precision == FV_GPU_PREC_FP8 ? 1 : 2;
     return tc_smem(g->kpad * esz / TC_KB_BYTES, ns, KP, epi) <= 227 * 1024;
 }
@@ -321,18 +325,30 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const int kelems = tf32 ? ((g->dpad + 31) & ~31) : g->kpad;
     const int kblocks = kelems * esz / TC_KB_BYTES;
     const int S = tf32 ? tf32_superset(g, topb, q_amax) : tc_superset(g, topb, q_amax);
-    const int KP = S < TC_MAX_LIST ? S : TC_MAX_LIST;
     g->last_superset = S;
     g->tc_unc = nullptr;
     if (!S || !(tf32 ? tf32_supported(g) : tc_supported(g)) || (rs && lz)) {
         snprintf(errbuf, errlen, "gpu: tensor-core scan not available for this batch");
         return -1;
     }
-    // epilogue warp groups (each owning every EPI-th tile): two when the
-    // lists fit with at least two pipeline stages, else one (three groups
-    // measured no faster at batch 64: 0.0654 vs 0.0643 ms; pv_tc_shape can
-    // ask for them). The automatic shape stays within smem_pref, which
-    // leaves each SM a few KB for a small kernel beside the scan (the
+    const int qtiles = (nq + TC_BM - 1) / TC_BM;
+    const int nqpad = qtiles * TC_BM;
+    // query replicas: as many as the batch leaves room for, while each
+    // part of a tile keeps at least 32 rows (one TMEM load)
+    int R = 1;
+    if (g->tune_rep > 0) R = g->tune_rep;
+    else if (qtiles == 1) R = nq <= 32 ? 4 : nq <= 64 ? 2 : 1;
+    while (R > 1 && (TC_BM / R < nq || TC_BN / R < 32)) R >>= 1;
+    const int bq = TC_BM / R;
+    // epilogue warp groups (each owning every EPI-th tile): three where every
+    // warp has 128 rows of a tile to go through (more than 64 queries: 0.227
+    // against 0.237 ms for 512 over 1M BF16 rows, 0.55 against 0.72 ms for
+    // 512 over 2M FP8 rows with supersets of 400), else two (with 64 queries
+    // three run the same: 0.0615 ms), one where a tile's rows take longer to
+    // arrive than one group to look through (16 queries over BF16 rows, 64
+    // over f32 rows: the same pass, half the lists to merge, 0.088 against
+    // 0.094 ms in all) or the lists do not fit with two. The automatic shape stays within smem_pref,
+    // which leaves each SM a few KB for a small kernel beside the scan (the
     // router's, a merge launched early).
     const size_t smem_cap = 227 * 1024;
     const size_t smem_pref = 222 * 1024;
@@ -340,11 +356,11 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const int ns0 = std::min(TC_MAX_STAGES, std::max(
         2, (int)(128 * 1024 / ((size_t)std::min(kblocks, TC_KBS) * TC_BOX))));
     int EPI = 0, NS = 0;
-    for (int e = 2; e >= 1 && !EPI; e--) {
-        const int nmin = e == 3 ? 3 : 2;
+    for (int e = kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 ? 3 : 2; e >= 1 && !EPI; e--) {
+        const int KPe = std::min(S, tc_list_cap(e));
         int n = ns0;
-        while (n > nmin && tc_smem(kblocks, n, KP, e, !tf32) > smem_pref) n--;
-        if (n >= nmin && tc_smem(kblocks, n, KP, e, !tf32) <= smem_pref) {
+        while (n > 2 && tc_smem(kblocks, n, KPe, e) > smem_pref) n--;
+        if (tc_smem(kblocks, n, KPe, e) <= smem_pref) {
             EPI = e;
             NS = n;
         }
@@ -356,21 +372,13 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     if (g->tune_epi || g->tune_ns) {  // a tuned shape, if it fits
         const int e = g->tune_epi ? g->tune_epi : EPI, n = g->tune_ns ? g->tune_ns : NS;
         if (e >= 1 && e <= 3 && n >= 2 && n <= TC_MAX_STAGES &&
-            tc_smem(kblocks, n, KP, e, !tf32) <= smem_cap) {
+            tc_smem(kblocks, n, std::min(S, tc_list_cap(e)), e) <= smem_cap) {
             EPI = e;
             NS = n;
         }
     }
-    const size_t smem = tc_smem(kblocks, NS, KP, EPI, !tf32);
-    const int qtiles = (nq + TC_BM - 1) / TC_BM;
-    const int nqpad = qtiles * TC_BM;
-    // query replicas: as many as the batch leaves room for, while each
-    // part of a tile keeps at least 32 rows (one TMEM load)
-    int R = 1;
-    if (g->tune_rep > 0) R = g->tune_rep;
-    else if (qtiles == 1) R = nq <= 32 ? 4 : nq <= 64 ? 2 : 1;
-    while (R > 1 && (TC_BM / R < nq || TC_BN / R < 32)) R >>= 1;
-    const int bq = TC_BM / R;
+    const int KP = std::min(S, tc_list_cap(EPI));
+    const size_t smem = tc_smem(kblocks, NS, KP, EPI);
     // rows scanned: the index's, or a compacted set
     const uint64_t nrows_scan = rs ? rs->nrows : g->count;
     const uint64_t ntiles_all = (nrows_scan + TC_BN - 1) / TC_BN;
@@ -490,7 +498,6 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     a.dense = s.part.as<uint64_t>();
     a.dcnt = d_dcnt;
     a.dcap = dcap;
-    a.kwrite = KP;
     a.fullmin = certify ? d_fullmin : nullptr;
     a.err = d_err;
     a.timeout_ns = g->tc_timeout_ns ? g->tc_timeout_ns : 2000000000ull;
@@ -522,40 +529,46 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     FvHit *cand = (FvHit *)(c + off_cand);
     uint32_t *ccnt = (uint32_t *)(c + off_ccnt);
     // Seeding pass: a few tiles per CTA from an evenly strided sample; the
-    // merged K'-th key of the sample bounds the K'-th key of the whole
-    // scan, so the main pass admits only rows that can still matter.
+    // rank-th key of the sample bounds the S-th key of the whole scan, so the
+    // main pass admits only rows that can still matter.
     const bool seed = g->tune_seed == 2 ? false : ntiles_all >= 8 * (uint64_t)grow;
+    bool estimated = false;
     if (seed) {
         TcArgs sa = a;
-        // larger supersets take a larger sample (up to 8 tiles per CTA,
-        // spread over the CTA's own range), so the bound stays near the
-        // S-th key and the final merge's survivors fit one pass
+        // Tiles per CTA, spread over its own range: a tile more costs the
+        // sample one tile's time, and a list of the main pass admits about
+        // S * tpc / (m * grow) rows; the sum is least near sqrt(S tpc / grow)
+        // times a constant measured at 1 (batch 512, 128 and 64 of 1M rows:
+        // half and twice as many tiles are both slower or the same).
         const uint64_t region = ntiles_all / grow;
-        const uint64_t m = std::min<uint64_t>(std::min<uint64_t>(8, region),
-                                              std::max<uint64_t>(1, ((uint64_t)S + 15) / 16));
+        const double best = sqrt((double)S * tpc / grow);
+        const uint64_t m = std::min<uint64_t>(region, best < 1.0 ? 1 : best > 8.0 ? 8 : (uint64_t)best);
         sa.tile0_mul = region;
         sa.tile_step = std::max<uint64_t>(1, region / m);
         sa.tiles_per_cta = m;
-        // only each list's best keys: the S-th key of a subset of the
-        // sample still bounds the S-th key of the scan, and a short run
-        // keeps the merge cheap (the radix select of S > 32 reads its run
-        // 8 times). The sample's S best keys are spread over many lists
-        // (S / nlists per list on average): 4S keys in all, at least one
-        // per list, never more than the main pass's list length (its
-        // shared memory). One key per list when that suffices measured
-        // 3.5 µs less before the main pass than two (batch 64, S = 10,
-        // 592 lists: heaps of one, half the seeding merge's keys), for a
-        // bound barely looser (the main pass ran the same).
-        sa.kwrite = std::min(KP, std::max(1, (4 * S + nlists - 1) / std::max(1, nlists)));
-        // lists need hold no more than that (short heaps admit fewer rows);
-        // a full list's last key bounds the S-th key only if it holds S
-        sa.KP = sa.kwrite;
+        // The sample's S-th key is a bound for certain, but with large
+        // supersets it admits S / share rows, far more than S. A sample
+        // holding `share` of the rows has S * share of the S best in
+        // expectation, with a Poisson spread: its key six deviations above
+        // that lies beyond the S-th key of the scan but for about one query
+        // in 10^9, and the merge sees such a query (fewer than S keys got
+        // through), which is then re-run exactly. Only where the merge
+        // certifies anyway (lists shorter than the superset).
+        const double share = std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan);
+        const int rank_est = (int)ceil(S * share + 6.0 * sqrt(S * share) + 8.0);
+        estimated = certify && rank_est < S;
+        const int rank = estimated ? rank_est : S;
+        // lists need hold no more than their share of 4 rank keys, at least
+        // one (short lists admit fewer rows, and the merge reads fewer keys);
+        // never more than the main pass's length (its shared memory). A full
+        // list's last key bounds the S-th key only if it holds S.
+        sa.KP = std::min(KP, std::max(1, (4 * rank + nlists - 1) / std::max(1, nlists)));
         sa.push_tau = sa.KP == S ? 1 : 0;
         sa.fullmin = nullptr;
         g->launches += 2;  // seeding pass + its merge
         PV_CUDA_OK(run(sa, true), errbuf, errlen);
         // the merge leaves the counts at zero for the main pass
-        PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, true, nullptr, a.tau, S, d_qprog,
+        PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, true, nullptr, a.tau, rank, d_qprog,
                                       popcnt, g->count, nq, cand, ccnt,
                                       (uint8_t *)(c + off_ctr), a.tau, nullptr, g->stream),
                    errbuf, errlen);
@@ -578,12 +591,13 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         g->launches--;
         PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, false, a.fullmin, a.tau, S,
                                       d_qprog, popcnt, g->count, nq, d_out, d_cnt, d_trunc,
-                                      nullptr, d_unc, g->stream),
+                                      nullptr, d_unc, g->stream, estimated),
                    errbuf, errlen);
     } else {
         PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, false, a.fullmin, a.tau, S,
                                       d_qprog, popcnt, g->count, nq, cand, ccnt,
-                                      (uint8_t *)(c + off_ctr), nullptr, d_unc, g->stream),
+                                      (uint8_t *)(c + off_ctr), nullptr, d_unc, g->stream,
+                                      estimated),
                    errbuf, errlen);
         RerankCert cert;
         if (num_cert) {

@@ -255,7 +255,7 @@ int autotune(PvStream *s, const float *tq, int ntq, char *errbuf, size_t errlen)
         if (v->precision != FV_GPU_PREC_FP32 && tc_supported(v)) {
             const int qtiles = (b->B + 127) / 128;
             const int g1 = std::max(1, v->sm_count / qtiles);
-            for (int epi : {1, 2})
+            for (int epi : {1, 2, 3})
                 for (int ns : {2, 3, 4, 6, 8})
                     if (tc_shape_fits(v, b->topb, epi, ns))
                         for (int grow : {g1, std::max(1, g1 / 2)})

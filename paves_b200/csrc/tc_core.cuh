@@ -42,6 +42,8 @@ constexpr int TC_KBS = 2;           // K-blocks per pipeline stage
 // certifies per query (queries it cannot certify are re-run exactly).
 constexpr int TC_MAX_SUPERSET = 1024;
 constexpr int TC_MAX_LIST = 64;
+constexpr int TC_MAX_LIST3 = 48;   // with three epilogue groups (their shared memory)
+inline int tc_list_cap(int epi) { return epi == 3 ? TC_MAX_LIST3 : TC_MAX_LIST; }
 constexpr int TC_MAX_STAGES = 8;   // TMA pipeline stages at most
 constexpr int TC_NR = 8;            // tiles of row norms in flight (shared-memory ring)
 // words per norm slot: norms, fp8 scales, then the index rows of a
@@ -108,12 +110,12 @@ struct TcArgs {
     const uint32_t *__restrict__ rowids;
     const unsigned long long *nrows_dev;
     unsigned long long *tau;  // [nq] grid-wide bound
-    // kept keys: each list appends its best kwrite keys to its query's dense
-    // run dense[q][0 .. dcnt[q]) (any order; dcap >= lists per query * kwrite)
+    // kept keys: each list appends its keys at or below the bound to its
+    // query's dense run dense[q][0 .. dcnt[q]) (any order; dcap >= lists per
+    // query * KP)
     uint64_t *dense;
     uint32_t *dcnt;
     uint64_t dcap;
-    int kwrite;
     // [nq] smallest last key of a full list (the merge's certificate), or null
     unsigned long long *fullmin;
     int *err;
@@ -134,26 +136,22 @@ struct TcSmem {
     unsigned char *sQ, *sX;
     size_t SB;  // bytes per pipeline stage
     uint64_t *lists;
-    float *stage, *snorm;
+    float *snorm;
     uint64_t *full, *empty, *tfull, *tempty, *qbar, *done, *nfull, *nempty;
 };
 
-// staged: the candidate staging slots exist (every kind but TF32, whose
-// admissions re-read the accumulator registers; its 32-32 KB go to stages)
 __device__ __forceinline__ TcSmem tc_carve(unsigned char *base, int KBt, int NS, int KPcap,
-                                           int EPI, bool staged = true) {
+                                           int EPI) {
     TcSmem m;
     m.sQ = base;                                       // KBt boxes
     m.sX = m.sQ + (size_t)KBt * TC_BOX;                // NS stages
     // a stage holds one K-chunk of a row tile: min(TC_KBS, KBt) boxes
     m.SB = (size_t)(KBt < TC_KBS ? KBt : TC_KBS) * TC_BOX;
-    // per (query, part) lists [KP][128*EPI] and candidate staging [32][128*EPI]
+    // per (query, part) lists [KP][128*EPI]
     m.lists = (uint64_t *)(m.sX + (size_t)NS * m.SB);
-    m.stage = (float *)(m.lists + (size_t)TC_BM * EPI * KPcap);
     // row norms (and fp8 scales, compacted-set row ids) of a tile, TC_NR
     // tiles in flight (slot = [norms 128][scales 128][row ids 128])
-    m.snorm = m.stage + (staged ? 32 * TC_BM * EPI : 0);
-    if (!staged) m.stage = nullptr;
+    m.snorm = (float *)(m.lists + (size_t)TC_BM * EPI * KPcap);
     uint64_t *bars = (uint64_t *)(m.snorm + (size_t)TC_NR * TC_NSLOT_F);
     m.full = bars;              // [NS]
     m.empty = m.full + NS;      // [NS]
@@ -166,11 +164,10 @@ __device__ __forceinline__ TcSmem tc_carve(unsigned char *base, int KBt, int NS,
     return m;
 }
 
-inline size_t tc_smem_bytes(int kblocks, int NS, int KPcap, int EPI, bool staged = true) {
+inline size_t tc_smem_bytes(int kblocks, int NS, int KPcap, int EPI) {
     return 1024 + (size_t)kblocks * TC_BOX +
            (size_t)NS * (kblocks < TC_KBS ? kblocks : TC_KBS) * TC_BOX +
-           (size_t)TC_BM * EPI * KPcap * 8 + (staged ? (size_t)32 * TC_BM * EPI * 4 : 0) +
-           (size_t)TC_NR * TC_NSLOT_F * 4 + (size_t)(2 * NS + 2 * TC_NACC + 2 + 2 * TC_NR) * 8;
+           (size_t)TC_BM * EPI * KPcap * 8 + (size_t)TC_NR * TC_NSLOT_F * 4 + (size_t)(2 * NS + 2 * TC_NACC + 2 + 2 * TC_NR) * 8;
 }
 
 // by one thread, before the CTA's first pass
@@ -181,7 +178,7 @@ __device__ __forceinline__ void tc_init_barriers(const TcSmem &m, int NS, int EP
     }
     for (int i = 0; i < TC_NACC; i++) {
         mbar_init(&m.tfull[i], 1);
-        mbar_init(&m.tempty[i], TC_BM);  // the epilogue group that owns the tile
+        mbar_init(&m.tempty[i], 4);  // one arrival per warp of the owning group
     }
     for (int i = 0; i < TC_NR; i++) {
         mbar_init(&m.nfull[i], 1);
@@ -222,7 +219,6 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
     unsigned char *sX = sm.sX;
     const size_t SB = sm.SB;
     uint64_t *lists = sm.lists;
-    float *stage = sm.stage;
     float *snorm = sm.snorm;
     uint64_t *full = sm.full, *empty = sm.empty, *tfull = sm.tfull, *tempty = sm.tempty;
     uint64_t *qbar = sm.qbar, *done = sm.done, *nfull = sm.nfull, *nempty = sm.nempty;
@@ -358,7 +354,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
         // tile's fixed costs (barrier waits, word loads, arrivals) once per
         // EPI tiles, and takes the CW rows of its replica from each of them.
         constexpr int CPH = TC_BN / 32;      // 32-row chunks per part at most
-        constexpr int NSLOT = TC_BM * EPI;   // list / stage slots
+        constexpr int NSLOT = TC_BM * EPI;   // list slots
         const int qd = warp & 3;
         const int half = (warp - 2) >> 2;
         const int m = qd * 32 + lane;        // TMEM lane = query slot of the tile
@@ -375,54 +371,43 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
         const bool lazy = a.lazy && *a.lazy;
         const uint32_t *bm = (pg >= 0 && !lazy) ? a.bitmaps + (uint64_t)pg * a.bm_words : nullptr;
         // lazy: the query's range program (AND of per-column intervals and
-        // small-integer sets, the encoding of common.cuh) in registers
-        int nterm = 0;
-        int tcol[PV_RANGE_MAX_TERMS];
-        double tlo[PV_RANGE_MAX_TERMS], thi[PV_RANGE_MAX_TERMS];
+        // small-integer sets, the encoding of common.cuh), its place only:
+        // the few rows tested read its constants again (cached), instead of
+        // 20 registers held through the hot loop of every batch
+        int nterm = 0, term0 = 0;
         if (lazy && pg >= 0) {
-            const PredProg pp = a.progs[pg];
-            const PredInsn r = a.insns[pp.insn0];
-            int ci = r.val0;
+            const PredInsn r = a.insns[a.progs[pg].insn0];
             nterm = min(max(r.n, 0), PV_RANGE_MAX_TERMS);
-#pragma unroll
-            for (int k = 0; k < PV_RANGE_MAX_TERMS; k++) {
-                tcol[k] = -1;  // a malformed term admits nothing
-                tlo[k] = 1.0;
-                thi[k] = 0.0;
-                if (k >= nterm || ci < 0 || ci + 2 > a.nconsts) continue;
-                const int meta = (int)a.consts[ci];
-                const int col = meta & 0xFFFF;
-                const bool mask = meta & PV_TERM_MASK;
-                if (col < a.ncols && (mask || ci + 3 <= a.nconsts)) {
-                    tcol[k] = col | (mask ? PV_TERM_MASK : 0);
-                    tlo[k] = a.consts[ci + 1];  // a mask term: its bits
-                    thi[k] = mask ? 0.0 : a.consts[ci + 2];
-                }
-                ci += mask ? 2 : 3;
-            }
+            term0 = r.val0;
         }
         // the range program on row `row`: f64 compares, NaN fails (the
-        // bitmap kernel's test of the same encoding)
+        // bitmap kernel's test of the same encoding); a malformed term
+        // admits nothing
         auto lazy_pass = [&](uint64_t row) -> bool {
-            bool ok = true;
-#pragma unroll
-            for (int k = 0; k < PV_RANGE_MAX_TERMS; k++) {
-                if (k >= nterm) break;
-                if (tcol[k] < 0) return false;
-                const int col = tcol[k] & 0xFFFF;
+            int ci = term0;
+#pragma unroll 1
+            for (int k = 0; k < nterm; k++) {
+                if (ci < 0 || ci + 2 > a.nconsts) return false;
+                const int meta = (int)__ldg(a.consts + ci);
+                const int col = meta & 0xFFFF;
+                const bool mask = meta & PV_TERM_MASK;
+                if (col >= a.ncols || (!mask && ci + 3 > a.nconsts)) return false;
                 const double v = __ldg(a.cols + (uint64_t)col * a.nrows + row);
-                if (tcol[k] & PV_TERM_MASK) {
+                if (mask) {
                     const bool in = v >= 0.0 && v < 64.0;
                     const int b = in ? (int)v : 64;
                     const int code = (in && (double)b == v) ? b : 64;
                     const unsigned long long bits =
-                        (unsigned long long)__double_as_longlong(tlo[k]);
-                    ok = ok && code < 64 && ((bits >> (code & 63)) & 1ull);
+                        (unsigned long long)__double_as_longlong(__ldg(a.consts + ci + 1));
+                    if (!(code < 64 && ((bits >> (code & 63)) & 1ull))) return false;
+                    ci += 2;
                 } else {
-                    ok = ok && v >= tlo[k] && v <= thi[k];
+                    if (!(v >= __ldg(a.consts + ci + 1) && v <= __ldg(a.consts + ci + 2)))
+                        return false;
+                    ci += 3;
                 }
             }
-            return ok;
+            return true;
         };
         // thread-private list, interleaved [KP][NSLOT] so a warp's accesses to
         // the same slot index hit 32 different banks
@@ -434,10 +419,8 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
         uint64_t thr = qvalid ? KEY_MAX : 0ull;  // admission threshold
         float thr_d = qvalid ? __int_as_float(0x7f800000) : -1.f;  // its distance
         bool ok = true;
-        // per-tile words in registers, loaded one tile ahead into the set the
-        // previous tile released (two sets, no register moves: a move would
-        // wait for the load): predicate words of the 32-row chunks and the
-        // grid-wide bound
+        // per-tile words in registers, loaded one tile ahead: predicate words
+        // of the 32-row chunks and the grid-wide bound
         auto load_words = [&](uint64_t tt, uint32_t (&w)[CPH], unsigned long long &g) {
             const uint64_t rb = (tile0 + tt * a.tile_step) * TC_BN + col0;
 #pragma unroll
@@ -445,7 +428,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                 if (j >= nch) break;
                 const uint64_t r0 = rb + j * 32;
                 uint32_t v = 0;
-                if (r0 < a.nrows) {
+                if (qvalid && r0 < a.nrows) {
                     v = bm ? __ldg(bm + (r0 >> 5)) : 0xFFFFFFFFu;
                     if (a.nrows - r0 < 32) v &= (1u << (a.nrows - r0)) - 1u;
                 }
@@ -453,17 +436,30 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
             }
             g = qvalid ? *((volatile unsigned long long *)(a.tau + qg)) : KEY_MAX;
         };
-        // one tile: false when a wait gave up
-        auto tile_body = [&](uint64_t t, const uint32_t (&bw)[CPH], unsigned long long gt,
-                             uint32_t (&nbw)[CPH], unsigned long long &ngt) -> bool {
+        uint32_t bw[CPH] = {};
+        unsigned long long gt = KEY_MAX;
+        // this group's first tile of the pass
+        const uint64_t tfirst = (uint64_t)((half - (int)(T0 % EPI) + EPI) % EPI);
+        if (tfirst < ntiles) load_words(tfirst, bw, gt);
+        // (one copy of the tile's code: with a copy for each of two word sets
+        // the warps waited for instructions, 18 % of their stalls)
+#pragma unroll 1
+        for (uint64_t t = tfirst; t < ntiles; t += EPI) {
+            uint32_t nbw[CPH] = {};
+            unsigned long long ngt = KEY_MAX;
             if (t + EPI < ntiles) load_words(t + EPI, nbw, ngt);
             const uint64_t T = T0 + t;  // running tile count: barrier phases
             const int acc = (int)(T % TC_NACC);
             const uint32_t aph = (uint32_t)((T / TC_NACC) & 1);
             const int ns = (int)(T % TC_NR);
-            if (!mbar_wait(&tfull[acc], aph, deadline, abort_flag)) return false;
-            if (!mbar_wait(&nfull[ns], (uint32_t)((T / TC_NR) & 1), deadline, abort_flag))
-                return false;
+            // (the lanes leave together: what follows reads TMEM by the warp)
+            const bool ready =
+                mbar_wait(&tfull[acc], aph, deadline, abort_flag) &&
+                mbar_wait(&nfull[ns], (uint32_t)((T / TC_NR) & 1), deadline, abort_flag);
+            if (!__all_sync(0xffffffffu, ready)) {
+                ok = false;
+                break;
+            }
             tc_fence_after();
             const bool tr =
                 a.trace && blockIdx.x == 0 && slot == 0 && t < (uint64_t)a.trace_tiles;
@@ -476,59 +472,97 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                 thr = gt;
                 thr_d = key_dist(gt);
             }
-            // one 32-row chunk of the tile, its accumulator columns in r
-            auto chunk = [&](const int c, const uint32_t(&r)[32]) {
-                // hot loop: distances and a candidate mask only; the rare
-                // admissions run below, outside the unrolled code (a negative
-                // norm-form value is clamped there). They take a candidate's
-                // distance from the staging slots, or, in a TF32 pass, again
-                // from the accumulator registers (the same operations on the
-                // same values: the same bits), whose freed shared memory
-                // holds a third stage of its 512-byte rows: measured at batch
-                // 64 the TF32 pass ran 0.098 vs 0.102 ms; the BF16 pass the
-                // same way ran 0.069 vs 0.064 ms (its accumulators stay live
-                // through the admissions: 144 registers instead of 128, and
-                // more stages did not help it)
-                constexpr bool RECOMP = KIND == TCK_TF32;
-                auto dist_of = [&](const int i, const uint32_t acc_bits) -> float {
-                    float dot = __uint_as_float(acc_bits);
-                    if (FP8) dot *= xsv[c * 32 + i] * qs;
-                    return fmaf(-2.f, dot, xnv[c * 32 + i] + qn);
-                };
-                uint32_t cmask = 0;
+            const uint32_t tbase =
+                tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)acc * TC_BN + col0;
+            auto dist_of = [&](const int i, const uint32_t acc_bits) -> float {
+                float dot = __uint_as_float(acc_bits);
+                if (FP8) dot *= xsv[i] * qs;
+                return fmaf(-2.f, dot, xnv[i] + qn);
+            };
+            // the tile's 32-row chunks, each chunk's accumulator columns in r
+#pragma unroll 1
+            for (int c = 0; c < nch; c++) {
+                const uint32_t word = c == 0 ? bw[0] : c == 1 ? bw[1] : c == 2 ? bw[2] : bw[3];
+                uint32_t r[32];
+                tmem_ld_32x32b_x32(tbase + c * 32, r);
+                tmem_ld_wait(r);
+                // Hot loop: two rows at a time, distance and its sign against
+                // the threshold, one mask bit each (2.5 instructions a row; a
+                // compare, a predicated store and a predicated mask update
+                // per row took 5.3 and held the pass at batch 512 to 0.49 ms).
+                // The same roundings as dist_of. A NaN difference (both
+                // infinite, or a NaN distance) is sorted out below.
+                const uint64_t qn2 = f2_pack(qn, qn), qs2 = f2_pack(qs, qs);
+                const uint64_t thr2 = f2_pack(thr_d, thr_d);
+                const uint64_t m2 = f2_pack(-2.f, -2.f), m1 = f2_pack(-1.f, -1.f);
+                // (four masks of eight rows: one chain of 32 shifts waits on itself)
+                uint32_t beyond[4] = {};
 #pragma unroll
                 for (int i4 = 0; i4 < 32; i4 += 4) {
                     const float4 xn4 = *(const float4 *)(xnv + c * 32 + i4);
-                    float4 xs4 = make_float4(1.f, 1.f, 1.f, 1.f);
-                    if (FP8) xs4 = *(const float4 *)(xsv + c * 32 + i4);
-                    const float xna[4] = {xn4.x, xn4.y, xn4.z, xn4.w};
-                    const float xsa[4] = {xs4.x, xs4.y, xs4.z, xs4.w};
+                    uint64_t xn2[2] = {f2_pack(xn4.x, xn4.y), f2_pack(xn4.z, xn4.w)};
+                    uint64_t xs2[2];
+                    if (FP8) {
+                        const float4 xs4 = *(const float4 *)(xsv + c * 32 + i4);
+                        xs2[0] = f2_pack(xs4.x, xs4.y);
+                        xs2[1] = f2_pack(xs4.z, xs4.w);
+                    }
 #pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int i = i4 + u;
-                        float dot = __uint_as_float(r[i]);
-                        if (FP8) dot *= xsa[u] * qs;
-                        const float d = fmaf(-2.f, dot, xna[u] + qn);
-                        if (d <= thr_d) {
-                            if (!RECOMP) stage[i * NSLOT + slot] = d;
-                            cmask |= 1u << i;
-                        }
+                    for (int u = 0; u < 2; u++) {
+                        uint64_t dot = f2_pack(r[i4 + 2 * u], r[i4 + 2 * u + 1]);
+                        if (FP8) dot = f2_mul(dot, f2_mul(xs2[u], qs2));
+                        const uint64_t d = f2_fma(m2, dot, f2_add(xn2[u], qn2));
+                        uint32_t s0, s1;  // threshold - distance
+                        f2_unpack(f2_fma(d, m1, thr2), s0, s1);
+                        beyond[i4 >> 3] = __funnelshift_l(s0, beyond[i4 >> 3], 1);
+                        beyond[i4 >> 3] = __funnelshift_l(s1, beyond[i4 >> 3], 1);
                     }
                 }
-                cmask &= bw[c];
+                // (row 8b + j in bit 7 - j of mask b)
+                uint32_t cmask = __brev(~(beyond[0] << 24 | beyond[1] << 16 | beyond[2] << 8 |
+                                          beyond[3])) & word;
                 // warm-up: an empty list facing more than KP candidates (a
                 // pass without a bound: the first chunk of a compacted set,
                 // of a seeding pass) admits only the chunk's KP best - the
                 // KP-th smallest distance becomes the admission bound -
-                // instead of inserting every candidate into its heap one by
-                // one (the bound: ascending distinct values, counting ties)
+                // instead of taking every candidate in one by one (the
+                // bound: ascending distinct values, counting ties)
+                if (WARM && !lazy && KP == 1) {
+                    // a list of one (most seeding passes) is a minimum: taken
+                    // over the chunk's candidates in place (every lane meets
+                    // its own record rows, so admitting them by row would
+                    // visit most rows of the first chunks)
+                    if (cmask) {
+                        float bd = __int_as_float(0x7f800000);
+                        int bi = -1;
+#pragma unroll
+                        for (int i = 0; i < 32; i++) {
+                            const float d = fmaxf(dist_of(c * 32 + i, r[i]), 0.f);
+                            if (((cmask >> i) & 1u) && (d < bd || (d == bd && bi < 0))) {
+                                bd = d;
+                                bi = i;
+                            }
+                        }
+                        if (bi >= 0) {
+                            const uint32_t rid = a.rowids ? ridv[c * 32 + bi]
+                                                          : (uint32_t)(rbase + c * 32 + bi);
+                            const uint64_t key = make_key(bd, rid);
+                            if (key <= thr) {
+                                n = 1;
+                                PV_L(0) = key;
+                                lmax = thr = key;
+                                thr_d = bd;
+                            }
+                        }
+                    }
+                    continue;
+                }
                 if (WARM && !lazy && n == 0 && __popc(cmask) > KP) {
                     float v[32];
 #pragma unroll
                     for (int i = 0; i < 32; i++)
-                        v[i] = ((cmask >> i) & 1u)
-                                   ? fmaxf(RECOMP ? dist_of(i, r[i]) : stage[i * NSLOT + slot], 0.f)
-                                   : __int_as_float(0x7f800000);
+                        v[i] = ((cmask >> i) & 1u) ? fmaxf(dist_of(c * 32 + i, r[i]), 0.f)
+                                                   : __int_as_float(0x7f800000);
                     float kth = -1.f;
                     for (int cnt = 0; cnt < KP;) {
                         float m = __int_as_float(0x7f800000);
@@ -546,43 +580,40 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                     for (int i = 0; i < 32; i++)
                         if (v[i] > thr_d) cmask &= ~(1u << i);
                 }
+                // The rare admissions: the rows that any lane admits, read
+                // again from the accumulator one by one (the chunk's
+                // registers are not kept for them, and their code is short:
+                // with four rows unrolled the warps waited for instructions a
+                // third of the time)
+                uint32_t rows = __reduce_or_sync(0xffffffffu, cmask);
 #pragma unroll 1
-                while (cmask) {
-                    const int i = __ffs(cmask) - 1;
-                    cmask &= cmask - 1;
-                    float dv;
-                    if (RECOMP) {
-                        uint32_t bits = 0;
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            if (j == i) bits = r[j];
-                        dv = dist_of(i, bits);
-                    } else {
-                        dv = stage[i * NSLOT + slot];
-                    }
-                    const float d = fmaxf(dv, 0.f);
+                while (rows) {
+                    const int i = __ffs(rows) - 1;
+                    rows &= rows - 1;
+                    uint32_t v;
+                    tmem_ld_32x32b_x1(tbase + c * 32 + i, v);
+                    tmem_ld_wait(v);
+                    if (!((cmask >> i) & 1u)) continue;
+                    const float dv = dist_of(c * 32 + i, v);
                     const uint64_t row = rbase + c * 32 + i;
                     const uint32_t rid = a.rowids ? ridv[c * 32 + i] : (uint32_t)row;
-                    const uint64_t key = make_key(d, rid);
+                    const uint64_t key = make_key(fmaxf(dv, 0.f), rid);
                     // <= : the seeded bound is itself a row key that this
                     // pass must admit again (keys are unique)
-                    if (key > thr) continue;
+                    if (!(dv <= thr_d) || key > thr) continue;
                     if (lazy && !lazy_pass(row)) continue;
-                    // the list is a max-heap (root = worst kept key): an
-                    // admission costs O(log KP) shared-memory steps
-                    if (n < KP) {
-                        int j = n++;
-                        while (j > 0) {
-                            const int p = (j - 1) >> 1;
-                            const uint64_t pv = PV_L(p);
-                            if (pv >= key) break;
-                            PV_L(j) = pv;
-                            j = p;
-                        }
-                        PV_L(j) = key;
-                        if (n < KP) continue;
-                    } else {
-                        int j = 0;
+                    int from = 0;
+                    uint64_t put = key;
+                    if (n < KP) {  // in any order until the list is full
+                        PV_L(n) = key;
+                        if (++n < KP) continue;
+                        // full: a max-heap from here on (root = worst kept)
+                        from = (KP >> 1) - 1;
+                        put = from >= 0 ? PV_L(from) : 0;
+                    }
+#pragma unroll 1
+                    for (; from >= 0; from--) {  // `put` to node `from` or below
+                        int j = from;
                         for (;;) {
                             int ch = 2 * j + 1;
                             if (ch >= KP) break;
@@ -594,11 +625,12 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                                     ch++;
                                 }
                             }
-                            if (cv <= key) break;
+                            if (cv <= put) break;
                             PV_L(j) = cv;
                             j = ch;
                         }
-                        PV_L(j) = key;
+                        PV_L(j) = put;
+                        if (from > 0) put = PV_L(from - 1);
                     }
                     lmax = PV_L(0);
                     if (lmax < thr) {
@@ -606,23 +638,13 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                         thr_d = key_dist(lmax);
                     }
                 }
-            };
-            // (loading two chunks before one wait measured slower: 0.0644 vs
-            // 0.0615 ms for the BF16 pass at batch 64)
-            const uint32_t tbase =
-                tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)acc * TC_BN + col0;
-#pragma unroll
-            for (int c = 0; c < CPH; c++) {
-                if (c >= nch) break;
-                uint32_t r0[32];
-                tmem_ld_32x32b_x32(tbase + c * 32, r0);
-                tmem_ld_wait();
-                chunk(c, r0);
             }
             tc_fence_before();
-            mbar_arrive(&tempty[acc]);
             __syncwarp();
-            if (lane == 0) mbar_arrive(&nempty[ns]);
+            if (lane == 0) {
+                mbar_arrive(&tempty[acc]);
+                mbar_arrive(&nempty[ns]);
+            }
             if (tr) a.trace[t * 4 + 3] = globaltimer();
             // a full list's last key bounds the grid-wide bound; pushed only
             // when it improved (all lists of a query push to one word)
@@ -630,57 +652,31 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                 atomicMin(a.tau + qg, lmax);
                 pushed = lmax;
             }
-            return true;
-        };
-        uint32_t wA[CPH], wB[CPH];
-        unsigned long long gA = KEY_MAX, gB = KEY_MAX;
-        // this group's first tile of the pass
-        const uint64_t tfirst = (uint64_t)((half - (int)(T0 % EPI) + EPI) % EPI);
-        if (tfirst < ntiles) load_words(tfirst, wA, gA);
-        for (uint64_t t = tfirst; t < ntiles; t += 2 * EPI) {
-            if (!tile_body(t, wA, gA, wB, gB)) { ok = false; break; }
-            if (t + EPI < ntiles && !tile_body(t + EPI, wB, gB, wA, gA)) { ok = false; break; }
+#pragma unroll
+            for (int j = 0; j < CPH; j++) bw[j] = nbw[j];
+            gt = ngt;
         }
         if (!ok) {
             *abort_flag = 1;
             atomicExch(a.err, 3);
         }
         if (qvalid) {
-            // heap -> ascending list (heapsort in place)
-            for (int end = n - 1; end > 0; end--) {
-                const uint64_t top = PV_L(0), v = PV_L(end);
-                PV_L(end) = top;
-                int j = 0;
-                for (;;) {
-                    int ch = 2 * j + 1;
-                    if (ch >= end) break;
-                    uint64_t cv = PV_L(ch);
-                    if (ch + 1 < end) {
-                        const uint64_t c2 = PV_L(ch + 1);
-                        if (c2 > cv) {
-                            cv = c2;
-                            ch++;
-                        }
-                    }
-                    if (cv <= v) break;
-                    PV_L(j) = cv;
-                    j = ch;
-                }
-                PV_L(j) = v;
-            }
-            // the list's best kwrite keys at or below the grid-wide bound join
-            // its query's dense run (one atomic per list: keys above the bound
-            // cannot be in the answer); a full list reports its last key,
-            // below which it cannot have dropped anything
+            // the list's keys at or below the grid-wide bound join its query's
+            // dense run (one atomic per list: keys above the bound cannot be
+            // in the answer); a full list reports its last key, below which
+            // it cannot have dropped anything
             const unsigned long long bound = *((volatile unsigned long long *)(a.tau + qg));
-            int nw = n < a.kwrite ? n : a.kwrite;
-            while (nw > 0 && PV_L(nw - 1) > bound) nw--;
+            int nw = 0;
+            for (int i = 0; i < n; i++) nw += PV_L(i) <= bound;
             if (nw > 0) {
-                const uint64_t b0 = atomicAdd(a.dcnt + qg, (uint32_t)nw);
+                uint64_t at = atomicAdd(a.dcnt + qg, (uint32_t)nw);
                 uint64_t *dst = a.dense + (uint64_t)qg * a.dcap;
-                for (int i = 0; i < nw && b0 + i < a.dcap; i++) dst[b0 + i] = PV_L(i);
+                for (int i = 0; i < n; i++) {
+                    const uint64_t key = PV_L(i);
+                    if (key <= bound && at < a.dcap) dst[at++] = key;
+                }
             }
-            if (a.fullmin && n == KP) atomicMin(a.fullmin + qg, (unsigned long long)PV_L(KP - 1));
+            if (a.fullmin && n == KP) atomicMin(a.fullmin + qg, (unsigned long long)lmax);
         }
 #undef PV_L
     }
@@ -874,7 +870,7 @@ static __device__ __noinline__ void dense_merge_query(
     const unsigned long long *tau, int KO, const int32_t *__restrict__ qprog,
     const unsigned long long *__restrict__ popcnt, uint64_t nrows, FvHit *__restrict__ out,
     uint32_t *__restrict__ out_cnt, uint8_t *__restrict__ trunc, unsigned long long *tau_out,
-    uint8_t *__restrict__ unc) {
+    uint8_t *__restrict__ unc, bool estimated = false) {
     uint64_t *buf = smem_keys;        // [stage_cap] staged keys
     uint64_t *res = buf + stage_cap;  // [DM_OUT] the answer, sorted
     __shared__ unsigned hist[256];
@@ -1024,7 +1020,10 @@ static __device__ __noinline__ void dense_merge_query(
             // member of it
             const unsigned long long lim = c == KO ? res[KO - 1] : bound;
             const unsigned long long fm = fullmin ? fullmin[q] : KEY_MAX;
-            unc[q] = (fm != KEY_MAX && fm <= lim) ? 1 : 0;
+            // an estimated bound that let through fewer than KO keys was too
+            // low (rows beyond it may belong to the answer)
+            const bool low = estimated && c < KO && bound != KEY_MAX;
+            unc[q] = (low || (fm != KEY_MAX && fm <= lim)) ? 1 : 0;
         }
     }
     __syncthreads();
