@@ -50,21 +50,29 @@ __global__ void to_bf16_kernel(const float *__restrict__ src, int dpad, int dim,
 }
 
 // ||x||^2 of the f32 rows (one warp per row) and their maximum (the bits
-// of non-negative floats order like the floats)
+// of non-negative floats order like the floats), nmax[0]; nmax[1]: the
+// largest ||x - t(x)||^2, t dropping the low 13 mantissa bits as the TF32
+// matrix instruction does (the part of a row its dot products miss)
 __global__ void norm32_kernel(const float *__restrict__ src, int dpad, uint64_t nrows,
                               float *__restrict__ norm, unsigned *__restrict__ nmax) {
     const int lane = threadIdx.x & 31;
     uint64_t row = (uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     if (row >= nrows) return;
-    float acc = 0.f;
+    float acc = 0.f, res = 0.f;
     for (int j = lane; j < dpad; j += 32) {
         const float v = src[row * dpad + j];
+        const float d = v - __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
         acc = fmaf(v, v, acc);
+        res = fmaf(d, d, res);
     }
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (int o = 16; o; o >>= 1) {
+        acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        res += __shfl_xor_sync(0xffffffffu, res, o);
+    }
     if (lane == 0) {
         norm[row] = acc;
         atomicMax(nmax, __float_as_uint(acc));
+        atomicMax(nmax + 1, __float_as_uint(res));
     }
 }
 
@@ -342,23 +350,24 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
     g->row_amax = prep ? prep->row_amax : pv_integral_amax(vectors, count * (uint64_t)dim);
 
     // f32 row norms for the exact mode's tensor-core scan (padded to whole
-    // 128-row tiles, then the maximum's word)
+    // 128-row tiles, then the maxima's words)
     {
         const size_t rows_pad32 = (size_t)((count + 127) / 128) * 128;
         if ((e = cudaMalloc(&g->d_norm32, rows_pad32 * 4 + 16)) != cudaSuccess)
             return bail("f32 norms", e);
         unsigned *d_max = (unsigned *)(g->d_norm32 + rows_pad32);
-        unsigned h_max = 0;
+        unsigned h_max[2] = {};
         if ((e = cudaMemsetAsync(g->d_norm32, 0, rows_pad32 * 4 + 16, g->stream)) != cudaSuccess)
             return bail("f32 norms", e);
         norm32_kernel<<<(unsigned)((count + 7) / 8), 256, 0, g->stream>>>(g->d_vecs, dpad, count,
                                                                          g->d_norm32, d_max);
         if ((e = cudaGetLastError()) != cudaSuccess) return bail("f32 norms", e);
-        if ((e = cudaMemcpyAsync(&h_max, d_max, 4, cudaMemcpyDeviceToHost, g->stream)) !=
+        if ((e = cudaMemcpyAsync(h_max, d_max, 8, cudaMemcpyDeviceToHost, g->stream)) !=
                 cudaSuccess ||
             (e = cudaStreamSynchronize(g->stream)) != cudaSuccess)
             return bail("f32 norms", e);
-        memcpy(&g->norm32_max, &h_max, 4);
+        memcpy(&g->norm32_max, &h_max[0], 4);
+        memcpy(&g->res32_max, &h_max[1], 4);
     }
 
     if (precision != FV_GPU_PREC_FP32) {
@@ -504,6 +513,7 @@ FvGpuIndex *index_view(const FvGpuIndex *g) {
     v->d_norm = g->d_norm;
     v->d_norm32 = g->d_norm32;
     v->norm32_max = g->norm32_max;
+    v->res32_max = g->res32_max;
     v->exact_tc = g->exact_tc;
     v->row_amax = g->row_amax;
     v->sorted_cols = g->sorted_cols;

@@ -114,6 +114,7 @@ struct FvGpuIndex {
     // the exact mode's tensor-core scan (f32 rows read as TF32)
     float *d_norm32 = nullptr;  // [rows padded to 128] ||x||^2 of the f32 rows
     float norm32_max = 0.f;     // largest of them
+    float res32_max = 0.f;      // largest squared part of a row that TF32 drops
     int exact_tc = 1;           // exact-mode batches may take it (0: CUDA cores only)
     int last_exact_tc = 0;      // the last brute batch took it
 

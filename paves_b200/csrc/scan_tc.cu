@@ -418,7 +418,8 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     g->launches += 4;  // query prep, main pass, merge, re-rank
     PV_CUDA_OK(launch_pdl(query_prep_kernel, dim3((nqpad + 7) / 8), dim3(256), 0, g->stream, d_q,
                           nq, g->dpad, g->dim, nqpad, R > 1 ? bq : nqpad, kelems, kind, c,
-                          (float *)(c + off_qn), fp8 ? (float *)(c + off_qs) : nullptr,
+                          (float *)(c + off_qn),
+                          fp8 || tf32 ? (float *)(c + off_qs) : nullptr,
                           s.tau.as<unsigned long long>(), d_dcnt,
                           certify ? d_fullmin : nullptr, d_err, behind_bitmaps ? 1 : 0),
                errbuf, errlen);
@@ -602,7 +603,9 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         RerankCert cert;
         if (num_cert) {
             cert.qnorm = (const float *)(c + off_qn);
+            cert.qres = (const float *)(c + off_qs);
             cert.xnmax = g->norm32_max;
+            cert.xrmax = g->res32_max;
             cert.dim = g->dpad;
             cert.unc = d_unc;
         }

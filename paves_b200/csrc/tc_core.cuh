@@ -713,7 +713,7 @@ __device__ __forceinline__ void query_prep_row(int qi, int lane, const float *__
         for (int j = lane; j < dim; j += 32) amax = fmaxf(amax, fabsf(q[(size_t)src * dpad + j]));
     for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     const float s = amax > 0.f ? amax / 448.f : 1.f;
-    float acc = 0.f;
+    float acc = 0.f, res = 0.f;
     for (int j = lane; j < kelems; j += 32) {
         const float v = (ok && j < dim) ? q[(size_t)src * dpad + j] : 0.f;
         float r;
@@ -722,10 +722,14 @@ __device__ __forceinline__ void query_prep_row(int qi, int lane, const float *__
             out[(size_t)qi * kelems + j] = *(unsigned char *)&b;
             r = float(b) * s;
         } else if (kind == TCK_TF32) {
-            // the f32 value itself (the MMA reads its tf32 part); the norm
-            // is the exact row's
-            ((float *)out)[(size_t)qi * kelems + j] = v;
+            // the nearest TF32 value (the MMA would drop the low bits, twice
+            // as far off); the norm is the exact row's
+            const uint32_t u = __float_as_uint(v);
+            float t = __uint_as_float((u + 0xFFFu + ((u >> 13) & 1u)) & 0xFFFFE000u);
+            if (!(fabsf(v) < 3e38f)) t = v;  // infinities and NaN as they are
+            ((float *)out)[(size_t)qi * kelems + j] = t;
             r = v;
+            res = fmaf(v - t, v - t, res);
         } else {
             __nv_bfloat16 b = __float2bfloat16_rn(v);
             ((__nv_bfloat16 *)out)[(size_t)qi * kelems + j] = b;
@@ -733,10 +737,14 @@ __device__ __forceinline__ void query_prep_row(int qi, int lane, const float *__
         }
         acc = fmaf(r, r, acc);
     }
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (int o = 16; o; o >>= 1) {
+        acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        res += __shfl_xor_sync(0xffffffffu, res, o);
+    }
     if (lane == 0) {
         qnorm[qi] = acc;
-        if (qscale) qscale[qi] = s;
+        // fp8: the scale; TF32: what the rounding left of the query, squared
+        if (qscale) qscale[qi] = kind == TCK_TF32 ? res : s;
     }
 }
 
@@ -749,21 +757,27 @@ __device__ __forceinline__ void query_prep_row(int qi, int lane, const float *__
 //     (A - E) * (1 - c2) > Dk,
 // E bounding |scan distance - true distance| and c2 the relative error of
 // the f32 difference-form sum (the exact distance) against the true one:
-//   * the MMA reads each f32 operand with its low 13 mantissa bits
-//     dropped, a relative change below 2^-10 per operand, so each product
-//     moves by at most (2^-9 + 2^-20) |x_i| |q_i|; the f32 accumulation in
-//     the tensor core adds at most about dim * 2^-22 of sum |x_i q_i|; and
-//     sum |x_i| |q_i| <= ||x|| ||q|| (Cauchy-Schwarz), with ||x||^2 at most
-//     xnmax over all rows;
+//   * the MMA sees t(x), the row without its low 13 mantissa bits, and q',
+//     the query rounded to TF32: x.q - t(x).q' = t(x).(q - q') + (x - t(x)).q,
+//     at most ||x|| ||q - q'|| + ||x - t(x)|| ||q|| (Cauchy-Schwarz, and
+//     ||t(x)|| <= ||x||), with ||x||^2 at most xnmax and ||x - t(x)||^2 at
+//     most xrmax over all rows: about 1.2 * 2^-10 ||x|| ||q|| on ordinary
+//     values, where 2^-9 per product is what any values allow (that bound
+//     left 3 of 64 queries of 1M real-valued rows uncertified, whose exact
+//     re-run took two thirds of the call);
+//   * the f32 accumulation in the tensor core adds at most about
+//     dim * 2^-22 of sum |x_i q_i| <= ||x|| ||q||;
 //   * the f32 norms (dim terms) and the two roundings of ||x||^2 + ||q||^2
 //     - 2 q.x stay within c2 = (dim + 8) * 2^-23 of the values they round.
-// E = 1.25 * 2^-8 ||q|| sqrt(xnmax) (1 + c2) + c2 (xnmax + ||q||^2 + A)
-// covers both terms with a margin (the first has 2^-8 * 1.25 against the
-// 2^-8 + 2^-19 + dim * 2^-21 the analysis needs for dim <= 128). Queries
-// that fail are flagged in unc[] for an exact re-run.
+// E = 2 (1 + 2^-6) (||x|| ||q - q'|| + ||x - t(x)|| ||q||) + dim 2^-20 ||x|| ||q||
+//     + c2 (xnmax + ||q||^2 + A): the first term's margin covers the f32
+// roundings of the norms themselves, the second is twice what the analysis
+// needs. Queries that fail are flagged in unc[] for an exact re-run.
 struct RerankCert {
     const float *qnorm = nullptr;  // [nq] ||q||^2 (f32)
+    const float *qres = nullptr;   // [nq] ||q - q'||^2 (f32)
     float xnmax = 0.f;             // max ||x||^2 over the rows (f32 norms)
+    float xrmax = 0.f;             // max ||x - t(x)||^2 over the rows
     int dim = 0;
     uint8_t *unc = nullptr;        // [nq] set to 1 when not certified
 };
@@ -844,7 +858,9 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
             const double Dk = (double)key_dist(keys[nout - 1]);
             const double qn = (double)cert.qnorm[q], xm = (double)cert.xnmax;
             const double c2 = (double)(cert.dim + 8) * 0x1p-23;
-            const double E = 1.25 * 0x1p-8 * sqrt(qn * xm) * (1.0 + c2) + c2 * (xm + qn + A);
+            const double qr = (double)cert.qres[q], xr = (double)cert.xrmax;
+            const double E = 2.0 * (1.0 + 0x1p-6) * (sqrt(xm * qr) + sqrt(xr * qn)) +
+                             cert.dim * 0x1p-20 * sqrt(qn * xm) + c2 * (xm + qn + A);
             if (!((A - E) * (1.0 - c2) > Dk)) cert.unc[q] = 1;
         }
     }
