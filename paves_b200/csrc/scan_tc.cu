@@ -540,10 +540,16 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         // sample one tile's time, and a list of the main pass admits about
         // S * tpc / (m * grow) rows; the sum is least near sqrt(S tpc / grow)
         // times a constant measured at 1 (batch 512, 128 and 64 of 1M rows:
-        // half and twice as many tiles are both slower or the same).
+        // half and twice as many tiles are both slower or the same). At most
+        // 24 (graph construction, 2048 queries with lists of 64: 62.6 ms
+        // for 60,000 rows with 24, 70.6 with 8; batch 1000 the same with
+        // both), 8 where an estimated bound makes up for a short sample.
         const uint64_t region = ntiles_all / grow;
         const double best = sqrt((double)S * tpc / grow);
-        const uint64_t m = std::min<uint64_t>(region, best < 1.0 ? 1 : best > 8.0 ? 8 : (uint64_t)best);
+        // (and chunks for four times the keys a certain bound needs)
+        const uint64_t least = certify ? 1 : ((uint64_t)S + grow - 1) / grow;
+        const uint64_t m = std::min<uint64_t>(
+            region, std::min<uint64_t>(certify ? 8 : 24, std::max<uint64_t>(least, (uint64_t)best)));
         sa.tile0_mul = region;
         sa.tile_step = std::max<uint64_t>(1, region / m);
         sa.tiles_per_cta = m;
@@ -559,11 +565,19 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         const int rank_est = (int)ceil(S * share + 6.0 * sqrt(S * share) + 8.0);
         estimated = certify && rank_est < S;
         const int rank = estimated ? rank_est : S;
-        // lists need hold no more than their share of 4 rank keys, at least
-        // one (short lists admit fewer rows, and the merge reads fewer keys);
-        // never more than the main pass's length (its shared memory). A full
-        // list's last key bounds the S-th key only if it holds S.
-        sa.KP = std::min(KP, std::max(1, (4 * rank + nlists - 1) / std::max(1, nlists)));
+        // A list keeps the best key of every few of its chunks, about 4 rank
+        // keys in all (the S-th key of a subset of the sample still bounds
+        // the S-th key of the scan, and short runs keep the merge cheap):
+        // the rank-th of 4 rank chunk minima lies about 1.15 times as deep as
+        // the sample's own rank-th key. Lazy batches, which cannot tell a
+        // chunk's best passing row, keep their share of the best keys; a
+        // full list's last key then bounds the S-th key if it holds S.
+        const int epiw = std::min(EPI, 2);
+        const int chunks = (int)((m + epiw - 1) / epiw) * (TC_BN / R / 32);  // of a list
+        const int lists = grow * (int)std::min<uint64_t>(m, epiw) * R;
+        const int want = std::max(1, (4 * rank + lists - 1) / lists);
+        sa.KP = std::min(KP, want);
+        sa.seed_group = std::max(1, std::max(chunks / want, (chunks + sa.KP - 1) / sa.KP));
         sa.push_tau = sa.KP == S ? 1 : 0;
         sa.fullmin = nullptr;
         g->launches += 2;  // seeding pass + its merge

@@ -86,6 +86,9 @@ struct TcArgs {
     int rep;            // query replicas down the tile's 128 slots (1, 2, 4)
     int bq;             // query slots per replica = TC_BM / rep
     int push_tau;       // a full list's last key bounds the superset (lists hold it all)
+    // > 0 (WARM passes, no lazy filters): each list takes the best key of
+    // every seed_group 32-row chunks instead of its best KP keys
+    int seed_group = 0;
     int NS;             // pipeline stages
     const float *__restrict__ xnorm;   // [rows padded to 128]
     const float *__restrict__ xscale;  // fp8: per-row scale, else null
@@ -416,6 +419,8 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
         int n = 0;
         uint64_t lmax = KEY_MAX;   // worst kept key once the list is full
         uint64_t pushed = KEY_MAX; // last key this list pushed to the grid-wide bound
+        uint64_t smin = KEY_MAX;   // seeding: best key of the chunks since the last one kept
+        int schunks = 0;
         uint64_t thr = qvalid ? KEY_MAX : 0ull;  // admission threshold
         float thr_d = qvalid ? __int_as_float(0x7f800000) : -1.f;  // its distance
         bool ok = true;
@@ -486,6 +491,34 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                 uint32_t r[32];
                 tmem_ld_32x32b_x32(tbase + c * 32, r);
                 tmem_ld_wait(r);
+                if (WARM && a.seed_group > 0 && !lazy) {
+                    // a seeding pass keeps the best passing row of every few
+                    // chunks: no bound, no heap, the same work for every lane
+                    // (lists of the best KP met their own record rows one by
+                    // one: 0.49 ms a pass with lists of 28, 2048 queries)
+                    float bd = __int_as_float(0x7f800000);
+                    int bi = -1;
+#pragma unroll
+                    for (int i = 0; i < 32; i++) {
+                        const float d = dist_of(c * 32 + i, r[i]);
+                        if (((word >> i) & 1u) && d < bd) {
+                            bd = d;
+                            bi = i;
+                        }
+                    }
+                    if (bi >= 0) {
+                        const uint32_t rid = a.rowids ? ridv[c * 32 + bi]
+                                                      : (uint32_t)(rbase + c * 32 + bi);
+                        const uint64_t key = make_key(fmaxf(bd, 0.f), rid);
+                        smin = key < smin ? key : smin;
+                    }
+                    if (++schunks >= a.seed_group) {
+                        if (smin != KEY_MAX && n < KP) PV_L(n++) = smin;
+                        smin = KEY_MAX;
+                        schunks = 0;
+                    }
+                    continue;
+                }
                 // Hot loop: two rows at a time, distance and its sign against
                 // the threshold, one mask bit each (2.5 instructions a row; a
                 // compare, a predicated store and a predicated mask update
@@ -527,36 +560,6 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                 // KP-th smallest distance becomes the admission bound -
                 // instead of taking every candidate in one by one (the
                 // bound: ascending distinct values, counting ties)
-                if (WARM && !lazy && KP == 1) {
-                    // a list of one (most seeding passes) is a minimum: taken
-                    // over the chunk's candidates in place (every lane meets
-                    // its own record rows, so admitting them by row would
-                    // visit most rows of the first chunks)
-                    if (cmask) {
-                        float bd = __int_as_float(0x7f800000);
-                        int bi = -1;
-#pragma unroll
-                        for (int i = 0; i < 32; i++) {
-                            const float d = fmaxf(dist_of(c * 32 + i, r[i]), 0.f);
-                            if (((cmask >> i) & 1u) && (d < bd || (d == bd && bi < 0))) {
-                                bd = d;
-                                bi = i;
-                            }
-                        }
-                        if (bi >= 0) {
-                            const uint32_t rid = a.rowids ? ridv[c * 32 + bi]
-                                                          : (uint32_t)(rbase + c * 32 + bi);
-                            const uint64_t key = make_key(bd, rid);
-                            if (key <= thr) {
-                                n = 1;
-                                PV_L(0) = key;
-                                lmax = thr = key;
-                                thr_d = bd;
-                            }
-                        }
-                    }
-                    continue;
-                }
                 if (WARM && !lazy && n == 0 && __popc(cmask) > KP) {
                     float v[32];
 #pragma unroll
@@ -665,6 +668,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
             // dense run (one atomic per list: keys above the bound cannot be
             // in the answer); a full list reports its last key, below which
             // it cannot have dropped anything
+            if (WARM && smin != KEY_MAX && n < KP) PV_L(n++) = smin;
             const unsigned long long bound = *((volatile unsigned long long *)(a.tau + qg));
             int nw = 0;
             for (int i = 0; i < n; i++) nw += PV_L(i) <= bound;
