@@ -47,7 +47,7 @@ cudaError_t launch_bitmaps_rank(const FvGpuIndex *g, const PredInsn *insns, cons
 // bound); KO <= 1024. Writes out [nq][KO] ascending, out_cnt, trunc (from
 // popcnt[qprog[q]] or nrows), tau_out[q] = min(tau_out[q], KO-th key) and
 // unc[q] (a full list's last key, fullmin[q], at or below the answer's end;
-// or, with an estimated bound, KO > 32, fewer than KO keys at or below it).
+// or, with an estimated bound, fewer than KO keys at or below it).
 cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *dcnt,
                                bool reset_cnt, const unsigned long long *fullmin,
                                const unsigned long long *tau, int KO, const int32_t *qprog,

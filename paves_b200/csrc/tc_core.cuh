@@ -1049,9 +1049,9 @@ static __device__ __noinline__ void dense_merge_query(
     __syncthreads();
 }
 
-// The same for KO <= 32, without block barriers in the hot loop: each warp
-// keeps its 32 best keys sorted across its lanes (one key per lane) and
-// folds in 32 new keys at a time (a shuffle bitonic sort of the new keys in
+// The same for KO <= 64, without block barriers in the hot loop: each warp
+// keeps its 32 (64) best keys sorted across its lanes (one or two keys per
+// lane) and folds in 32 new keys at a time (a shuffle bitonic sort of the new keys in
 // descending order, an elementwise min with the list, which leaves the 32
 // smallest as a bitonic sequence, and a bitonic clean back to ascending);
 // a batch none of whose keys beats the list's last key is skipped. The
@@ -1078,16 +1078,34 @@ __device__ __forceinline__ uint64_t warp_clean32(uint64_t x, int lane) {
     return x;
 }
 
-// One query's merge for KO <= 32 by all threads of the block (any whole
-// number of warps); lists: one 32-key slot per warp in shared memory.
-// Ends with the block synchronized.
+// One query's merge for KO <= 32 W (W 1 or 2 keys per lane, the second the
+// larger half of the list) by all threads of the block (any whole number of
+// warps); lists: one slot per warp in shared memory. Ends with the block
+// synchronized.
+template <int W>
+__device__ __forceinline__ void warp_fold32(uint64_t (&best)[W], uint64_t d, int lane) {
+    // d: 32 keys, descending across the lanes
+    if (W == 1) {
+        best[0] = warp_clean32(best[0] < d ? best[0] : d, lane);
+    } else {
+        // the upper half takes the 32 smallest of itself and d, then trades
+        // with the lower half
+        const uint64_t h = warp_clean32(best[W - 1] < d ? best[W - 1] : d, lane);
+        const uint64_t r = __shfl_sync(0xffffffffu, h, 31 - lane);
+        const uint64_t lo = best[0];
+        best[0] = warp_clean32(lo < r ? lo : r, lane);
+        best[W - 1] = warp_clean32(lo < r ? r : lo, lane);
+    }
+}
+
+template <int W = 1>
 __device__ __forceinline__ void dense_top32_query(
-    int q, uint64_t (*lists)[32], const uint64_t *__restrict__ dense, uint64_t dcap,
+    int q, uint64_t (*lists)[32 * W], const uint64_t *__restrict__ dense, uint64_t dcap,
     uint32_t *__restrict__ dcnt, int reset_cnt, const unsigned long long *__restrict__ fullmin,
     const unsigned long long *tau, int KO, const int32_t *__restrict__ qprog,
     const unsigned long long *__restrict__ popcnt, uint64_t nrows, FvHit *__restrict__ out,
     uint32_t *__restrict__ out_cnt, uint8_t *__restrict__ trunc, unsigned long long *tau_out,
-    uint8_t *__restrict__ unc, long long passing_pre = -1) {
+    uint8_t *__restrict__ unc, long long passing_pre = -1, bool estimated = false) {
     const int NW = blockDim.x >> 5;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned long long bound = tau ? tau[q] : KEY_MAX;
@@ -1096,7 +1114,9 @@ __device__ __forceinline__ void dense_top32_query(
     const uint64_t *src = dense + (uint64_t)q * dcap;
     __syncthreads();
     if (reset_cnt && tid == 0) dcnt[q] = 0;  // every thread has read it
-    uint64_t best = KEY_MAX;  // ascending across the lanes
+    uint64_t best[W];  // ascending across the lanes, half by half
+#pragma unroll
+    for (int h = 0; h < W; h++) best[h] = KEY_MAX;
     for (uint64_t b = (uint64_t)warp * 64; b < n; b += NW * 64) {
         uint64_t k2[2];
 #pragma unroll
@@ -1107,36 +1127,44 @@ __device__ __forceinline__ void dense_top32_query(
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            const uint64_t worst = __shfl_sync(0xffffffffu, best, 31);
+            const uint64_t worst = __shfl_sync(0xffffffffu, best[W - 1], 31);
             if (!__any_sync(0xffffffffu, k2[u] < worst)) continue;
-            const uint64_t d = warp_sort32(k2[u], lane, true);
-            best = warp_clean32(best < d ? best : d, lane);
+            warp_fold32<W>(best, warp_sort32(k2[u], lane, true), lane);
         }
     }
     // the warps' lists fold pairwise, log2(NW) rounds (warp w takes in
     // warp w + step's list, read descending, while w is a multiple of 2 step)
-    lists[warp][lane] = best;
+#pragma unroll
+    for (int h = 0; h < W; h++) lists[warp][h * 32 + lane] = best[h];
     for (int step = 1; step < NW; step <<= 1) {
         __syncthreads();
         if ((warp & (2 * step - 1)) == 0 && warp + step < NW) {
-            const uint64_t d = lists[warp + step][31 - lane];
-            const uint64_t m = best < d ? best : d;
-            if (__any_sync(0xffffffffu, m != best)) {
-                best = warp_clean32(m, lane);
-                lists[warp][lane] = best;
+#pragma unroll
+            for (int h = 0; h < W; h++) {
+                const uint64_t d = lists[warp + step][h * 32 + 31 - lane];
+                const uint64_t worst = __shfl_sync(0xffffffffu, best[W - 1], 31);
+                if (__any_sync(0xffffffffu, d < worst)) warp_fold32<W>(best, d, lane);
             }
+#pragma unroll
+            for (int h = 0; h < W; h++) lists[warp][h * 32 + lane] = best[h];
         }
     }
     if (warp == 0) {
-        const bool have = lane < KO && best != KEY_MAX;
-        const int c = __popc(__ballot_sync(0xffffffffu, have));
-        if (have) {
-            FvHit h;
-            h.node = (uint64_t)key_row(best);
-            h.dist = key_dist(best);
-            out[(uint64_t)q * KO + lane] = h;
+        int c = 0;
+        uint64_t last = 0;
+#pragma unroll
+        for (int h = 0; h < W; h++) {
+            const bool have = h * 32 + lane < KO && best[h] != KEY_MAX;
+            c += __popc(__ballot_sync(0xffffffffu, have));
+            if (have) {
+                FvHit hit;
+                hit.node = (uint64_t)key_row(best[h]);
+                hit.dist = key_dist(best[h]);
+                out[(uint64_t)q * KO + h * 32 + lane] = hit;
+            }
+            const uint64_t l = __shfl_sync(0xffffffffu, best[h], (KO - 1) & 31);
+            if ((KO - 1) >> 5 == h) last = l;
         }
-        const uint64_t last = __shfl_sync(0xffffffffu, best, KO - 1);
         if (lane == 0) {
             out_cnt[q] = (uint32_t)c;
             unsigned long long passing = (unsigned long long)passing_pre;
@@ -1149,7 +1177,8 @@ __device__ __forceinline__ void dense_top32_query(
             if (unc) {
                 const unsigned long long lim = c == KO ? last : bound;
                 const unsigned long long fm = fullmin ? fullmin[q] : KEY_MAX;
-                unc[q] = (fm != KEY_MAX && fm <= lim) ? 1 : 0;
+                const bool low = estimated && c < KO && bound != KEY_MAX;
+                unc[q] = (low || (fm != KEY_MAX && fm <= lim)) ? 1 : 0;
             }
         }
     }
