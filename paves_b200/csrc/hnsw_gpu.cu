@@ -62,7 +62,7 @@ __device__ __forceinline__ void hg_row(float4 (&r)[NV], const float *x, uint64_t
 // itself are skipped. A lane holds dims 4 lane + 128 i of a row; the kept
 // rows are compared JB at a time and the next candidate's row loads
 // meanwhile: one after another each waited out an L2 round trip (0.27 ms a
-// batch of 2048 nodes, 64 candidates, now 0.10 ms).
+// batch of 2048 nodes, 64 candidates, now 0.20 ms).
 template <int NV>
 __device__ int hg_select(const uint64_t *ck, int n, uint32_t v, int R, const float *x, int dpad,
                          uint32_t *kept, uint32_t *rej, int lane) {
