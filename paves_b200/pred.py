@@ -179,9 +179,18 @@ def concat(preds: Sequence[Optional[Pred]], count: int,
     qd["total"] = count
     if entries is not None:
         qd["entry"] = np.asarray(entries)[:nq]
+    recs, children, invals = [], [], []
+    if nq - sum(p is None for p in preds) <= 8:
+        # a few filters: every query's slice in place (the gather below costs
+        # 45 us whatever the batch)
+        roots = [-1 if p is None else _flat(p, recs, children, invals) for p in preds]
+        qd["proot"] = roots
+        return BatchPred(qd, np.frombuffer(b"".join(recs), NODE_DTYPE).copy(),
+                         np.array(children, np.int32), np.array(invals, np.float64),
+                         np.zeros(0, SPAN_DTYPE), np.zeros(0, np.uint64), np.zeros(nq, np.uint8),
+                         np.array(roots, np.int32))
     # each distinct tree once, then every query's slice gathered from it with
     # its indexes moved to the slice's place
-    recs, children, invals = [], [], []
     place, size = {}, [(0, 0, 0)]  # tree -> its number; running ends of the three arrays
     which = []
     for p in preds:
