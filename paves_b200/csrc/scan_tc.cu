@@ -387,12 +387,53 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // rows scanned: the index's, or a compacted set
     const uint64_t nrows_scan = rs ? rs->nrows : g->count;
     const uint64_t ntiles_all = (nrows_scan + TC_BN - 1) / TC_BN;
-    int grow = g->tune_grow > 0 ? g->tune_grow : g->sm_count / qtiles;
-    if (grow < 1) grow = 1;
-    uint64_t maxg = (ntiles_all + 3) / 4;
-    if ((uint64_t)grow > maxg) grow = (int)maxg;
-    const uint64_t tpc = (ntiles_all + grow - 1) / grow;
-    grow = (int)((ntiles_all + tpc - 1) / tpc);
+    const bool certify = KP < S;  // lists shorter than the superset
+    int grow = std::max(1, g->tune_grow > 0 ? g->tune_grow : g->sm_count / qtiles);
+    auto split = [&](uint64_t most) {  // CTAs along the rows, evenly loaded
+        if ((uint64_t)grow > most) grow = (int)most;
+        const uint64_t per = (ntiles_all + grow - 1) / grow;
+        grow = (int)((ntiles_all + per - 1) / per);
+        return per;
+    };
+    uint64_t tpc = split((ntiles_all + 1) / 2);
+    // Seeding pass: a few tiles per CTA from an evenly strided sample; the
+    // rank-th key of the sample bounds the S-th key of the whole scan, so the
+    // main pass admits only rows that can still matter. Tiles per CTA, spread
+    // over its own range: a tile more costs the sample one tile's time, and a
+    // list of the main pass admits about S * tpc / (m * grow) rows; the sum is
+    // least near sqrt(S tpc / grow) times a constant measured at 1 (batch 512,
+    // 128 and 64 of 1M rows: half and twice as many tiles are both slower or
+    // the same). At most 24 (graph construction, 2048 queries with lists of
+    // 64: 62.6 ms for 60,000 rows with 24, 70.6 with 8; batch 1000 the same
+    // with both), 8 where an estimated bound makes up for a short sample; and
+    // chunks for four times the keys a certain bound needs.
+    const uint64_t region = ntiles_all / grow;
+    const double best = sqrt((double)S * tpc / grow);
+    const uint64_t least = certify ? 1 : ((uint64_t)S + grow - 1) / grow;
+    const uint64_t m = std::min<uint64_t>(
+        region, std::min<uint64_t>(certify ? 8 : 24, std::max<uint64_t>(least, (uint64_t)best)));
+    // The sample's S-th key is a bound for certain, but with large supersets
+    // it admits S / share rows, far more than S. A sample holding `share` of
+    // the rows has S * share of the S best in expectation, with a Poisson
+    // spread: its key six deviations above that lies beyond the S-th key of
+    // the scan but for about one query in 10^9, and the merge sees such a
+    // query (fewer than S keys got through), which is then re-run exactly.
+    // Only where the merge certifies anyway (lists shorter than the superset).
+    const double share = std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan);
+    const int rank_est = (int)ceil(S * share + 6.0 * sqrt(S * share) + 8.0);
+    const bool estimated = certify && rank_est < S;
+    const int rank = estimated ? rank_est : S;
+    // Seeding pays from two tiles per CTA on, as long as the sample's chunk
+    // minima are at least twice the keys its bound needs: small tables took
+    // 2 to 4 times as long filling their lists behind no bound (100,000 BF16
+    // rows, 73 queries: k 2, 25, 100 in 0.106, 0.158, 0.343 ms, seeded 0.043,
+    // 0.044, 0.079). Without it every tile gets its own CTA.
+    const bool seed =
+        g->tune_seed != 2 && m * grow * (TC_BN / 32) >= 2 * (uint64_t)rank;
+    if (!seed) {
+        grow = std::max(1, g->tune_grow > 0 ? g->tune_grow : g->sm_count / qtiles);
+        tpc = split(ntiles_all);
+    }
 
     ScanScratch &s = g->scan;
     const size_t qbytes = (size_t)nqpad * kelems * esz;
@@ -416,7 +457,6 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     unsigned long long *d_fullmin = (unsigned long long *)(s.part_cnt.as<char>() + off_fm);
     unsigned char *c = s.cand.as<unsigned char>();
     int *d_err = (int *)(c + off_err);
-    const bool certify = KP < S;  // lists shorter than the superset
     // inexact scan distances of exact-mode batches: the re-rank certifies
     const bool num_cert = tf32 && S > (int)topb;
 
@@ -520,7 +560,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
             a.trace_tiles = 64;
         }
     }
-    // warm: a pass that starts without a bound (see tc_pass)
+    // warm: a seeding pass, or one that starts without a bound (see tc_pass)
     // (a warm pass with three groups would not fit its registers: it runs
     // with two, inside the same shared-memory carve and dense runs)
     auto run = [&](const TcArgs &args, bool warm) {
@@ -534,42 +574,11 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     };
     FvHit *cand = (FvHit *)(c + off_cand);
     uint32_t *ccnt = (uint32_t *)(c + off_ccnt);
-    // Seeding pass: a few tiles per CTA from an evenly strided sample; the
-    // rank-th key of the sample bounds the S-th key of the whole scan, so the
-    // main pass admits only rows that can still matter.
-    const bool seed = g->tune_seed == 2 ? false : ntiles_all >= 8 * (uint64_t)grow;
-    bool estimated = false;
     if (seed) {
         TcArgs sa = a;
-        // Tiles per CTA, spread over its own range: a tile more costs the
-        // sample one tile's time, and a list of the main pass admits about
-        // S * tpc / (m * grow) rows; the sum is least near sqrt(S tpc / grow)
-        // times a constant measured at 1 (batch 512, 128 and 64 of 1M rows:
-        // half and twice as many tiles are both slower or the same). At most
-        // 24 (graph construction, 2048 queries with lists of 64: 62.6 ms
-        // for 60,000 rows with 24, 70.6 with 8; batch 1000 the same with
-        // both), 8 where an estimated bound makes up for a short sample.
-        const uint64_t region = ntiles_all / grow;
-        const double best = sqrt((double)S * tpc / grow);
-        // (and chunks for four times the keys a certain bound needs)
-        const uint64_t least = certify ? 1 : ((uint64_t)S + grow - 1) / grow;
-        const uint64_t m = std::min<uint64_t>(
-            region, std::min<uint64_t>(certify ? 8 : 24, std::max<uint64_t>(least, (uint64_t)best)));
         sa.tile0_mul = region;
         sa.tile_step = std::max<uint64_t>(1, region / m);
         sa.tiles_per_cta = m;
-        // The sample's S-th key is a bound for certain, but with large
-        // supersets it admits S / share rows, far more than S. A sample
-        // holding `share` of the rows has S * share of the S best in
-        // expectation, with a Poisson spread: its key six deviations above
-        // that lies beyond the S-th key of the scan but for about one query
-        // in 10^9, and the merge sees such a query (fewer than S keys got
-        // through), which is then re-run exactly. Only where the merge
-        // certifies anyway (lists shorter than the superset).
-        const double share = std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan);
-        const int rank_est = (int)ceil(S * share + 6.0 * sqrt(S * share) + 8.0);
-        estimated = certify && rank_est < S;
-        const int rank = estimated ? rank_est : S;
         // A list keeps the best key of every few of its chunks, about 4 rank
         // keys in all (the S-th key of a subset of the sample still bounds
         // the S-th key of the scan, and short runs keep the merge cheap):
@@ -601,7 +610,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // spread over the CTAs
     a.tile0_mul = rs ? 1 : tpc;
     a.tile_step = rs ? (uint64_t)grow : 1;
-    PV_CUDA_OK(run(a, rs != nullptr), errbuf, errlen);
+    PV_CUDA_OK(run(a, rs != nullptr || !seed), errbuf, errlen);
     if (ev) cudaEventRecord(ev[2], g->stream);
     uint8_t *d_unc = (certify || num_cert) ? (uint8_t *)(c + off_unc) : nullptr;
     if (S == (int)topb) {
@@ -611,13 +620,13 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         g->launches--;
         PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, false, a.fullmin, a.tau, S,
                                       d_qprog, popcnt, g->count, nq, d_out, d_cnt, d_trunc,
-                                      nullptr, d_unc, g->stream, estimated),
+                                      nullptr, d_unc, g->stream, seed && estimated),
                    errbuf, errlen);
     } else {
         PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, false, a.fullmin, a.tau, S,
                                       d_qprog, popcnt, g->count, nq, cand, ccnt,
                                       (uint8_t *)(c + off_ctr), nullptr, d_unc, g->stream,
-                                      estimated),
+                                      seed && estimated),
                    errbuf, errlen);
         RerankCert cert;
         if (num_cert) {
