@@ -84,10 +84,10 @@ int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &
     // sparse route: one filter shared by the whole batch whose matches are
     // bounded by a small count (the scan then reads only those rows)
     db.sparse_bound = 0;
+    db.one_prog = P == 1;
+    for (int q = 0; q < nq && db.one_prog; q++) db.one_prog = pb.qprog[q] == 0;
     if (P == 1 && !g->sorted_cols.empty()) {
-        bool all = true;
-        for (int q = 0; q < nq && all; q++) all = pb.qprog[q] == 0;
-        if (all) {
+        if (db.one_prog) {
             const uint64_t b = prog_upper_bound(g, pb.insns.data() + pb.progs[0].insn0,
                                                 pb.progs[0].ninsn, pb.consts.data());
             // (the route holds one key per query and listed row: 128 MB at most)
@@ -165,8 +165,20 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     ScanScratch &s = g->scan;
 
     if (ev) cudaEventRecord(ev[0], g->stream);
-    if (bitmaps_ready) {
-        // the caller launched the bitmaps of this batch
+    const bool sparse_route = db.sparse_bound > 0 && !db.counts_on_device && topb <= 1024;
+    const bool low_tc_can = mode == 1 && tc_supported(g) && tc_superset(g, topb, db.q_amax) > 0;
+    const bool exact_tc_can = mode == PV_MODE_EXACT && nq >= PV_EXACT_TC_MIN_NQ &&
+                              tf32_supported(g) && tf32_superset(g, topb, db.q_amax) > 0;
+    const bool sparse_tc = sparse_route && (low_tc_can || exact_tc_can) &&
+                           db.sparse_bound >= PV_SPARSE_TC_MIN_ROWS;
+    // a few queries answered exactly on the CUDA cores: only the rows their
+    // filter passes are read (a selective filter's list would be made first)
+    const bool rows_route =
+        !db.counts_on_device && scan_rows_fits(nq, g->dpad, topb) && !sparse_tc &&
+        (sparse_route || !(low_tc_can || exact_tc_can));
+    db.rows_fused = rows_route && !bitmaps_ready && db.one_range && db.one_prog;
+    if (bitmaps_ready || db.rows_fused) {
+        // the caller launched the bitmaps of this batch, or none are needed
     } else if (P > 0) {
         if (brute_bitmaps(g, db, errbuf, errlen)) return -1;
     } else {
@@ -177,29 +189,34 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     // by asking for bm_done
     const bool bm_launched =
         !db.counts_on_device && P > 0 && (!bitmaps_ready || bm_done != nullptr);
-    const bool sparse_route = db.sparse_bound > 0 && !db.counts_on_device && topb <= 1024;
-    const bool low_tc_route =
-        !sparse_route && mode == 1 && tc_supported(g) && tc_superset(g, topb, db.q_amax) > 0;
-    const bool exact_tc_route = !sparse_route && !low_tc_route && mode == PV_MODE_EXACT &&
-                                nq >= PV_EXACT_TC_MIN_NQ && tf32_supported(g) &&
-                                tf32_superset(g, topb, db.q_amax) > 0;
+    const bool low_tc_route = !sparse_route && low_tc_can;
+    const bool exact_tc_route = !sparse_route && exact_tc_can;
     // bm_done: the bitmaps are complete once query prep, run beside them,
     // completes (tensor-core routes), else at once in stream order
     if (bm_done && !(low_tc_route || exact_tc_route))
         PV_CUDA_OK(cudaEventRecord(bm_done, g->stream), errbuf, errlen);
     g->last_sparse = 0;
     g->last_exact_tc = 0;
+    if (rows_route) {
+        g->last_sparse = sparse_route ? 1 : 0;
+        g->tc_err = nullptr;
+        g->tc_unc = nullptr;
+        if (ev) cudaEventRecord(ev[1], g->stream);
+        if (scan_rows_launch(g, db, topb, d_out, d_cnt, d_trunc, errbuf, errlen)) return -1;
+        if (ev) {
+            cudaEventRecord(ev[2], g->stream);
+            cudaEventRecord(ev[3], g->stream);
+            cudaEventRecord(ev[4], g->stream);
+        }
+        return 0;
+    }
     if (sparse_route) {
         g->last_sparse = 1;
-        // the matching rows on the tensor cores, when the mode scans there
-        const bool low_tc = mode == 1 && tc_supported(g) && tc_superset(g, topb, db.q_amax) > 0;
-        const bool exact_tc = mode == PV_MODE_EXACT && nq >= PV_EXACT_TC_MIN_NQ &&
-                              tf32_supported(g) && tf32_superset(g, topb, db.q_amax) > 0;
-        if ((low_tc || exact_tc) && db.sparse_bound >= PV_SPARSE_TC_MIN_ROWS) {
-            if (sparse_tc_launch(g, db, topb, db.sparse_bound, exact_tc, d_out, d_cnt, d_trunc,
+        if (sparse_tc) {  // the matching rows on the tensor cores
+            if (sparse_tc_launch(g, db, topb, db.sparse_bound, exact_tc_can, d_out, d_cnt, d_trunc,
                                  ev, errbuf, errlen))
                 return -1;
-            g->last_exact_tc = exact_tc ? 1 : 0;
+            g->last_exact_tc = exact_tc_can ? 1 : 0;
             if (ev) cudaEventRecord(ev[4], g->stream);
             return 0;
         }

@@ -48,13 +48,14 @@ cudaError_t launch_bitmaps_rank(const FvGpuIndex *g, const PredInsn *insns, cons
 // popcnt[qprog[q]] or nrows), tau_out[q] = min(tau_out[q], KO-th key) and
 // unc[q] (a full list's last key, fullmin[q], at or below the answer's end;
 // or, with an estimated bound, fewer than KO keys at or below it).
+// late_counts: the kernel ahead on the stream writes popcnt.
 cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *dcnt,
                                bool reset_cnt, const unsigned long long *fullmin,
                                const unsigned long long *tau, int KO, const int32_t *qprog,
                                const unsigned long long *popcnt, uint64_t nrows, int nq,
                                FvHit *out, uint32_t *out_cnt, uint8_t *trunc,
                                unsigned long long *tau_out, uint8_t *unc, cudaStream_t st,
-                               bool estimated = false);
+                               bool estimated = false, bool late_counts = false);
 
 // ---- exact FP32 scan (scan_f32.cu)
 struct ScanF32Args {
@@ -120,6 +121,8 @@ struct DevBatch {
     bool one_range = false;
     // many programs, all of the form bitmap_rank.cu takes
     bool rank_ok = false;
+    bool one_prog = false;    // P == 1 and every query uses it
+    bool rows_fused = false;  // scan_rows.cu tests the one filter itself
 };
 
 int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &pb,
@@ -143,6 +146,12 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
 int redo_flagged(FvGpuIndex *g, int nq, const float *queries, const PredBatch &pb,
                  uint32_t topb, const uint8_t *unc, FvHit *out, uint32_t *out_cnt,
                  uint8_t *truncated, char *errbuf, size_t errlen);
+// ---- exact scan of a few queries over the rows their filter passes
+// (scan_rows.cu)
+bool scan_rows_fits(int nq, int dpad, uint32_t topb);
+int scan_rows_launch(FvGpuIndex *g, const DevBatch &db, uint32_t topb, FvHit *d_out,
+                     uint32_t *d_cnt, uint8_t *d_trunc, char *errbuf, size_t errlen);
+
 // ---- selective filters (sparse.cu)
 // Filters bounded by at most this many rows take the sparse route: exact
 // distances of the listed rows cost less than a full scan below ~1/16 of

@@ -170,13 +170,14 @@ dense_top32_kernel(const uint64_t *__restrict__ dense, uint64_t dcap, uint32_t *
                    const unsigned long long *__restrict__ popcnt, uint64_t nrows,
                    FvHit *__restrict__ out, uint32_t *__restrict__ out_cnt,
                    uint8_t *__restrict__ trunc, unsigned long long *tau_out,
-                   uint8_t *__restrict__ unc, int estimated) {
+                   uint8_t *__restrict__ unc, int estimated, int late_counts) {
     __shared__ uint64_t lists[DM_THREADS / 32][32 * W];
     // the batch's programs and the bitmap kernel's counts were written two
     // or more kernels back (each kernel of the chain triggers the next only
-    // after its own wait): read them while the kernel ahead finishes
+    // after its own wait): read them while the kernel ahead finishes, unless
+    // that is the one that counts (late_counts)
     long long passing = -1;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && !late_counts) {
         const int pg = qprog[blockIdx.x];
         passing = (long long)(pg >= 0 ? popcnt[pg] : nrows);
     }
@@ -193,13 +194,13 @@ cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *d
                                const unsigned long long *popcnt, uint64_t nrows, int nq,
                                FvHit *out, uint32_t *out_cnt, uint8_t *trunc,
                                unsigned long long *tau_out, uint8_t *unc, cudaStream_t st,
-                               bool estimated) {
+                               bool estimated, bool late_counts) {
     if (KO < 1 || KO > DM_OUT) return cudaErrorInvalidValue;
     if (KO <= 64) {
         auto *kern = KO <= 32 ? dense_top32_kernel<1> : dense_top32_kernel<2>;
         return launch_pdl(kern, dim3(nq), dim3(DM_THREADS), 0, st, dense, dcap, dcnt,
                           reset_cnt ? 1 : 0, fullmin, tau, KO, qprog, popcnt, nrows, out, out_cnt,
-                          trunc, tau_out, unc, estimated ? 1 : 0);
+                          trunc, tau_out, unc, estimated ? 1 : 0, late_counts ? 1 : 0);
     }
     // the stage holds a whole run when it can (runs never exceed dcap)
     const int stage_cap = (int)std::min<uint64_t>(std::max<uint64_t>(dcap, 1), DM_CAP_MAX);
