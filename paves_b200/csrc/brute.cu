@@ -90,6 +90,10 @@ int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &
         if (db.one_prog) {
             const uint64_t b = prog_upper_bound(g, pb.insns.data() + pb.progs[0].insn0,
                                                 pb.progs[0].ninsn, pb.consts.data());
+            db.pass = (double)b / (double)std::max<uint64_t>(1, g->count);
+            if (db.one_range)
+                db.pass = std::min(db.pass, prog_pass_estimate(g, pb.insns.data() + pb.progs[0].insn0,
+                                                               1, pb.consts.data()));
             // (the route holds one key per query and listed row: 128 MB at most)
             if (b <= sparse_limit(g->count) && (uint64_t)nq * b <= (1ull << 24))
                 db.sparse_bound = b;
@@ -240,7 +244,7 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
         if (launch_scan_tc(g, nq, db.q_amax, d_q, d_qprog, s.bitmaps.as<uint32_t>(), bm_words,
                            s.popcnt.as<unsigned long long>(), topb, d_out, d_cnt, d_trunc, ev,
                            errbuf, errlen, db.counts_on_device ? &lz : nullptr, false, nullptr,
-                           bm_launched, bm_done))
+                           bm_launched, bm_done, db.pass))
             return -1;
         if (ev) cudaEventRecord(ev[4], g->stream);
         return 0;
@@ -251,7 +255,7 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
         if (launch_scan_tc(g, nq, db.q_amax, d_q, d_qprog, s.bitmaps.as<uint32_t>(), bm_words,
                            s.popcnt.as<unsigned long long>(), topb, d_out, d_cnt, d_trunc, ev,
                            errbuf, errlen, db.counts_on_device ? &lz : nullptr, true, nullptr,
-                           bm_launched, bm_done))
+                           bm_launched, bm_done, db.pass))
             return -1;
         g->last_exact_tc = 1;
         if (ev) cudaEventRecord(ev[4], g->stream);

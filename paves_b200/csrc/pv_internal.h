@@ -122,6 +122,7 @@ struct DevBatch {
     // many programs, all of the form bitmap_rank.cu takes
     bool rank_ok = false;
     bool one_prog = false;    // P == 1 and every query uses it
+    double pass = 1.0;        // share of the rows its filter passes, at most or estimated
     bool rows_fused = false;  // scan_rows.cu tests the one filter itself
 };
 
@@ -229,10 +230,11 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
                    uint32_t *d_cnt, uint8_t *d_trunc, cudaEvent_t *ev, char *errbuf,
                    size_t errlen, const TcLazy *lz = nullptr, bool tf32 = false,
                    const TcRowSet *rs = nullptr, bool behind_bitmaps = false,
-                   cudaEvent_t prep_done = nullptr);
+                   cudaEvent_t prep_done = nullptr, double pass = 1.0);
 // behind_bitmaps: the last launch on the stream is this batch's bitmap
 // kernel (query prep then runs beside it); prep_done: recorded behind
-// query prep
+// query prep; pass: the share of the rows that the batch's filters let
+// through, as far as it is known
 // Reads and clears the watchdog word of the last tensor-core scan after the
 // stream was synchronized; -1 + errbuf if a bounded wait expired.
 int check_tc_watchdog(FvGpuIndex *g, char *errbuf, size_t errlen);

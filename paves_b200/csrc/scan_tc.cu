@@ -322,7 +322,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
                    const unsigned long long *popcnt, uint32_t topb, FvHit *d_out,
                    uint32_t *d_cnt, uint8_t *d_trunc, cudaEvent_t *ev, char *errbuf,
                    size_t errlen, const TcLazy *lz, bool tf32, const TcRowSet *rs,
-                   bool behind_bitmaps, cudaEvent_t prep_done) {
+                   bool behind_bitmaps, cudaEvent_t prep_done, double pass) {
     const bool fp8 = !tf32 && g->precision == FV_GPU_PREC_FP8;
     const int kind = tf32 ? TCK_TF32 : fp8 ? TCK_FP8 : TCK_BF16;
     const int esz = tck_esz(kind);
@@ -429,8 +429,20 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // 2 to 4 times as long filling their lists behind no bound (100,000 BF16
     // rows, 73 queries: k 2, 25, 100 in 0.106, 0.158, 0.343 ms, seeded 0.043,
     // 0.044, 0.079). Without it every tile gets its own CTA.
-    const bool seed =
-        g->tune_seed != 2 && m * grow * (TC_BN / 32) >= 2 * (uint64_t)rank;
+    // Nor does it pay when lists fill little without a bound: few kept keys
+    // for the merge and few admissions per warp (one tile per CTA, a list's
+    // passing rows p; it keeps min(S, p) and admits about S (1 + ln(p / S))).
+    // The sample and its merge take 15 to 20 us; 1 to 7 queries of 50,000 to
+    // 100,000 rows with k of 1 or 2, or 1.6 % of the rows passing, took 10 to
+    // 20 us more with them.
+    const uint64_t ugrow = std::min<uint64_t>(std::max(1, g->sm_count / qtiles), ntiles_all);
+    const double p = pass * (double)nrows_scan / (double)(ugrow * EPI * R);
+    const double kept = std::min<double>(KP, p);
+    const double admits = p <= KP ? p : KP * (1.0 + log(p / KP));
+    const bool little = kept * ugrow * EPI * R <= 3000.0 &&
+                        admits * std::min(32, qtiles > 1 ? 32 : nq) <= 150.0;
+    const bool seed = g->tune_seed != 2 && !little &&
+                      m * grow * (TC_BN / 32) >= 2 * (uint64_t)rank;
     if (!seed) {
         grow = std::max(1, g->tune_grow > 0 ? g->tune_grow : g->sm_count / qtiles);
         tpc = split(ntiles_all);
