@@ -279,6 +279,100 @@ gather_dist_kernel(const float *__restrict__ vecs, int dpad, const float *__rest
     }
 }
 
+// The same for larger batches: a block takes 64 listed rows x 64 queries,
+// 128 dims at a time in shared memory (all of their 16-byte copies in flight
+// together: the rows are scattered, and a stage of 32 dims at a time waited
+// out four round trips), a thread 4 rows x 4 queries (16 apart: a warp's
+// reads fall on distinct banks and its keys on whole lines), two dims at a time (sub /
+// fma.rn.f32x2). Measured for 64 queries x 10,000 rows of 128 dims: 0.016 ms;
+// the row-per-warp kernel, which spends 5 shuffles per (row, query), 0.032 ms.
+constexpr int GT_T = 64;         // rows and queries per block
+constexpr int GT_D = 128;        // dims per stage
+constexpr int GT_S = GT_D + 4;   // padded stride (floats)
+constexpr int GT_MIN_NQ = 12;    // smaller batches leave most of a tile empty
+constexpr size_t GT_SMEM = (size_t)2 * GT_T * GT_S * 4;
+
+__global__ void __launch_bounds__(256)
+gather_tile_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict__ queries,
+                   int nq, const uint32_t *__restrict__ rowids,
+                   const unsigned long long *__restrict__ count, uint64_t cap,
+                   uint64_t *__restrict__ keys, uint32_t *__restrict__ dcnt) {
+    extern __shared__ __align__(16) float gt_smem[];
+    float *sx = gt_smem, *sq = gt_smem + GT_T * GT_S;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int q0 = blockIdx.y * GT_T;
+    const uint64_t n = min((unsigned long long)cap, *count);
+    if (blockIdx.x == 0 && tid < GT_T && q0 + tid < nq) dcnt[q0 + tid] = (uint32_t)n;
+    // copies: 32 threads along a row's 16-byte pieces, 8 rows at a time
+    const int cr = tid >> 5, cc = (tid & 31) * 4;
+    auto copy = [](float *dst, const float *src, bool in) {  // zeros outside
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(src), "r"(in ? 16 : 0));
+    };
+    for (uint64_t r0 = (uint64_t)blockIdx.x * GT_T; r0 < n; r0 += (uint64_t)gridDim.x * GT_T) {
+        uint64_t acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = 0;
+        uint32_t mine[GT_T / 8];  // this thread's rows
+#pragma unroll
+        for (int u = 0; u < GT_T / 8; u++) {
+            const uint64_t r = r0 + cr + 8 * u;
+            mine[u] = __ldg(rowids + (r < n ? r : r0));
+        }
+        for (int d0 = 0; d0 < dpad; d0 += GT_D) {
+            __syncthreads();  // the previous stage is done with
+            const int c = d0 + cc;
+            const bool in = c < dpad;
+#pragma unroll
+            for (int u = 0; u < GT_T / 8; u++) {
+                const int r = cr + 8 * u;
+                copy(sx + r * GT_S + cc, vecs + (uint64_t)mine[u] * dpad + (in ? c : 0), in);
+                const bool have = in && q0 + r < nq;
+                copy(sq + r * GT_S + cc, queries + (have ? (size_t)(q0 + r) * dpad + c : 0), have);
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            const int dn = min(GT_D, dpad - d0);
+#pragma unroll 4
+            for (int k = 0; k < dn; k += 4) {
+                ulonglong2 x[4], q[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    x[i] = *(const ulonglong2 *)(sx + (tx + 16 * i) * GT_S + k);
+                    q[i] = *(const ulonglong2 *)(sq + (ty + 16 * i) * GT_S + k);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        uint64_t d;
+                        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x[i].x), "l"(q[j].x));
+                        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc[i][j]) : "l"(d));
+                        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x[i].y), "l"(q[j].y));
+                        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc[i][j]) : "l"(d));
+                    }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint64_t r = r0 + tx + 16 * i;
+            if (r >= n) continue;
+            const uint32_t row = __ldg(rowids + r);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int q = q0 + ty + 16 * j;
+                if (q >= nq) continue;
+                const float lo = __uint_as_float((uint32_t)acc[i][j]);
+                const float hi = __uint_as_float((uint32_t)(acc[i][j] >> 32));
+                keys[(uint64_t)q * cap + r] = make_key(lo + hi, row);
+            }
+        }
+    }
+}
+
 // The listed rows in the tensor-core scan's operand layout: compacted row i
 // (i < min(*count, cap)) is index row ids[i] — its operand row (row_bytes,
 // a multiple of 16), norm and fp8 scale; one warp per row, 16-byte copies.
@@ -395,6 +489,21 @@ int sparse_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, uint64_t bound, Fv
     compact_kernel<<<blocks, 256, 0, g->stream>>>(s.bitmaps.as<uint32_t>(), bm_words, g->count,
                                                   ids, d_count, cap);
     PV_CUDA_OK(cudaGetLastError(), errbuf, errlen);
+    if (nq >= GT_MIN_NQ) {
+        const unsigned ty = (unsigned)((nq + GT_T - 1) / GT_T);
+        const unsigned tx = (unsigned)std::max<uint64_t>(
+            1, std::min<uint64_t>((cap + GT_T - 1) / GT_T, std::max(1u, 4u * g->sm_count / ty)));
+        PV_CUDA_OK(raise_smem_limit((const void *)gather_tile_kernel, GT_SMEM), errbuf, errlen);
+        gather_tile_kernel<<<dim3(tx, ty), 256, GT_SMEM, g->stream>>>(g->d_vecs, g->dpad, d_q, nq, ids,
+                                                                d_count, cap, keys, dcnt);
+        PV_CUDA_OK(cudaGetLastError(), errbuf, errlen);
+        g->launches += 3;  // compaction, distances, selection
+        PV_CUDA_OK(launch_dense_merge(keys, cap, dcnt, false, nullptr, nullptr, (int)topb, d_qprog,
+                                      s.popcnt.as<unsigned long long>(), g->count, nq, d_out,
+                                      d_cnt, d_trunc, nullptr, nullptr, g->stream),
+                   errbuf, errlen);
+        return 0;
+    }
     const int qtiles = (nq + GD_QT - 1) / GD_QT;
     const uint64_t bx = std::max<uint64_t>(
         1, std::min<uint64_t>((cap + 63) / 64, std::max(1, 4 * g->sm_count / qtiles)));
