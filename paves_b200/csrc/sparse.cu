@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "pv_internal.h"
+#include "sm100.cuh"
 
 namespace pv {
 
@@ -279,18 +280,21 @@ gather_dist_kernel(const float *__restrict__ vecs, int dpad, const float *__rest
     }
 }
 
-// The same for larger batches: a block takes 64 listed rows x 64 queries,
-// 128 dims at a time in shared memory (all of their 16-byte copies in flight
-// together: the rows are scattered, and a stage of 32 dims at a time waited
-// out four round trips), a thread 4 rows x 4 queries (16 apart: a warp's
-// reads fall on distinct banks and its keys on whole lines), two dims at a time (sub /
-// fma.rn.f32x2). Measured for 64 queries x 10,000 rows of 128 dims: 0.016 ms;
-// the row-per-warp kernel, which spends 5 shuffles per (row, query), 0.032 ms.
+// The same for larger batches of rows up to 128 dims: a block takes 64 listed
+// rows x 64 queries, a thread 4 rows x 4 queries, two queries per packed
+// instruction (sub / fma.rn.f32x2; the queries lie transposed in shared
+// memory, four of a dim in one 16-byte read). Each distance is summed in the
+// row-per-warp kernel's order, so both give the same bits: what lane L sums
+// there, dims 4L .. 4L + 3, is a leaf here, and leaves join in the order of
+// its shuffles (16, 8, 4, 2, 1 lanes apart): bit-reversed, pairs of equal
+// depth added as they complete. Measured for 64 queries x 10,000 rows of 128
+// dims: 0.022 ms; the row-per-warp kernel, which spends 5 shuffles per
+// (row, query), 0.032 ms.
 constexpr int GT_T = 64;         // rows and queries per block
-constexpr int GT_D = 128;        // dims per stage
-constexpr int GT_S = GT_D + 4;   // padded stride (floats)
+constexpr int GT_D = 128;        // dims at most
+constexpr int GT_S = GT_D + 4;   // padded stride of the rows (floats)
 constexpr int GT_MIN_NQ = 12;    // smaller batches leave most of a tile empty
-constexpr size_t GT_SMEM = (size_t)2 * GT_T * GT_S * 4;
+constexpr size_t GT_SMEM = (size_t)(GT_T * GT_S + GT_D * GT_T) * 4;
 
 __global__ void __launch_bounds__(256)
 gather_tile_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict__ queries,
@@ -298,63 +302,98 @@ gather_tile_kernel(const float *__restrict__ vecs, int dpad, const float *__rest
                    const unsigned long long *__restrict__ count, uint64_t cap,
                    uint64_t *__restrict__ keys, uint32_t *__restrict__ dcnt) {
     extern __shared__ __align__(16) float gt_smem[];
-    float *sx = gt_smem, *sq = gt_smem + GT_T * GT_S;
+    float *sx = gt_smem, *sq = gt_smem + GT_T * GT_S;  // [row][dim], [dim][query]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int q0 = blockIdx.y * GT_T;
     const uint64_t n = min((unsigned long long)cap, *count);
     if (blockIdx.x == 0 && tid < GT_T && q0 + tid < nq) dcnt[q0 + tid] = (uint32_t)n;
-    // copies: 32 threads along a row's 16-byte pieces, 8 rows at a time
+    for (int i = tid; i < GT_T * (GT_D / 4); i += 256) {
+        const int r = i & (GT_T - 1), c = (i / GT_T) * 4;
+        const float4 v = q0 + r < nq && c < dpad
+                             ? __ldg((const float4 *)(queries + (size_t)(q0 + r) * dpad + c))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        sq[(c + 0) * GT_T + r] = v.x;
+        sq[(c + 1) * GT_T + r] = v.y;
+        sq[(c + 2) * GT_T + r] = v.z;
+        sq[(c + 3) * GT_T + r] = v.w;
+    }
+    // row copies: 32 threads along a row's 16-byte pieces, 8 rows at a time,
+    // all of a tile's in flight together (the rows are scattered)
     const int cr = tid >> 5, cc = (tid & 31) * 4;
-    auto copy = [](float *dst, const float *src, bool in) {  // zeros outside
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                         (uint32_t)__cvta_generic_to_shared(dst)),
-                     "l"(src), "r"(in ? 16 : 0));
-    };
     for (uint64_t r0 = (uint64_t)blockIdx.x * GT_T; r0 < n; r0 += (uint64_t)gridDim.x * GT_T) {
-        uint64_t acc[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] = 0;
-        uint32_t mine[GT_T / 8];  // this thread's rows
+        __syncthreads();  // the previous tile is done with
 #pragma unroll
         for (int u = 0; u < GT_T / 8; u++) {
             const uint64_t r = r0 + cr + 8 * u;
-            mine[u] = __ldg(rowids + (r < n ? r : r0));
+            const uint32_t row = __ldg(rowids + (r < n ? r : r0));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(sx + (cr + 8 * u) * GT_S + cc)),
+                         "l"(vecs + (uint64_t)row * dpad + (cc < dpad ? cc : 0)),
+                         "r"(cc < dpad ? 16 : 0));  // zeros outside
         }
-        for (int d0 = 0; d0 < dpad; d0 += GT_D) {
-            __syncthreads();  // the previous stage is done with
-            const int c = d0 + cc;
-            const bool in = c < dpad;
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        // [row][pair of queries] packed
+        uint64_t s0[4][2], s1[4][2], s2[4][2], sum[4][2];
+        auto leaf = [&](int l, uint64_t (&acc)[4][2]) {
+            float4 x[4];
+            ulonglong2 q[4];
 #pragma unroll
-            for (int u = 0; u < GT_T / 8; u++) {
-                const int r = cr + 8 * u;
-                copy(sx + r * GT_S + cc, vecs + (uint64_t)mine[u] * dpad + (in ? c : 0), in);
-                const bool have = in && q0 + r < nq;
-                copy(sq + r * GT_S + cc, queries + (have ? (size_t)(q0 + r) * dpad + c : 0), have);
+            for (int i = 0; i < 4; i++) {
+                x[i] = *(const float4 *)(sx + (tx + 16 * i) * GT_S + 4 * l);
+                q[i] = *(const ulonglong2 *)(sq + (4 * l + i) * GT_T + 4 * ty);
             }
-            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            const int dn = min(GT_D, dpad - d0);
-#pragma unroll 4
-            for (int k = 0; k < dn; k += 4) {
-                ulonglong2 x[4], q[4];
+#pragma unroll
+            for (int d = 0; d < 4; d++)
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    x[i] = *(const ulonglong2 *)(sx + (tx + 16 * i) * GT_S + k);
-                    q[i] = *(const ulonglong2 *)(sq + (ty + 16 * i) * GT_S + k);
-                }
+                    const float xv = d == 0 ? x[i].x : d == 1 ? x[i].y : d == 2 ? x[i].z : x[i].w;
+                    const uint64_t x2 = sm100::f2_pack(xv, xv);
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        uint64_t d;
-                        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x[i].x), "l"(q[j].x));
-                        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc[i][j]) : "l"(d));
-                        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x[i].y), "l"(q[j].y));
-                        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc[i][j]) : "l"(d));
+                    for (int j = 0; j < 2; j++) {
+                        uint64_t t;
+                        asm("sub.rn.f32x2 %0, %1, %2;"
+                            : "=l"(t) : "l"(x2), "l"(j ? q[d].y : q[d].x));
+                        acc[i][j] = d == 0 ? sm100::f2_fma(t, t, 0ull)
+                                           : sm100::f2_fma(t, t, acc[i][j]);
                     }
+                }
+        };
+        auto add = [](uint64_t (&d)[4][2], const uint64_t (&a)[4][2], const uint64_t (&b)[4][2]) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) d[i][j] = sm100::f2_add(a[i][j], b[i][j]);
+        };
+#pragma unroll 1
+        for (int u = 0; u < 8; u++) {
+            const int b = ((u & 1) << 2) | (u & 2) | (u >> 2);  // the leaves b + 0, 16, 8, 24
+            uint64_t t[4][2], v[4][2];
+            leaf(b, t);
+            leaf(b + 16, v);
+            add(sum, t, v);
+            leaf(b + 8, t);
+            leaf(b + 24, v);
+            add(t, t, v);
+            add(sum, sum, t);
+            if (!(u & 1)) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) s0[i >> 1][i & 1] = sum[i >> 1][i & 1];
+                continue;
             }
+            add(sum, s0, sum);
+            if (!(u & 2)) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) s1[i >> 1][i & 1] = sum[i >> 1][i & 1];
+                continue;
+            }
+            add(sum, s1, sum);
+            if (!(u & 4)) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) s2[i >> 1][i & 1] = sum[i >> 1][i & 1];
+                continue;
+            }
+            add(sum, s2, sum);
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -362,12 +401,13 @@ gather_tile_kernel(const float *__restrict__ vecs, int dpad, const float *__rest
             if (r >= n) continue;
             const uint32_t row = __ldg(rowids + r);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int q = q0 + ty + 16 * j;
-                if (q >= nq) continue;
-                const float lo = __uint_as_float((uint32_t)acc[i][j]);
-                const float hi = __uint_as_float((uint32_t)(acc[i][j] >> 32));
-                keys[(uint64_t)q * cap + r] = make_key(lo + hi, row);
+            for (int j = 0; j < 2; j++) {
+                uint32_t lo, hi;
+                sm100::f2_unpack(sum[i][j], lo, hi);
+                const int q = q0 + 4 * ty + 2 * j;
+                if (q < nq) keys[(uint64_t)q * cap + r] = make_key(__uint_as_float(lo), row);
+                if (q + 1 < nq)
+                    keys[(uint64_t)(q + 1) * cap + r] = make_key(__uint_as_float(hi), row);
             }
         }
     }
@@ -489,7 +529,7 @@ int sparse_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, uint64_t bound, Fv
     compact_kernel<<<blocks, 256, 0, g->stream>>>(s.bitmaps.as<uint32_t>(), bm_words, g->count,
                                                   ids, d_count, cap);
     PV_CUDA_OK(cudaGetLastError(), errbuf, errlen);
-    if (nq >= GT_MIN_NQ) {
+    if (nq >= GT_MIN_NQ && g->dpad <= GT_D) {
         const unsigned ty = (unsigned)((nq + GT_T - 1) / GT_T);
         const unsigned tx = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((cap + GT_T - 1) / GT_T, std::max(1u, 4u * g->sm_count / ty)));

@@ -33,3 +33,22 @@ def test_listed_rows_match_oracle(nq, dim, rows, k):
         assert cnt[i] == m == min(k, rows) and trunc[i] == (rows > k)
         assert np.array_equal(ids[i, :m], o_ids[i, :m].astype(np.uint64))
         assert np.array_equal(dists[i, :m], o_d[i, :m])
+
+
+@pytest.mark.parametrize("dim", [128, 100, 36])
+def test_same_bits_as_the_row_per_warp_kernel(dim):
+    # real-valued rows: 12 queries take the tiles, each one alone does not
+    n, rows, k = 30_000, 900, 64
+    rng = np.random.default_rng(dim)
+    x = rng.standard_normal((n, dim)).astype(np.float32)
+    cols = np.full((1, n), 5.0)
+    cols[0, rng.choice(n, rows, replace=False)] = 1.0
+    q = rng.standard_normal((12, dim)).astype(np.float32)
+    gi = GpuIndex(x, cols, device=0, precision=_lib.FV_GPU_PREC_FP32)
+    f = Cmp(0, "<", 2.0)
+    ids, dists, cnt, _ = gi.brute_batch(q, [f] * 12, k)
+    for s in (slice(0, 9), slice(3, 12)):  # nine queries: gather_dist_kernel
+        i2, d2, c2, _ = gi.brute_batch(q[s], [f] * 9, k)
+        assert np.array_equal(ids[s], i2) and np.array_equal(cnt[s], c2)
+        assert np.array_equal(dists[s].view(np.uint32), d2.view(np.uint32))
+    gi.close()
