@@ -69,9 +69,11 @@ __device__ __forceinline__ float rs_butterfly(float (&p)[32], int lane) {
 
 template <int QT, int DCH, int W>
 __global__ void __launch_bounds__(32 * RS_WARPS, 2) scan_rows_kernel(RowScanArgs a) {
-    constexpr int R = 32 / QT;  // rows read together
+    constexpr int R = 32 / QT;  // rows of a butterfly
+    // butterflies whose rows are read together (with 8 queries one has only four)
+    constexpr int NB = QT == 8 && W == 1 ? 2 : 1;
     __shared__ uint32_t s_queue[RS_WARPS][64];
-    __shared__ uint64_t s_lists[RS_WARPS][32 * W];
+    __shared__ uint64_t s_new[RS_WARPS][QT][64];  // keys not yet folded in
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -95,50 +97,93 @@ __global__ void __launch_bounds__(32 * RS_WARPS, 2) scan_rows_kernel(RowScanArgs
     const int my_r = lane / QT, my_q = lane % QT;
     const int my_pg = my_q < a.nq && a.bitmaps ? a.qprog[my_q] : -1;
     unsigned head = 0, tail = 0;
-
-    auto take = [&](int cnt) {  // the queue's first cnt <= R rows
-        float p[32];
+    // this lane's query (the same in all lanes of the query): keys waiting,
+    // and the K-th of its list
+    int fill = 0;
+    uint64_t thr = KEY_MAX;
+    uint64_t *mynew = s_new[warp][my_q];
+    unsigned qlanes = 0;
 #pragma unroll
-        for (int r = 0; r < R; r++) {
+    for (int r = 0; r < R; r++) qlanes |= 1u << (r * QT);
+    qlanes <<= my_q;
+    auto ballot_of = [&](bool p) { return __ballot_sync(0xffffffffu, p) & qlanes; };
+    // folds the waiting keys of every query that has more than `most`
+    auto fold = [&](int most) {
+        __syncwarp();
+#pragma unroll
+        for (int qq = 0; qq < QT; qq++) {
+            const int n = __shfl_sync(0xffffffffu, fill, qq);
+            if (n <= most) continue;
+            for (int b = 0; b < n; b += 32) {
+                const uint64_t k = b + lane < n ? s_new[warp][qq][b + lane] : KEY_MAX;
+                warp_fold32<W>(best[qq], warp_sort32(k, lane, true), lane);
+            }
+            const uint64_t last = W == 1 || a.K <= 32 ? best[qq][0] : best[qq][W - 1];
+            const uint64_t kth = __shfl_sync(0xffffffffu, last, (a.K - 1) & 31);
+            if (my_q == qq) {
+                thr = kth;
+                fill = 0;
+            }
+        }
+        __syncwarp();
+    };
+
+    auto take = [&](int cnt) {  // the queue's first cnt <= R * NB rows
+        float4 x[NB][NB > 1 ? R : 1][DCH];  // NB > 1: all rows' reads first
+        auto read = [&](int r, float4 (&v)[DCH]) {
             const uint32_t row = queue[(head + (r < cnt ? r : 0)) & 63];
-            float4 x[DCH];
 #pragma unroll
             for (int c = 0; c < DCH; c++) {
                 const int j = c * 128 + lane * 4;
-                x[c] = j < a.dpad
+                v[c] = j < a.dpad
                            ? __ldg((const float4 *)(a.vecs + (uint64_t)row * a.dpad + j))
                            : make_float4(0.f, 0.f, 0.f, 0.f);
             }
+        };
+        if (NB > 1) {
 #pragma unroll
-            for (int qq = 0; qq < QT; qq++) {
-                float s = 0.f;
+            for (int b = 0; b < NB; b++)
 #pragma unroll
-                for (int c = 0; c < DCH; c++) {
-                    const float d0 = x[c].x - qr[qq][c].x, d1 = x[c].y - qr[qq][c].y;
-                    const float d2 = x[c].z - qr[qq][c].z, d3 = x[c].w - qr[qq][c].w;
-                    s = fmaf(d0, d0, s);
-                    s = fmaf(d1, d1, s);
-                    s = fmaf(d2, d2, s);
-                    s = fmaf(d3, d3, s);
-                }
-                p[r * QT + qq] = s;
-            }
+                for (int r = 0; r < R; r++) read(b * R + r, x[b][NB > 1 ? r : 0]);
         }
-        const float dist = rs_butterfly(p, lane);
-        const uint32_t row = queue[(head + (my_r < cnt ? my_r : 0)) & 63];
-        bool ok = my_r < cnt && my_q < a.nq;
-        // queries with filters of their own: the row passes one of them
-        if (ok && !a.shared_prog && my_pg >= 0)
-            ok = (__ldg(a.bitmaps + (uint64_t)my_pg * a.bm_words + (row >> 5)) >> (row & 31)) & 1u;
-        const uint64_t key = ok ? make_key(dist, row) : KEY_MAX;
 #pragma unroll
-        for (int qq = 0; qq < QT; qq++) {
-            const uint64_t k = QT == 1 || my_q == qq ? key : KEY_MAX;
-            const int kh = (a.K - 1) >> 5;
-            const uint64_t last = W == 1 || kh == 0 ? best[qq][0] : best[qq][W - 1];
-            const uint64_t worst = __shfl_sync(0xffffffffu, last, (a.K - 1) & 31);
-            if (__any_sync(0xffffffffu, k < worst))
-                warp_fold32<W>(best[qq], warp_sort32(k, lane, true), lane);
+        for (int b = 0; b < NB; b++) {
+            if (b * R >= cnt) break;
+            float p[32];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if (NB == 1) read(r, x[0][0]);
+                const float4(&v)[DCH] = x[b][NB > 1 ? r : 0];
+#pragma unroll
+                for (int qq = 0; qq < QT; qq++) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int c = 0; c < DCH; c++) {
+                        const float d0 = v[c].x - qr[qq][c].x, d1 = v[c].y - qr[qq][c].y;
+                        const float d2 = v[c].z - qr[qq][c].z, d3 = v[c].w - qr[qq][c].w;
+                        s = fmaf(d0, d0, s);
+                        s = fmaf(d1, d1, s);
+                        s = fmaf(d2, d2, s);
+                        s = fmaf(d3, d3, s);
+                    }
+                    p[r * QT + qq] = s;
+                }
+            }
+            const float dist = rs_butterfly(p, lane);
+            const int at = b * R + my_r;
+            const uint32_t row = queue[(head + (at < cnt ? at : 0)) & 63];
+            bool ok = at < cnt && my_q < a.nq;
+            // queries with filters of their own: the row passes one of them
+            if (ok && !a.shared_prog && my_pg >= 0)
+                ok = (__ldg(a.bitmaps + (uint64_t)my_pg * a.bm_words + (row >> 5)) >> (row & 31)) & 1u;
+            // keys better than the list's K-th wait in shared memory until a
+            // batch of them is worth a sort (8 queries get 4 keys each here)
+            const uint64_t key = make_key(dist, row);
+            const bool want = ok && key < thr;
+            const unsigned same = ballot_of(want);
+            if (want) mynew[fill + __popc(same & lt)] = key;
+            fill += __popc(same);
+            if (__any_sync(0xffffffffu, fill > 64 - R)) fold(64 - R);
         }
     };
 
@@ -210,54 +255,51 @@ __global__ void __launch_bounds__(32 * RS_WARPS, 2) scan_rows_kernel(RowScanArgs
                 queue[(tail + __popc(word & lt)) & 63] = (uint32_t)((ws + j) * 32 + lane);
             tail += __popc(word);
             __syncwarp();
-            while (tail - head >= (unsigned)R) {
-                take(R);
-                head += R;
+            while (tail - head >= (unsigned)(R * NB)) {
+                take(R * NB);
+                head += R * NB;
             }
             __syncwarp();
         }
     }
     if (tail != head) take((int)(tail - head));
+    fold(0);
 
     if (a.fused) {
         passing = __reduce_add_sync(0xffffffffu, passing);
         if (lane == 0 && passing) atomicAdd(a.popcnt, (unsigned long long)passing);
     }
-    // the block's warps fold pairwise into warp 0, query by query, and its K
-    // best keys join the query's run
+    // the warps' lists meet in shared memory (the waiting keys' place); each
+    // query's are folded by a warp of its own, and its K best keys join the
+    // query's run
 #pragma unroll
-    for (int qq = 0; qq < QT; qq++) {
-        if (qq >= a.nq) break;
-        __syncthreads();
+    for (int qq = 0; qq < QT; qq++)
 #pragma unroll
-        for (int h = 0; h < W; h++) s_lists[warp][h * 32 + lane] = best[qq][h];
-        for (int step = 1; step < RS_WARPS; step <<= 1) {
-            __syncthreads();
-            if ((warp & (2 * step - 1)) == 0) {
+        for (int h = 0; h < W; h++) s_new[warp][qq][h * 32 + lane] = best[qq][h];
+    __syncthreads();
+    if (warp < a.nq) {
+        const int qq = warp;
+        uint64_t all[W];
 #pragma unroll
-                for (int h = 0; h < W; h++) {
-                    const uint64_t d = s_lists[warp + step][h * 32 + 31 - lane];
-                    const uint64_t worst = __shfl_sync(0xffffffffu, best[qq][W - 1], 31);
-                    if (__any_sync(0xffffffffu, d < worst)) warp_fold32<W>(best[qq], d, lane);
-                }
+        for (int h = 0; h < W; h++) all[h] = s_new[0][qq][h * 32 + lane];
+        for (int o = 1; o < RS_WARPS; o++)
 #pragma unroll
-                for (int h = 0; h < W; h++) s_lists[warp][h * 32 + lane] = best[qq][h];
+            for (int h = 0; h < W; h++) {
+                const uint64_t d = s_new[o][qq][h * 32 + 31 - lane];
+                const uint64_t worst = __shfl_sync(0xffffffffu, all[W - 1], 31);
+                if (__any_sync(0xffffffffu, d < worst)) warp_fold32<W>(all, d, lane);
             }
-        }
-        if (warp == 0) {
-            int n = 0;
+        int n = 0;
 #pragma unroll
-            for (int h = 0; h < W; h++)
-                n += __popc(__ballot_sync(0xffffffffu,
-                                          h * 32 + lane < a.K && best[qq][h] != KEY_MAX));
-            uint32_t at = 0;
-            if (lane == 0 && n) at = atomicAdd(a.dcnt + qq, (uint32_t)n);
-            at = __shfl_sync(0xffffffffu, at, 0);
+        for (int h = 0; h < W; h++)
+            n += __popc(
+                __ballot_sync(0xffffffffu, h * 32 + lane < a.K && all[h] != KEY_MAX));
+        uint32_t at = 0;
+        if (lane == 0 && n) at = atomicAdd(a.dcnt + qq, (uint32_t)n);
+        at = __shfl_sync(0xffffffffu, at, 0);
 #pragma unroll
-            for (int h = 0; h < W; h++)
-                if (h * 32 + lane < n)
-                    a.dense[(uint64_t)qq * a.dcap + at + h * 32 + lane] = best[qq][h];
-        }
+        for (int h = 0; h < W; h++)
+            if (h * 32 + lane < n) a.dense[(uint64_t)qq * a.dcap + at + h * 32 + lane] = all[h];
     }
 }
 
