@@ -430,7 +430,7 @@ int pv_tc_wide_superset(FvGpuIndex *g, int on);
  * "wait expired" in errbuf; the index stays usable. -1: bad value. */
 int pv_tc_timeout(FvGpuIndex *g, uint64_t ns);
 /* Exact-mode batches (FP32 uploads through fv_gpu_brute_batch, or
- * PV_MODE_EXACT) of 16+ queries over rows of at most 128 dims scan on the
+ * PV_MODE_EXACT) of 16+ queries over rows of at most 512 dims scan on the
  * tensor cores: the f32 rows read as TF32, the top 4 x topb (at least 16;
  * topb itself on integer rows, where the distances are exact) re-ranked in
  * FP32, and each query's answer certified by an error bound of the scan

@@ -171,7 +171,10 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     if (ev) cudaEventRecord(ev[0], g->stream);
     const bool sparse_route = db.sparse_bound > 0 && !db.counts_on_device && topb <= 1024;
     const bool low_tc_can = mode == 1 && tc_supported(g) && tc_superset(g, topb, db.q_amax) > 0;
-    const bool exact_tc_can = mode == PV_MODE_EXACT && nq >= PV_EXACT_TC_MIN_NQ &&
+    // exact answers from the f32 rows: the exact mode, and low-precision
+    // uploads whose rows are too wide for their own scan
+    const bool exact_mode = mode == PV_MODE_EXACT || (mode == 1 && !tc_supported(g));
+    const bool exact_tc_can = exact_mode && nq >= PV_EXACT_TC_MIN_NQ &&
                               tf32_supported(g) && tf32_superset(g, topb, db.q_amax) > 0;
     const bool sparse_tc = sparse_route && (low_tc_can || exact_tc_can) &&
                            db.sparse_bound >= PV_SPARSE_TC_MIN_ROWS;

@@ -55,7 +55,7 @@ scan_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte alignment for the swizzled operand tiles
     unsigned char *base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const TcSmem sm = tc_carve(base, a.kblocks, a.NS, a.KP, EPI);
+    const TcSmem sm = tc_carve(base, a.kblocks, a.NS, a.KP, EPI, KIND == TCK_TF32 && a.qstream);
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int warp = threadIdx.x >> 5;
@@ -119,6 +119,7 @@ __global__ void query_prep_kernel(const float *__restrict__ q, int nq, int dpad,
 // (up to TC_MAX_SUPERSET, row stride S); keeps the best topb by (dist, id).
 // One CTA (8 warps) per query: 8 lanes per candidate, 32 candidates in
 // flight, then a bitonic sort of the keys in shared memory.
+template <int ORDER>
 __global__ void __launch_bounds__(256)
 rerank_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict__ queries,
               const FvHit *__restrict__ cand, const uint32_t *__restrict__ cand_cnt, int S,
@@ -129,7 +130,7 @@ rerank_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict_
     __shared__ uint64_t keys[TC_MAX_SUPERSET];
     pdl_wait();
     pdl_trigger();
-    rerank_query<256>(blockIdx.x, keys, vecs, dpad, queries, cand, cand_cnt, S, topb, qprog, popcnt,
+    rerank_query<256, ORDER>(blockIdx.x, keys, vecs, dpad, queries, cand, cand_cnt, S, topb, qprog, popcnt,
                       nrows, out, out_cnt, trunc, cert);
 }
 
@@ -270,10 +271,10 @@ int tf32_superset(const FvGpuIndex *g, uint32_t topb, float q_amax) {
     return s <= TC_MAX_SUPERSET ? s : 0;
 }
 
-// Rows of at most 128 f32 (the query tile stays 64 KB of shared memory),
+// Rows of at most 512 f32 (beyond 128 the query tile streams with the rows),
 // at least 8 row tiles, and not switched off for the index.
 bool tf32_supported(const FvGpuIndex *g) {
-    return g->exact_tc && g->d_norm32 && g->dpad <= 128 && g->count >= 8 * (uint64_t)TC_BN;
+    return g->exact_tc && g->d_norm32 && g->dpad <= 512 && g->count >= 8 * (uint64_t)TC_BN;
 }
 
 bool tc_supported(const FvGpuIndex *g) {
@@ -282,8 +283,10 @@ bool tc_supported(const FvGpuIndex *g) {
     return row_bytes <= 512;  // query tile <= 64 KB of shared memory
 }
 
+// (kinds other than TF32 have at most 4 K-blocks)
+static bool tc_qstream(int kblocks) { return kblocks > 4; }
 static size_t tc_smem(int kblocks, int NS, int KP, int EPI) {
-    return tc_smem_bytes(kblocks, NS, KP, EPI);
+    return tc_smem_bytes(kblocks, NS, KP, EPI, tc_qstream(kblocks));
 }
 
 bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns) {
@@ -360,7 +363,8 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const size_t smem_pref = 222 * 1024;
     // stages: up to 128 KB of rows in flight
     const int ns0 = std::min(TC_MAX_STAGES, std::max(
-        2, (int)(128 * 1024 / ((size_t)std::min(kblocks, TC_KBS) * TC_BOX))));
+        2, (int)(128 * 1024 / ((size_t)std::min(kblocks, TC_KBS) * TC_BOX *
+                                         (tc_qstream(kblocks) ? 2 : 1)))));
     int EPI = 0, NS = 0;
     for (int e = kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 ? 3 : 2; e >= 1 && !EPI; e--) {
         const int KPe = std::min(S, tc_list_cap(e));
@@ -537,6 +541,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     a.bq = bq;
     a.push_tau = KP == S ? 1 : 0;
     a.NS = NS;
+    a.qstream = tc_qstream(kblocks) ? 1 : 0;
     a.xnorm = rs ? rs->norms : tf32 ? g->d_norm32 : g->d_norm;
     a.xscale = fp8 ? (rs ? rs->scales : g->d_vscale) : nullptr;
     a.rowids = rs ? rs->rowids : nullptr;
@@ -650,7 +655,13 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
             cert.dim = g->dpad;
             cert.unc = d_unc;
         }
-        PV_CUDA_OK(launch_pdl(rerank_kernel, dim3(nq), dim3(256), 0, g->stream, g->d_vecs,
+        auto *rerank = rerank_kernel<RR_LANES8>;
+        if (tf32 && g->dpad > 128) {
+            ScanPlan pl;
+            rerank = !rs && plan_scan_f32t(g->count, g->dpad, nq, (int)topb, g->sm_count, pl)
+                         ? rerank_kernel<RR_THREAD> : rerank_kernel<RR_WARP>;
+        }
+        PV_CUDA_OK(launch_pdl(rerank, dim3(nq), dim3(256), 0, g->stream, g->d_vecs,
                               g->dpad, d_q, cand, ccnt, S, topb, d_qprog, popcnt, g->count, d_out,
                               d_cnt, d_trunc, cert),
                    errbuf, errlen);

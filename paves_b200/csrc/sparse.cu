@@ -530,10 +530,12 @@ int sparse_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, uint64_t bound, Fv
                                                   ids, d_count, cap);
     PV_CUDA_OK(cudaGetLastError(), errbuf, errlen);
     const unsigned ty = (unsigned)((nq + GT_T - 1) / GT_T);
-    // (tiles for half the SMs at least: 276 queries x 394 rows make 35, and
-    // took 3 us longer than the row-per-warp kernel's many small blocks)
+    // (tiles for half the SMs at least, by the rows expected: 276 queries x
+    // 394 rows make 35, and took 3 us longer than the row-per-warp kernel's
+    // many small blocks)
+    const uint64_t expect = std::min<uint64_t>(cap, (uint64_t)(db.pass * (double)g->count) + 1);
     if (nq >= GT_MIN_NQ && g->dpad <= GT_D &&
-        (cap + GT_T - 1) / GT_T * ty >= (uint64_t)g->sm_count / 2) {
+        (expect + GT_T - 1) / GT_T * ty >= (uint64_t)g->sm_count / 2) {
         const unsigned tx = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((cap + GT_T - 1) / GT_T, std::max(1u, 4u * g->sm_count / ty)));
         PV_CUDA_OK(raise_smem_limit((const void *)gather_tile_kernel, GT_SMEM), errbuf, errlen);

@@ -90,6 +90,10 @@ struct TcArgs {
     // every seed_group 32-row chunks instead of its best KP keys
     int seed_group = 0;
     int NS;             // pipeline stages
+    // TF32 rows beyond 128 dims: the query tile (64 KB and more) does not stay
+    // in shared memory; each stage brings the queries' K-blocks beside the
+    // rows' (from L2: they are the same for every tile)
+    int qstream = 0;
     const float *__restrict__ xnorm;   // [rows padded to 128]
     const float *__restrict__ xscale;  // fp8: per-row scale, else null
     const float *__restrict__ qnorm;   // [nqpad]
@@ -144,12 +148,13 @@ struct TcSmem {
 };
 
 __device__ __forceinline__ TcSmem tc_carve(unsigned char *base, int KBt, int NS, int KPcap,
-                                           int EPI) {
+                                           int EPI, bool qstream = false) {
     TcSmem m;
     m.sQ = base;                                       // KBt boxes
-    m.sX = m.sQ + (size_t)KBt * TC_BOX;                // NS stages
-    // a stage holds one K-chunk of a row tile: min(TC_KBS, KBt) boxes
-    m.SB = (size_t)(KBt < TC_KBS ? KBt : TC_KBS) * TC_BOX;
+    m.sX = m.sQ + (qstream ? 0 : (size_t)KBt * TC_BOX);  // NS stages
+    // a stage holds one K-chunk of a row tile: min(TC_KBS, KBt) boxes (and
+    // of the query tile: as many again)
+    m.SB = (size_t)(KBt < TC_KBS ? KBt : TC_KBS) * TC_BOX * (qstream ? 2 : 1);
     // per (query, part) lists [KP][128*EPI]
     m.lists = (uint64_t *)(m.sX + (size_t)NS * m.SB);
     // row norms (and fp8 scales, compacted-set row ids) of a tile, TC_NR
@@ -167,9 +172,9 @@ __device__ __forceinline__ TcSmem tc_carve(unsigned char *base, int KBt, int NS,
     return m;
 }
 
-inline size_t tc_smem_bytes(int kblocks, int NS, int KPcap, int EPI) {
-    return 1024 + (size_t)kblocks * TC_BOX +
-           (size_t)NS * (kblocks < TC_KBS ? kblocks : TC_KBS) * TC_BOX +
+inline size_t tc_smem_bytes(int kblocks, int NS, int KPcap, int EPI, bool qstream = false) {
+    return 1024 + (qstream ? 0 : (size_t)kblocks * TC_BOX) +
+           (size_t)NS * (kblocks < TC_KBS ? kblocks : TC_KBS) * TC_BOX * (qstream ? 2 : 1) +
            (size_t)TC_BM * EPI * KPcap * 8 + (size_t)TC_NR * TC_NSLOT_F * 4 + (size_t)(2 * NS + 2 * TC_NACC + 2 + 2 * TC_NR) * 8;
 }
 
@@ -226,6 +231,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
     uint64_t *full = sm.full, *empty = sm.empty, *tfull = sm.tfull, *tempty = sm.tempty;
     uint64_t *qbar = sm.qbar, *done = sm.done, *nfull = sm.nfull, *nempty = sm.nempty;
     constexpr bool FP8 = KIND == TCK_FP8;
+    const bool qstream = KIND == TCK_TF32 && a.qstream;
     constexpr int BOXE = TC_KB_BYTES / tck_esz(KIND);  // elements of K per box
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // this CTA's tiles: tile0 + t * tile_step, t < ntiles
@@ -249,10 +255,12 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
         if (lane == 0) {
             prefetch_tmap(&tmX);
             prefetch_tmap(&tmQ);
-            mbar_arrive_expect_tx(qbar, (uint32_t)KBt * TC_BOX);
-            for (int kb = 0; kb < KBt; kb++)
-                tma_load_2d(sQ + (size_t)kb * TC_BOX, &tmQ, kb * BOXE,
-                            qtile * TC_BM, qbar);
+            if (!qstream) {
+                mbar_arrive_expect_tx(qbar, (uint32_t)KBt * TC_BOX);
+                for (int kb = 0; kb < KBt; kb++)
+                    tma_load_2d(sQ + (size_t)kb * TC_BOX, &tmQ, kb * BOXE,
+                                qtile * TC_BM, qbar);
+            }
             const uint32_t nbytes = ((FP8 ? 2 : 1) + (a.rowids ? 1 : 0)) * TC_BN * 4;
             uint64_t it = it0, nt = T0;  // stages and norm slots issued (running)
             bool ok = true;
@@ -282,10 +290,14 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                     const uint32_t ph = (uint32_t)((it / NS) & 1);
                     if (!mbar_wait(&empty[s], ph ^ 1, deadline, abort_flag)) { ok = false; break; }
                     const int nkb = min(TC_KBS, KBt - kc * TC_KBS);
-                    mbar_arrive_expect_tx(&full[s], (uint32_t)nkb * TC_BOX);
+                    mbar_arrive_expect_tx(&full[s], (uint32_t)nkb * TC_BOX * (qstream ? 2 : 1));
                     for (int kb = 0; kb < nkb; kb++)
                         tma_load_2d(sX + (size_t)s * SB + (size_t)kb * TC_BOX, &tmX,
                                     (kc * TC_KBS + kb) * BOXE, y, &full[s]);
+                    if (qstream)
+                        for (int kb = 0; kb < nkb; kb++)
+                            tma_load_2d(sX + (size_t)s * SB + (size_t)(TC_KBS + kb) * TC_BOX, &tmQ,
+                                        (kc * TC_KBS + kb) * BOXE, qtile * TC_BM, &full[s]);
                 }
                 if (a.trace && blockIdx.x == 0 && t < (uint64_t)a.trace_tiles)
                     a.trace[t * 4 + 0] = globaltimer();
@@ -303,7 +315,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
             const uint64_t nfirst = nt > T0 + TC_NR ? nt - TC_NR : T0;
             for (uint64_t j = nfirst; j < nt; j++)
                 mbar_wait(&nfull[j % TC_NR], (uint32_t)((j / TC_NR) & 1), d2, &zero);
-            mbar_wait(qbar, qph, d2, &zero);
+            if (!qstream) mbar_wait(qbar, qph, d2, &zero);
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
@@ -311,7 +323,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
             const uint32_t idesc = FP8 ? idesc_make(FMT_E4M3, FMT_E4M3, TC_BM, TC_BN)
                                    : KIND == TCK_TF32 ? idesc_make(FMT_TF32, FMT_TF32, TC_BM, TC_BN)
                                                       : idesc_make(FMT_BF16, FMT_BF16, TC_BM, TC_BN);
-            bool ok = mbar_wait(qbar, qph, deadline, abort_flag);
+            bool ok = qstream || mbar_wait(qbar, qph, deadline, abort_flag);
             uint64_t it = it0;
             for (uint64_t t = 0; t < ntiles && ok; t++) {
                 const uint64_t T = T0 + t;
@@ -327,7 +339,9 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                     tc_fence_after();
                     const int nkb = min(TC_KBS, KBt - kc * TC_KBS);
                     for (int kb = 0; kb < nkb; kb++) {
-                        const uint64_t ad = desc_sw128(sQ + (size_t)(kc * TC_KBS + kb) * TC_BOX);
+                        const uint64_t ad = desc_sw128(
+                            qstream ? sX + (size_t)s * SB + (size_t)(TC_KBS + kb) * TC_BOX
+                                    : sQ + (size_t)(kc * TC_KBS + kb) * TC_BOX);
                         const uint64_t bd = desc_sw128(sX + (size_t)s * SB + (size_t)kb * TC_BOX);
 #pragma unroll
                         for (int kk = 0; kk < 4; kk++)  // 4 x 32 bytes of K per block
@@ -786,10 +800,18 @@ struct RerankCert {
     uint8_t *unc = nullptr;        // [nq] set to 1 when not certified
 };
 
+// Orders of the exact distance's sum. Rows up to 128 dims: 8 lanes a
+// candidate (RR_LANES8). Wider rows reach the re-rank only on batches that
+// the CUDA-core scans answered before, and keep those kernels' sums bit for
+// bit, so near ties order as they do there: the warp's of scan_f32.cu and of
+// a selective filter's listed rows (RR_WARP), or the thread's of scan_f32t.cu,
+// even and odd dims apart (RR_THREAD).
+constexpr int RR_LANES8 = 0, RR_WARP = 1, RR_THREAD = 2;
+
 // One query's re-rank by the block's NT threads (8 lanes per candidate,
 // NT / 8 in flight); keys: TC_MAX_SUPERSET slots of shared memory. Ends
 // with the block synchronized.
-template <int NT>
+template <int NT, int ORDER = RR_LANES8>
 __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float *__restrict__ vecs,
                                              int dpad, const float *__restrict__ queries,
                                              const FvHit *__restrict__ cand,
@@ -806,7 +828,61 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
     int n = ncand;
     if (n > S) n = S;
     const float *qv = queries + (size_t)q * dpad;
-    for (int base = 0; base < n; base += NT / 8) {
+    if (ORDER == RR_WARP) {
+        const int lane = tid & 31, warp = tid >> 5;
+        constexpr int U = 4;  // candidates of a warp in flight
+        for (int base = warp * U; base < n; base += NT / 32 * U) {
+            float s[U];
+            uint32_t row[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                row[u] = (uint32_t)cand[(size_t)q * S + min(base + u, n - 1)].node;
+                s[u] = 0.f;
+            }
+            for (int k = lane * 4; k < dpad; k += 128) {
+                const float4 w = __ldg((const float4 *)(qv + k));
+                float4 v[U];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    v[u] = __ldg((const float4 *)(vecs + (size_t)row[u] * dpad + k));
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const float d0 = v[u].x - w.x, d1 = v[u].y - w.y, d2 = v[u].z - w.z,
+                                d3 = v[u].w - w.w;
+                    s[u] = fmaf(d0, d0, s[u]);
+                    s[u] = fmaf(d1, d1, s[u]);
+                    s[u] = fmaf(d2, d2, s[u]);
+                    s[u] = fmaf(d3, d3, s[u]);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int u = 0; u < U; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+            if (lane == 0)
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (base + u < n) keys[base + u] = make_key(s[u], row[u]);
+        }
+    }
+    if (ORDER == RR_THREAD)
+        for (int j = tid; j < n; j += NT) {
+            const uint32_t row = (uint32_t)cand[(size_t)q * S + j].node;
+            const float *x = vecs + (size_t)row * dpad;
+            float even = 0.f, odd = 0.f;
+#pragma unroll 8
+            for (int k = 0; k < dpad; k += 4) {
+                const float4 v = __ldg((const float4 *)(x + k));
+                const float4 w = __ldg((const float4 *)(qv + k));
+                const float d0 = v.x - w.x, d1 = v.y - w.y, d2 = v.z - w.z, d3 = v.w - w.w;
+                even = fmaf(d0, d0, even);
+                odd = fmaf(d1, d1, odd);
+                even = fmaf(d2, d2, even);
+                odd = fmaf(d3, d3, odd);
+            }
+            keys[j] = make_key(even + odd, row);
+        }
+    for (int base = 0; ORDER == RR_LANES8 && base < n; base += NT / 8) {
         const int j = base + grp;
         const bool ok = j < n;
         const uint32_t row = (uint32_t)cand[(size_t)q * S + (ok ? j : 0)].node;
