@@ -94,6 +94,7 @@ int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &
             if (db.one_range)
                 db.pass = std::min(db.pass, prog_pass_estimate(g, pb.insns.data() + pb.progs[0].insn0,
                                                                1, pb.consts.data()));
+            db.bound = b;
             // (the route holds one key per query and listed row: 128 MB at most)
             if (b <= sparse_limit(g->count) && (uint64_t)nq * b <= (1ull << 24))
                 db.sparse_bound = b;
@@ -169,15 +170,25 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     ScanScratch &s = g->scan;
 
     if (ev) cudaEventRecord(ev[0], g->stream);
-    const bool sparse_route = db.sparse_bound > 0 && !db.counts_on_device && topb <= 1024;
+    bool sparse_route = db.sparse_bound > 0 && !db.counts_on_device && topb <= 1024;
     const bool low_tc_can = mode == 1 && tc_supported(g) && tc_superset(g, topb, db.q_amax) > 0;
     // exact answers from the f32 rows: the exact mode, and low-precision
     // uploads whose rows are too wide for their own scan
     const bool exact_mode = mode == PV_MODE_EXACT || (mode == 1 && !tc_supported(g));
     const bool exact_tc_can = exact_mode && nq >= PV_EXACT_TC_MIN_NQ &&
                               tf32_supported(g) && tf32_superset(g, topb, db.q_amax) > 0;
-    const bool sparse_tc = sparse_route && (low_tc_can || exact_tc_can) &&
-                           db.sparse_bound >= PV_SPARSE_TC_MIN_ROWS;
+    bool sparse_tc = sparse_route && (low_tc_can || exact_tc_can) &&
+                     db.sparse_bound >= PV_SPARSE_TC_MIN_ROWS;
+    uint64_t list_bound = db.sparse_bound;
+    // a shared filter that passes more rows than that: gathered where it pays
+    if (!sparse_route && !db.counts_on_device && topb <= 1024 && (low_tc_can || exact_tc_can) &&
+        gather_pays(g, nq, db.bound, db.pass,
+                    low_tc_can ? tc_superset(g, topb, db.q_amax) : tf32_superset(g, topb, db.q_amax),
+                    !low_tc_can) &&
+        sparse_tc_reserve(g, db.bound, !low_tc_can)) {
+        sparse_route = sparse_tc = true;
+        list_bound = db.bound;
+    }
     // a few queries answered exactly on the CUDA cores: only the rows their
     // filter passes are read (a selective filter's list would be made first)
     const bool rows_route =
@@ -220,7 +231,7 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     if (sparse_route) {
         g->last_sparse = 1;
         if (sparse_tc) {  // the matching rows on the tensor cores
-            if (sparse_tc_launch(g, db, topb, db.sparse_bound, exact_tc_can, d_out, d_cnt, d_trunc,
+            if (sparse_tc_launch(g, db, topb, list_bound, exact_tc_can, d_out, d_cnt, d_trunc,
                                  ev, errbuf, errlen))
                 return -1;
             g->last_exact_tc = exact_tc_can ? 1 : 0;

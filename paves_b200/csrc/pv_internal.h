@@ -122,6 +122,7 @@ struct DevBatch {
     // many programs, all of the form bitmap_rank.cu takes
     bool rank_ok = false;
     bool one_prog = false;    // P == 1 and every query uses it
+    uint64_t bound = 0;       // one_prog: at most this many rows pass (0: not known)
     double pass = 1.0;        // share of the rows its filter passes, at most or estimated
     bool rows_fused = false;  // scan_rows.cu tests the one filter itself
 };
@@ -177,6 +178,8 @@ constexpr uint64_t PV_SPARSE_TC_MIN_ROWS = 16384;
 int sparse_tc_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, uint64_t bound, bool tf32,
                      FvHit *d_out, uint32_t *d_cnt, uint8_t *d_trunc, cudaEvent_t *ev,
                      char *errbuf, size_t errlen);
+bool gather_pays(const FvGpuIndex *g, int nq, uint64_t bound, double pass, int S, bool tf32);
+bool sparse_tc_reserve(FvGpuIndex *g, uint64_t bound, bool tf32);
 int sparse_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, uint64_t bound, FvHit *d_out,
                   uint32_t *d_cnt, uint8_t *d_trunc, char *errbuf, size_t errlen);
 int tc_redo_uncertain(FvGpuIndex *g, int nq, const float *queries, const PredBatch &pb,

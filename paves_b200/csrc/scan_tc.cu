@@ -412,11 +412,15 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // 64: 62.6 ms for 60,000 rows with 24, 70.6 with 8; batch 1000 the same
     // with both), 8 where an estimated bound makes up for a short sample; and
     // chunks for four times the keys a certain bound needs.
-    const uint64_t region = ntiles_all / grow;
-    const double best = sqrt((double)S * tpc / grow);
+    // A compacted set has room for more rows than pass: the tiles that exist
+    // are a prefix, so the sample's are dealt round robin (every CTA has some
+    // of them) and as many more are drawn as `pass` leaves empty.
+    const double fill = !rs || pass > 0.9 ? 1.0 : std::max(pass, 1.0 / 64);
+    const uint64_t region = rs ? tpc : ntiles_all / grow;
+    const double best = sqrt((double)S * tpc * fill / grow);
     const uint64_t least = certify ? 1 : ((uint64_t)S + grow - 1) / grow;
-    const uint64_t m = std::min<uint64_t>(
-        region, std::min<uint64_t>(certify ? 8 : 24, std::max<uint64_t>(least, (uint64_t)best)));
+    const double want_m = std::min<double>(certify ? 8 : 24, std::max<double>(least, floor(best)));
+    const uint64_t m = (uint64_t)std::min<double>((double)region, ceil(want_m / fill));
     // The sample's S-th key is a bound for certain, but with large supersets
     // it admits S / share rows, far more than S. A sample holding `share` of
     // the rows has S * share of the S best in expectation, with a Poisson
@@ -446,7 +450,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const bool little = kept * ugrow * EPI * R <= 3000.0 &&
                         admits * std::min(32, qtiles > 1 ? 32 : nq) <= 150.0;
     const bool seed = g->tune_seed != 2 && !little &&
-                      m * grow * (TC_BN / 32) >= 2 * (uint64_t)rank;
+                      (uint64_t)(m * fill * grow * (TC_BN / 32)) >= 2 * (uint64_t)rank;
     if (!seed) {
         grow = std::max(1, g->tune_grow > 0 ? g->tune_grow : g->sm_count / qtiles);
         tpc = split(ntiles_all);
@@ -594,8 +598,8 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     uint32_t *ccnt = (uint32_t *)(c + off_ccnt);
     if (seed) {
         TcArgs sa = a;
-        sa.tile0_mul = region;
-        sa.tile_step = std::max<uint64_t>(1, region / m);
+        sa.tile0_mul = rs ? 1 : region;
+        sa.tile_step = std::max<uint64_t>(1, region / m) * (rs ? grow : 1);
         sa.tiles_per_cta = m;
         // A list keeps the best key of every few of its chunks, about 4 rank
         // keys in all (the S-th key of a subset of the sample still bounds
@@ -608,8 +612,9 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         const int chunks = (int)((m + epiw - 1) / epiw) * (TC_BN / R / 32);  // of a list
         const int lists = grow * (int)std::min<uint64_t>(m, epiw) * R;
         const int want = std::max(1, (4 * rank + lists - 1) / lists);
-        sa.KP = std::min(KP, want);
-        sa.seed_group = std::max(1, std::max(chunks / want, (chunks + sa.KP - 1) / sa.KP));
+        sa.KP = std::min(KP, (int)ceil(want / fill));
+        sa.seed_group = std::max(1, std::max((int)(chunks * fill) / want,
+                                             (chunks + sa.KP - 1) / sa.KP));
         sa.push_tau = sa.KP == S ? 1 : 0;
         sa.fullmin = nullptr;
         g->launches += 2;  // seeding pass + its merge
