@@ -290,17 +290,25 @@ void launch_final(uint64_t *fwd, uint32_t *fwd_cnt, const uint64_t *rev, const u
 // Exact nearest neighbours of rows [r0, r0 + nq) of g among all rows of g:
 // the tensor-core scan when its BF16 distances are certified exact for
 // these rows, else the exact FP32 scan (queries read in place from g's f32
-// rows). out [nq][topb] ascending, cnt [nq].
+// rows). out [nq][topb] ascending, cnt [nq]; unc [nq]: nonzero where short
+// lists may have dropped a neighbour (the batch is then run again, `exact`).
 int knn_batch(FvGpuIndex *g, uint64_t r0, int nq, uint32_t topb, const int32_t *d_qprog,
               const unsigned long long *d_popcnt, FvHit *d_out, uint32_t *d_cnt, uint8_t *d_tr,
-              char *errbuf, size_t errlen) {
+              uint8_t *d_unc, bool exact, char *errbuf, size_t errlen) {
     const float *d_q = g->d_vecs + r0 * (uint64_t)g->dpad;
     const uint64_t bm_words = (g->count + 31) / 32;
-    // (lists of at most 64 keys hold the whole answer: no certification)
-    if (g->precision != FV_GPU_PREC_FP32 && tc_supported(g) && topb <= 64 &&
+    g->tc_unc = nullptr;
+    if (!exact && g->precision != FV_GPU_PREC_FP32 && tc_supported(g) && topb <= 64 &&
         tc_superset(g, topb, g->row_amax) == (int)topb) {
-        return launch_scan_tc(g, nq, g->row_amax, d_q, d_qprog, nullptr, bm_words, d_popcnt,
-                              topb, d_out, d_cnt, d_tr, nullptr, errbuf, errlen);
+        if (launch_scan_tc(g, nq, g->row_amax, d_q, d_qprog, nullptr, bm_words, d_popcnt, topb,
+                           d_out, d_cnt, d_tr, nullptr, errbuf, errlen))
+            return -1;
+        if (g->tc_unc)
+            PV_CUDA_OK(cudaMemcpyAsync(d_unc, g->tc_unc, (size_t)nq, cudaMemcpyDeviceToDevice,
+                                       g->stream),
+                       errbuf, errlen);
+        g->tc_unc = nullptr;
+        return 0;
     }
     ScanPlan pl;
     const bool tiled = plan_scan_f32t(g->count, g->dpad, nq, (int)topb, g->sm_count, pl);
@@ -362,7 +370,7 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
         memcpy(g->tmap_x, &m, sizeof(m));
         g->tmap_x_ok = true;
     }
-    DevArr qprog, popcnt, out, cnt, tr, lst, lcnt, in_cnt, in_off, cursor, rev;
+    DevArr qprog, popcnt, out, cnt, tr, unc, lst, lcnt, in_cnt, in_off, cursor, rev;
     const int topb_max = (int)std::min<uint64_t>((uint64_t)C + 1, n);  // self included
     HG_OK(qprog.alloc((size_t)B * 4));
     HG_OK(cudaMemsetAsync(qprog.p, 0xFF, (size_t)B * 4, st));  // no filter
@@ -370,6 +378,7 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
     HG_OK(out.alloc((size_t)B * topb_max * sizeof(FvHit)));
     HG_OK(cnt.alloc((size_t)B * 4));
     HG_OK(tr.alloc((size_t)B));
+    HG_OK(unc.alloc((size_t)n));
     HG_OK(lst.alloc((size_t)n * R * 8));
     HG_OK(lcnt.alloc((size_t)n * 4));
     HG_OK(in_cnt.alloc((size_t)n * 4));
@@ -377,6 +386,7 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
     HG_OK(in_off.alloc((size_t)(n + 1) * 8));
     HG_OK(cudaMemsetAsync(lcnt.p, 0, (size_t)n * 4, st));
     std::vector<uint32_t> h_in;
+    std::vector<uint8_t> h_unc;
     std::vector<uint64_t> h_off;
     size_t rev_cap = 0;
     int rc = 0;
@@ -385,12 +395,13 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
         // 1-2: candidates among the inserted prefix [0, hi), forward selection
         g->count = hi;
         const int topb = (int)std::min<uint64_t>((uint64_t)C + 1, hi);
-        for (uint64_t r0 = lo; r0 < hi && rc == 0; r0 += B) {
+        HG_OK(cudaMemsetAsync(unc.p, 0, (size_t)(hi - lo), st));
+        auto batch = [&](uint64_t r0, bool exact) {
             const int nq = (int)std::min<uint64_t>(B, hi - r0);
-            rc = knn_batch(g, r0, nq, (uint32_t)topb, qprog.as<int32_t>(),
-                           popcnt.as<unsigned long long>(), out.as<FvHit>(), cnt.as<uint32_t>(),
-                           tr.as<uint8_t>(), errbuf, errlen);
-            if (rc) break;
+            if (knn_batch(g, r0, nq, (uint32_t)topb, qprog.as<int32_t>(),
+                          popcnt.as<unsigned long long>(), out.as<FvHit>(), cnt.as<uint32_t>(),
+                          tr.as<uint8_t>(), unc.as<uint8_t>() + (r0 - lo), exact, errbuf, errlen))
+                return -1;
             if (NVn <= 1)
                 launch_forward<1>(out.as<FvHit>(), cnt.as<uint32_t>(), topb, r0, nq, R, g->d_vecs,
                                   dpad, lst.as<uint64_t>(), lcnt.as<uint32_t>(), st);
@@ -400,11 +411,25 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
             else
                 launch_forward<4>(out.as<FvHit>(), cnt.as<uint32_t>(), topb, r0, nq, R, g->d_vecs,
                                   dpad, lst.as<uint64_t>(), lcnt.as<uint32_t>(), st);
-            if (cudaGetLastError() != cudaSuccess) rc = -1;
+            return cudaGetLastError() == cudaSuccess ? 0 : -1;
+        };
+        for (uint64_t r0 = lo; r0 < hi && rc == 0; r0 += B) rc = batch(r0, false);
+        if (!rc) rc = check_tc_watchdog(g, errbuf, errlen);
+        if (!rc) {
+            h_unc.resize(hi - lo);
+            if (cudaMemcpyAsync(h_unc.data(), unc.p, (size_t)(hi - lo), cudaMemcpyDeviceToHost, st) !=
+                    cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                rc = -1;
+        }
+        for (uint64_t r0 = lo; r0 < hi && rc == 0; r0 += B) {
+            const uint64_t r1 = std::min<uint64_t>(r0 + B, hi);
+            if (std::any_of(h_unc.begin() + (r0 - lo), h_unc.begin() + (r1 - lo),
+                            [](uint8_t u) { return u != 0; }))
+                rc = batch(r0, true);
         }
         g->count = n;
         if (rc) break;
-        if ((rc = check_tc_watchdog(g, errbuf, errlen))) break;
         // 3: reverse edges of the new nodes' lists
         const uint64_t nu = hi - lo;
         HG_OK(cudaMemsetAsync(in_cnt.p, 0, (size_t)hi * 4, st));

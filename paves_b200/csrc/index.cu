@@ -76,6 +76,31 @@ __global__ void norm32_kernel(const float *__restrict__ src, int dpad, uint64_t 
     }
 }
 
+// Whether the rows lie in an order that says nothing of where they are: of
+// `samples` evenly spaced rows, a warp each, how many are nearer to a row at
+// most 31 places on than to one half the table away, less how many are
+// farther (rows in random order: zero within a few times sqrt(samples)).
+__global__ void order_kernel(const float *__restrict__ src, int dpad, uint64_t nrows, int samples,
+                             int *__restrict__ nearer) {
+    const int lane = threadIdx.x & 31;
+    const int p = (int)(blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5));
+    if (p >= samples) return;
+    const uint64_t i = (uint64_t)p * nrows / samples;
+    const uint64_t a = (i + 1 + p % 31) % nrows, b = (i + nrows / 2 + p * 37ull) % nrows;
+    float da = 0.f, db = 0.f;
+    for (int j = lane; j < dpad; j += 32) {
+        const float v = src[i * dpad + j];
+        const float x = v - src[a * dpad + j], y = v - src[b * dpad + j];
+        da = fmaf(x, x, da);
+        db = fmaf(y, y, db);
+    }
+    for (int o = 16; o; o >>= 1) {
+        da += __shfl_xor_sync(0xffffffffu, da, o);
+        db += __shfl_xor_sync(0xffffffffu, db, o);
+    }
+    if (lane == 0 && da != db) atomicAdd(nearer, da < db ? 1 : -1);
+}
+
 // fp32 rows -> fp8-e4m3 rows with one scale per row (absmax / 448), plus
 // the squared norm of the dequantized row.
 __global__ void to_fp8_kernel(const float *__restrict__ src, int dpad, int dim,
@@ -356,18 +381,24 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         if ((e = cudaMalloc(&g->d_norm32, rows_pad32 * 4 + 16)) != cudaSuccess)
             return bail("f32 norms", e);
         unsigned *d_max = (unsigned *)(g->d_norm32 + rows_pad32);
-        unsigned h_max[2] = {};
+        const int samples = (int)std::min<uint64_t>(count, 4096);
+        unsigned h_max[3] = {};
         if ((e = cudaMemsetAsync(g->d_norm32, 0, rows_pad32 * 4 + 16, g->stream)) != cudaSuccess)
             return bail("f32 norms", e);
         norm32_kernel<<<(unsigned)((count + 7) / 8), 256, 0, g->stream>>>(g->d_vecs, dpad, count,
                                                                          g->d_norm32, d_max);
         if ((e = cudaGetLastError()) != cudaSuccess) return bail("f32 norms", e);
-        if ((e = cudaMemcpyAsync(h_max, d_max, 8, cudaMemcpyDeviceToHost, g->stream)) !=
+        order_kernel<<<(unsigned)((samples + 7) / 8), 256, 0, g->stream>>>(
+            g->d_vecs, dpad, count, samples, (int *)(d_max + 2));
+        if ((e = cudaGetLastError()) != cudaSuccess) return bail("row order", e);
+        if ((e = cudaMemcpyAsync(h_max, d_max, 12, cudaMemcpyDeviceToHost, g->stream)) !=
                 cudaSuccess ||
             (e = cudaStreamSynchronize(g->stream)) != cudaSuccess)
             return bail("f32 norms", e);
         memcpy(&g->norm32_max, &h_max[0], 4);
         memcpy(&g->res32_max, &h_max[1], 4);
+        // (the line: six deviations of a fair coin's, and 5 % of rows more)
+        g->rows_mixed = (int)h_max[2] <= std::max(samples / 10, (int)(6.0 * sqrt((double)samples)));
     }
 
     if (precision != FV_GPU_PREC_FP32) {
@@ -514,6 +545,7 @@ FvGpuIndex *index_view(const FvGpuIndex *g) {
     v->d_norm32 = g->d_norm32;
     v->norm32_max = g->norm32_max;
     v->res32_max = g->res32_max;
+    v->rows_mixed = g->rows_mixed;
     v->exact_tc = g->exact_tc;
     v->row_amax = g->row_amax;
     v->sorted_cols = g->sorted_cols;

@@ -115,6 +115,9 @@ struct FvGpuIndex {
     float *d_norm32 = nullptr;  // [rows padded to 128] ||x||^2 of the f32 rows
     float norm32_max = 0.f;     // largest of them
     float res32_max = 0.f;      // largest squared part of a row that TF32 drops
+    // rows in an order unrelated to where they lie (order_kernel): a query's
+    // nearest spread over the table, so short lists and samples of tiles serve
+    bool rows_mixed = false;
     int exact_tc = 1;           // exact-mode batches may take it (0: CUDA cores only)
     int last_exact_tc = 0;      // the last brute batch took it
 

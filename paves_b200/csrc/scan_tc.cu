@@ -293,9 +293,9 @@ bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns) {
     if (!tc_supported(g) || epi < 1 || epi > 3 || ns < 2 || ns > TC_MAX_STAGES) return false;
     const int S = tc_superset(g, topb, -1.f);
     if (!S) return false;
-    const int KP = std::min(S, tc_list_cap(epi));
-    const int esz = g->precision == FV_GPU_PREC_FP8 ? 1 : 2;
-    return tc_smem(g->kpad * esz / TC_KB_BYTES, ns, KP, epi) <= 227 * 1024;
+    const int kblocks = g->kpad * (g->precision == FV_GPU_PREC_FP8 ? 1 : 2) / TC_KB_BYTES;
+    const int KP = std::min(S, tc_list_cap(epi, kblocks));
+    return tc_smem(kblocks, ns, KP, epi) <= 227 * 1024;
 }
 
 template <int KIND, int EPI, bool WARM>
@@ -356,7 +356,10 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // three run the same: 0.0615 ms), one where a tile's rows take longer to
     // arrive than one group to look through (16 queries over BF16 rows, 64
     // over f32 rows: the same pass, half the lists to merge, 0.088 against
-    // 0.094 ms in all) or the lists do not fit with two. The automatic shape stays within smem_pref,
+    // 0.094 ms in all) or the lists do not fit with two. With three, lists of
+    // up to 32 keys that spill: 64 keys left room for one group (2048 queries,
+    // 500,000 BF16 rows, k 64: the pass 2.25 ms, 48 keys and two groups 1.08
+    // for k 48; now 0.80 and 0.76). The automatic shape stays within smem_pref,
     // which leaves each SM a few KB for a small kernel beside the scan (the
     // router's, a merge launched early).
     const size_t smem_cap = 227 * 1024;
@@ -366,33 +369,41 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         2, (int)(128 * 1024 / ((size_t)std::min(kblocks, TC_KBS) * TC_BOX *
                                          (tc_qstream(kblocks) ? 2 : 1)))));
     int EPI = 0, NS = 0;
-    for (int e = kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 ? 3 : 2; e >= 1 && !EPI; e--) {
-        const int KPe = std::min(S, tc_list_cap(e));
-        int n = ns0;
-        while (n > 2 && tc_smem(kblocks, n, KPe, e) > smem_pref) n--;
-        if (tc_smem(kblocks, n, KPe, e) <= smem_pref) {
-            EPI = e;
-            NS = n;
+    auto shape = [&](int most) {
+        EPI = 0;
+        for (int e = most; e >= 1 && !EPI; e--) {
+            const int KPe = std::min(S, tc_list_cap(e, kblocks));
+            int n = ns0;
+            while (n > 2 && tc_smem(kblocks, n, KPe, e) > smem_pref) n--;
+            if (tc_smem(kblocks, n, KPe, e) <= smem_pref) {
+                EPI = e;
+                NS = n;
+            }
         }
-    }
-    if (!EPI) {  // the smallest shape, within the hard limit
-        EPI = 1;
-        NS = 2;
-    }
+        if (!EPI) {  // the smallest shape, within the hard limit
+            EPI = 1;
+            NS = 2;
+        }
+    };
+    // (three groups' lists hold every nearest row of the query that a list
+    // meets: where rows are stored cluster by cluster, only whole lists do)
+    const bool whole3 = S <= tc_list_cap(3, kblocks);
+    shape(kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 && (g->rows_mixed || whole3) ? 3 : 2);
+    bool tuned = false;
     if (g->tune_epi || g->tune_ns) {  // a tuned shape, if it fits
         const int e = g->tune_epi ? g->tune_epi : EPI, n = g->tune_ns ? g->tune_ns : NS;
         if (e >= 1 && e <= 3 && n >= 2 && n <= TC_MAX_STAGES &&
-            tc_smem(kblocks, n, std::min(S, tc_list_cap(e)), e) <= smem_cap) {
+            tc_smem(kblocks, n, std::min(S, tc_list_cap(e, kblocks)), e) <= smem_cap) {
             EPI = e;
             NS = n;
+            tuned = true;
         }
     }
-    const int KP = std::min(S, tc_list_cap(EPI));
-    const size_t smem = tc_smem(kblocks, NS, KP, EPI);
+    int KP = std::min(S, tc_list_cap(EPI, kblocks));
     // rows scanned: the index's, or a compacted set
     const uint64_t nrows_scan = rs ? rs->nrows : g->count;
     const uint64_t ntiles_all = (nrows_scan + TC_BN - 1) / TC_BN;
-    const bool certify = KP < S;  // lists shorter than the superset
+    bool certify = KP < S;  // lists shorter than the superset
     int grow = std::max(1, g->tune_grow > 0 ? g->tune_grow : g->sm_count / qtiles);
     auto split = [&](uint64_t most) {  // CTAs along the rows, evenly loaded
         if ((uint64_t)grow > most) grow = (int)most;
@@ -418,22 +429,33 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const double fill = !rs || pass > 0.9 ? 1.0 : std::max(pass, 1.0 / 64);
     const uint64_t region = rs ? tpc : ntiles_all / grow;
     const double best = sqrt((double)S * tpc * fill / grow);
-    const uint64_t least = certify ? 1 : ((uint64_t)S + grow - 1) / grow;
-    const double want_m = std::min<double>(certify ? 8 : 24, std::max<double>(least, floor(best)));
-    const uint64_t m = (uint64_t)std::min<double>((double)region, ceil(want_m / fill));
+    const bool may_est = certify && S > TC_MAX_LIST && g->rows_mixed;
+    const uint64_t least = may_est ? 1 : ((uint64_t)S + grow - 1) / grow;
+    const double want_m = std::min<double>(may_est ? 8 : 24, std::max<double>(least, floor(best)));
+    uint64_t m = (uint64_t)std::min<double>((double)region, ceil(want_m / fill));
     // The sample's S-th key is a bound for certain, but with large supersets
     // it admits S / share rows, far more than S. A sample holding `share` of
     // the rows has S * share of the S best in expectation, with a Poisson
     // spread: its key six deviations above that lies beyond the S-th key of
     // the scan but for about one query in 10^9, and the merge sees such a
     // query (fewer than S keys got through), which is then re-run exactly.
-    // Only where the merge certifies anyway (lists shorter than the superset).
-    const double share = std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan);
-    const int rank_est = (int)ceil(S * share + 6.0 * sqrt(S * share) + 8.0);
-    const bool estimated = certify && rank_est < S;
-    const int rank = estimated ? rank_est : S;
+    // Only where the merge certifies anyway (lists shorter than the superset)
+    // and rows lie in no order (else the best clump in the sample's tiles),
+    // and not for up to 64 keys, which a certain bound costs little (512
+    // queries, 500,000 rows, S 40: 0.180 against 0.170 ms).
+    int rank_est = S;
+    auto enough = [&]() {  // chunk minima for the bound's rank, twice over
+        const double share = std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan);
+        rank_est = may_est ? (int)ceil(S * share + 6.0 * sqrt(S * share) + 8.0) : S;
+        return (uint64_t)(m * fill * grow * (TC_BN / 32)) >= 2 * (uint64_t)std::min(S, rank_est);
+    };
+    // (a table of few tiles is sampled more of: 60,000 rows, 512 queries,
+    // S 800 took 1.08 ms without a bound, 0.36 seeded)
+    while (!enough() && m < region) m++;
+    const bool estimated = rank_est < S;
+    const int rank = std::min(S, rank_est);
     // Seeding pays from two tiles per CTA on, as long as the sample's chunk
-    // minima are at least twice the keys its bound needs: small tables took
+    // minima are at least twice the keys its bound needs (enough): small tables took
     // 2 to 4 times as long filling their lists behind no bound (100,000 BF16
     // rows, 73 queries: k 2, 25, 100 in 0.106, 0.158, 0.343 ms, seeded 0.043,
     // 0.044, 0.079). Without it every tile gets its own CTA.
@@ -449,9 +471,13 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const double admits = p <= KP ? p : KP * (1.0 + log(p / KP));
     const bool little = kept * ugrow * EPI * R <= 3000.0 &&
                         admits * std::min(32, qtiles > 1 ? 32 : nq) <= 150.0;
-    const bool seed = g->tune_seed != 2 && !little &&
-                      (uint64_t)(m * fill * grow * (TC_BN / 32)) >= 2 * (uint64_t)rank;
+    const bool seed = g->tune_seed != 2 && !little && enough();
     if (!seed) {
+        if (EPI == 3 && !tuned) {  // without a bound: lists that keep the best
+            shape(2);
+            KP = std::min(S, tc_list_cap(EPI, kblocks));
+            certify = KP < S;
+        }
         grow = std::max(1, g->tune_grow > 0 ? g->tune_grow : g->sm_count / qtiles);
         tpc = split(ntiles_all);
     }
@@ -468,8 +494,11 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const size_t cbytes = off_unc + (size_t)nq + 256;
     PV_CUDA_OK(s.cand.ensure(cbytes), errbuf, errlen);
     PV_CUDA_OK(s.tau.ensure((size_t)nq * 8), errbuf, errlen);
+    const size_t smem = tc_smem(kblocks, NS, KP, EPI);
     const int nlists = grow * EPI * R;  // lists per query
-    const uint64_t dcap = (uint64_t)nlists * KP;  // a query's dense run at most
+    const bool spill = seed && certify && EPI == 3;
+    // a query's dense run at most
+    const uint64_t dcap = (uint64_t)nlists * (spill ? std::min(S, TC_MAX_LIST) : KP);
     PV_CUDA_OK(s.part.ensure((size_t)nq * dcap * 8), errbuf, errlen);
     // [dcnt u32 x nq][fullmin u64 x nq]
     const size_t off_fm = ((size_t)nq * 4 + 255) & ~(size_t)255;
@@ -544,6 +573,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     a.rep = R;
     a.bq = bq;
     a.push_tau = KP == S ? 1 : 0;
+    a.spill = spill ? 1 : 0;
     a.NS = NS;
     a.qstream = tc_qstream(kblocks) ? 1 : 0;
     a.xnorm = rs ? rs->norms : tf32 ? g->d_norm32 : g->d_norm;
@@ -612,10 +642,11 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         const int chunks = (int)((m + epiw - 1) / epiw) * (TC_BN / R / 32);  // of a list
         const int lists = grow * (int)std::min<uint64_t>(m, epiw) * R;
         const int want = std::max(1, (4 * rank + lists - 1) / lists);
-        sa.KP = std::min(KP, (int)ceil(want / fill));
+        sa.KP = std::min(KP * EPI / epiw, (int)ceil(want / fill));
         sa.seed_group = std::max(1, std::max((int)(chunks * fill) / want,
                                              (chunks + sa.KP - 1) / sa.KP));
         sa.push_tau = sa.KP == S ? 1 : 0;
+        sa.spill = 0;
         sa.fullmin = nullptr;
         g->launches += 2;  // seeding pass + its merge
         PV_CUDA_OK(run(sa, true), errbuf, errlen);
@@ -633,7 +664,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // spread over the CTAs
     a.tile0_mul = rs ? 1 : tpc;
     a.tile_step = rs ? (uint64_t)grow : 1;
-    PV_CUDA_OK(run(a, rs != nullptr || !seed), errbuf, errlen);
+    PV_CUDA_OK(run(a, !seed), errbuf, errlen);
     if (ev) cudaEventRecord(ev[2], g->stream);
     uint8_t *d_unc = (certify || num_cert) ? (uint8_t *)(c + off_unc) : nullptr;
     if (S == (int)topb) {

@@ -42,8 +42,12 @@ constexpr int TC_KBS = 2;           // K-blocks per pipeline stage
 // certifies per query (queries it cannot certify are re-run exactly).
 constexpr int TC_MAX_SUPERSET = 1024;
 constexpr int TC_MAX_LIST = 64;
-constexpr int TC_MAX_LIST3 = 48;   // with three epilogue groups (their shared memory)
-inline int tc_list_cap(int epi) { return epi == 3 ? TC_MAX_LIST3 : TC_MAX_LIST; }
+// With three epilogue groups the lists are short (their shared memory beside
+// a query tile of kblocks K-blocks and two stages); full ones of a pass with
+// a bound spill into the dense run (TcArgs::spill).
+inline int tc_list_cap(int epi, int kblocks) {
+    return epi < 3 ? TC_MAX_LIST : kblocks <= 2 ? 32 : kblocks <= 4 ? 24 : 16;
+}
 constexpr int TC_MAX_STAGES = 8;   // TMA pipeline stages at most
 constexpr int TC_NR = 8;            // tiles of row norms in flight (shared-memory ring)
 // words per norm slot: norms, fp8 scales, then the index rows of a
@@ -86,6 +90,10 @@ struct TcArgs {
     int rep;            // query replicas down the tile's 128 slots (1, 2, 4)
     int bq;             // query slots per replica = TC_BM / rep
     int push_tau;       // a full list's last key bounds the superset (lists hold it all)
+    // a full list moves its keys to the query's dense run and starts anew
+    // while the run has room (a pass behind a seeded bound): nothing is
+    // dropped, and short lists leave shared memory for three epilogue groups
+    int spill = 0;
     // > 0 (WARM passes, no lazy filters): each list takes the best key of
     // every seed_group 32-row chunks instead of its best KP keys
     int seed_group = 0;
@@ -624,6 +632,17 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                     if (n < KP) {  // in any order until the list is full
                         PV_L(n) = key;
                         if (++n < KP) continue;
+                        if (!WARM && a.spill) {
+                            const uint32_t at = atomicAdd(a.dcnt + qg, (uint32_t)KP);
+                            const int w = at < a.dcap ? (int)min((uint64_t)KP, a.dcap - at) : 0;
+                            uint64_t *dst = a.dense + (uint64_t)qg * a.dcap + at;
+#pragma unroll 1
+                            for (int j = 0; j < w; j++) dst[j] = PV_L(j);
+#pragma unroll 1
+                            for (int j = w; j < KP; j++) PV_L(j - w) = PV_L(j);
+                            n = KP - w;
+                            if (w > 0) continue;
+                        }
                         // full: a max-heap from here on (root = worst kept)
                         from = (KP >> 1) - 1;
                         put = from >= 0 ? PV_L(from) : 0;
@@ -689,10 +708,15 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
             if (nw > 0) {
                 uint64_t at = atomicAdd(a.dcnt + qg, (uint32_t)nw);
                 uint64_t *dst = a.dense + (uint64_t)qg * a.dcap;
+                uint64_t lost = KEY_MAX;  // (a spilled run may have no room left)
                 for (int i = 0; i < n; i++) {
                     const uint64_t key = PV_L(i);
-                    if (key <= bound && at < a.dcap) dst[at++] = key;
+                    if (key > bound) continue;
+                    if (at < a.dcap) dst[at++] = key;
+                    else if (key < lost) lost = key;
                 }
+                if (a.spill && lost != KEY_MAX)
+                    atomicMin(a.fullmin + qg, (unsigned long long)lost);
             }
             if (a.fullmin && n == KP) atomicMin(a.fullmin + qg, (unsigned long long)lmax);
         }
