@@ -161,6 +161,25 @@ __global__ void hg_count_kernel(const uint64_t *__restrict__ fwd,
     atomicAdd(&in_cnt[key_row(fwd[u * R + i % R])], 1u);
 }
 
+// Each node's run among the reverse edges, anywhere (one claim per warp).
+__global__ void hg_runs_kernel(const uint32_t *__restrict__ in_cnt, uint64_t n,
+                               uint64_t *__restrict__ in_off,
+                               unsigned long long *__restrict__ total) {
+    const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const uint32_t c = v < n ? in_cnt[v] : 0u;
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t w = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += w;
+    }
+    unsigned long long base = 0;
+    if (lane == 31 && incl) base = atomicAdd(total, (unsigned long long)incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (v < n) in_off[v] = base + incl - c;
+}
+
 __global__ void hg_scatter_kernel(const uint64_t *__restrict__ fwd,
                                   const uint32_t *__restrict__ fwd_cnt, uint64_t u0, uint64_t nu,
                                   int R, const uint64_t *__restrict__ in_off,
@@ -236,6 +255,25 @@ hg_final_kernel(uint64_t *__restrict__ fwd, uint32_t *__restrict__ fwd_cnt,
     if (lane == 0) fwd_cnt[v] = (uint32_t)nk;
 }
 
+// The rows of an upper level, out of the table's: f32 rows and, where the
+// scans read them, the BF16 rows and norms (kpad16: 16-byte pieces of one).
+__global__ void hg_gather_kernel(const float *__restrict__ x, int dpad,
+                                 const unsigned char *__restrict__ lo, int kpad16,
+                                 const float *__restrict__ norm, const uint32_t *__restrict__ ids,
+                                 uint64_t n, float *__restrict__ xs, unsigned char *__restrict__ los,
+                                 float *__restrict__ norms) {
+    const int d16 = dpad / 4, per = d16 + kpad16;
+    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n * per) return;
+    const uint64_t i = p / per, r = ids[i];
+    const int j = (int)(p % per);
+    if (j < d16)
+        ((uint4 *)xs)[i * d16 + j] = __ldg((const uint4 *)x + r * d16 + j);
+    else
+        ((uint4 *)los)[i * kpad16 + j - d16] = __ldg((const uint4 *)lo + r * kpad16 + j - d16);
+    if (j == 0 && norm) norms[i] = __ldg(norm + r);
+}
+
 // The lists in the file layout: [cnt, ids...] of stride R + 1.
 __global__ void hg_export_kernel(const uint64_t *__restrict__ lst,
                                  const uint32_t *__restrict__ cnt, uint64_t n, int R,
@@ -250,12 +288,8 @@ __global__ void hg_export_kernel(const uint64_t *__restrict__ lst,
 
 namespace {
 
-struct DevArr {
+struct DevArr {  // a part of HgWork's allocation
     void *p = nullptr;
-    ~DevArr() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t bytes) { return cudaMalloc(&p, bytes ? bytes : 16); }
     template <typename T>
     T *as() const {
         return (T *)p;
@@ -298,7 +332,7 @@ int knn_batch(FvGpuIndex *g, uint64_t r0, int nq, uint32_t topb, const int32_t *
     const float *d_q = g->d_vecs + r0 * (uint64_t)g->dpad;
     const uint64_t bm_words = (g->count + 31) / 32;
     g->tc_unc = nullptr;
-    if (!exact && g->precision != FV_GPU_PREC_FP32 && tc_supported(g) && topb <= 64 &&
+    if (!exact && g->precision != FV_GPU_PREC_FP32 && tc_supported(g) &&
         tc_superset(g, topb, g->row_amax) == (int)topb) {
         if (launch_scan_tc(g, nq, g->row_amax, d_q, d_qprog, nullptr, bm_words, d_popcnt, topb,
                            d_out, d_cnt, d_tr, nullptr, errbuf, errlen))
@@ -347,13 +381,61 @@ int knn_batch(FvGpuIndex *g, uint64_t r0, int nq, uint32_t topb, const int32_t *
     return 0;
 }
 
-// One level over the rows of g by batched insertion: lists [count][R + 1]
-// (device) of local ids.
-int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, size_t errlen) {
+constexpr int HG_BATCH = 2048;  // scan batch (queries per call)
+
+// Workspace of the levels, sized for the largest (level 0 has the most rows
+// and the longest lists, an upper level may have the longest answers), and
+// the upper levels' rows: one allocation (17 of them, and their frees, took
+// 3 of a build's 30 ms and at times ten times that).
+struct HgWork {
+    void *base = nullptr;
+    DevArr qprog, popcnt, out, cnt, tr, unc, lst, lcnt, in_cnt, in_off, cursor, rev, lists;
+    DevArr ids, xs, los, norms;  // of n1 rows
+    ~HgWork() {
+        if (base) cudaFree(base);
+    }
+    cudaError_t alloc(uint64_t n, uint64_t n1, int topb, int R, int dpad, size_t lo_bytes) {
+        const struct {
+            DevArr *a;
+            size_t bytes;
+        } parts[] = {{&qprog, (size_t)HG_BATCH * 4},
+                     {&popcnt, 8},
+                     {&out, (size_t)HG_BATCH * topb * sizeof(FvHit)},
+                     {&cnt, (size_t)HG_BATCH * 4},
+                     {&tr, (size_t)HG_BATCH},
+                     {&unc, (size_t)n},
+                     {&lst, (size_t)n * R * 8},
+                     {&lcnt, (size_t)n * 4},
+                     {&in_cnt, (size_t)n * 4},
+                     {&cursor, (size_t)n * 4},
+                     {&in_off, (size_t)(n + 1) * 8},
+                     // (an insertion batch is at most the rows before it)
+                     {&rev, (size_t)std::max<uint64_t>(64, (n + 1) / 2) * R * 8},
+                     {&lists, (size_t)n * (R + 1) * 4},
+                     {&ids, (size_t)n1 * 4},
+                     {&xs, (size_t)n1 * dpad * 4},
+                     {&los, (size_t)n1 * lo_bytes},
+                     {&norms, (size_t)((n1 + 127) & ~127ull) * 4}};  // whole tiles
+        size_t bytes = 0;
+        for (const auto &p : parts) bytes += (p.bytes + 255) & ~(size_t)255;
+        const cudaError_t e = cudaMalloc(&base, bytes);
+        if (e != cudaSuccess) return e;
+        char *at = (char *)base;
+        for (const auto &p : parts) {
+            p.a->p = at;
+            at += (p.bytes + 255) & ~(size_t)255;
+        }
+        return cudaSuccess;
+    }
+};
+
+// One level over the rows of g by batched insertion: w.lists [count][R + 1]
+// of local ids.
+int build_level(FvGpuIndex *g, HgWork &w, int R, int C, char *errbuf, size_t errlen) {
     const uint64_t n = g->count;
     const int dpad = g->dpad;
     const int NVn = (dpad + 127) / 128;
-    const int B = 2048;          // scan batch (queries per call)
+    const int B = HG_BATCH;
     // first insertion batch: a few rows spread over the whole data set, so
     // the earliest lists link distant regions (then doubling batches)
     const uint64_t first = 64;
@@ -370,25 +452,12 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
         memcpy(g->tmap_x, &m, sizeof(m));
         g->tmap_x_ok = true;
     }
-    DevArr qprog, popcnt, out, cnt, tr, unc, lst, lcnt, in_cnt, in_off, cursor, rev;
-    const int topb_max = (int)std::min<uint64_t>((uint64_t)C + 1, n);  // self included
-    HG_OK(qprog.alloc((size_t)B * 4));
+    DevArr &qprog = w.qprog, &popcnt = w.popcnt, &out = w.out, &cnt = w.cnt, &tr = w.tr,
+           &unc = w.unc, &lst = w.lst, &lcnt = w.lcnt, &in_cnt = w.in_cnt, &in_off = w.in_off,
+           &cursor = w.cursor, &rev = w.rev;
     HG_OK(cudaMemsetAsync(qprog.p, 0xFF, (size_t)B * 4, st));  // no filter
-    HG_OK(popcnt.alloc(8));
-    HG_OK(out.alloc((size_t)B * topb_max * sizeof(FvHit)));
-    HG_OK(cnt.alloc((size_t)B * 4));
-    HG_OK(tr.alloc((size_t)B));
-    HG_OK(unc.alloc((size_t)n));
-    HG_OK(lst.alloc((size_t)n * R * 8));
-    HG_OK(lcnt.alloc((size_t)n * 4));
-    HG_OK(in_cnt.alloc((size_t)n * 4));
-    HG_OK(cursor.alloc((size_t)n * 4));
-    HG_OK(in_off.alloc((size_t)(n + 1) * 8));
     HG_OK(cudaMemsetAsync(lcnt.p, 0, (size_t)n * 4, st));
-    std::vector<uint32_t> h_in;
     std::vector<uint8_t> h_unc;
-    std::vector<uint64_t> h_off;
-    size_t rev_cap = 0;
     int rc = 0;
     for (uint64_t lo = 0; lo < n && rc == 0;) {
         const uint64_t hi = lo == 0 ? std::min(n, first) : std::min(n, 2 * lo);
@@ -438,27 +507,12 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
         hg_count_kernel<<<eb, 256, 0, st>>>(lst.as<uint64_t>(), lcnt.as<uint32_t>(), lo, nu, R,
                                             in_cnt.as<uint32_t>());
         HG_OK(cudaGetLastError());
-        h_in.resize(hi);
-        h_off.resize(hi + 1);
-        HG_OK(cudaMemcpyAsync(h_in.data(), in_cnt.p, (size_t)hi * 4, cudaMemcpyDeviceToHost, st));
-        HG_OK(cudaStreamSynchronize(st));
-        uint64_t tot = 0;
-        for (uint64_t i = 0; i < hi; i++) {
-            h_off[i] = tot;
-            tot += h_in[i];
-        }
-        h_off[hi] = tot;
-        HG_OK(cudaMemcpyAsync(in_off.p, h_off.data(), (size_t)(hi + 1) * 8,
-                              cudaMemcpyHostToDevice, st));
-        if (tot > rev_cap) {
-            if (rev.p) {
-                HG_OK(cudaStreamSynchronize(st));
-                cudaFree(rev.p);
-                rev.p = nullptr;
-            }
-            HG_OK(rev.alloc((size_t)tot * 8));
-            rev_cap = tot;
-        }
+        // (the batch's edges fit rev; in_off's last word counts them)
+        unsigned long long *tot = w.in_off.as<unsigned long long>() + n;
+        HG_OK(cudaMemsetAsync(tot, 0, 8, st));
+        hg_runs_kernel<<<(unsigned)((hi + 255) / 256), 256, 0, st>>>(
+            in_cnt.as<uint32_t>(), hi, in_off.as<uint64_t>(), tot);
+        HG_OK(cudaGetLastError());
         hg_scatter_kernel<<<eb, 256, 0, st>>>(lst.as<uint64_t>(), lcnt.as<uint32_t>(), lo, nu, R,
                                               in_off.as<uint64_t>(), cursor.as<uint32_t>(),
                                               rev.as<uint64_t>());
@@ -477,17 +531,113 @@ int build_level(FvGpuIndex *g, int R, int C, uint32_t *d_lists, char *errbuf, si
                             in_off.as<uint64_t>(), in_cnt.as<uint32_t>(), hi, lo, R, g->d_vecs,
                             dpad, st);
         HG_OK(cudaGetLastError());
-        HG_OK(cudaStreamSynchronize(st));  // rev and the host offsets are reused next batch
         lo = hi;
     }
     g->count = n;
     if (rc) return -1;
     const uint64_t total = n * (uint64_t)(R + 1);
     hg_export_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-        lst.as<uint64_t>(), lcnt.as<uint32_t>(), n, R, d_lists);
+        lst.as<uint64_t>(), lcnt.as<uint32_t>(), n, R, w.lists.as<uint32_t>());
     HG_OK(cudaGetLastError());
     HG_OK(cudaStreamSynchronize(st));
     return 0;
+}
+
+// All levels of the graph, over the uploaded rows: level 0 all of them, R =
+// 2M; levels 1..top the rows of each level, R = M, gathered on the device
+// into one set of buffers that stands in for the table's (an upload of its
+// own per level took 8 of a build's 50 ms, 60,000 rows).
+int build_levels(PvHnsw *h, FvGpuIndex *g, int M, int candidates, int top, char *errbuf,
+                 size_t errlen) {
+    std::lock_guard<std::mutex> lk(g->mu);
+    const uint64_t count = g->count;
+    const uint8_t *lev = hnsw_levels(h);
+    std::vector<uint32_t> ids;
+    for (uint64_t i = 0; i < count; i++)
+        if (lev[i] >= 1) ids.push_back((uint32_t)i);
+    // upper levels are small: twice the candidates (with self: one more)
+    auto upper = [&](uint64_t n) {
+        return (int)std::min<uint64_t>((uint64_t)std::min(2 * candidates + 1, 1023), n - 1);
+    };
+    const int C1 = ids.size() >= 2 ? upper(ids.size()) : 0;
+    HgWork w;
+    const bool low = g->d_vlow != nullptr;
+    const size_t lo_bytes = low ? (size_t)g->kpad * (g->precision == FV_GPU_PREC_FP8 ? 1 : 2) : 0;
+    HG_OK(w.alloc(count, ids.size(),
+                  (int)std::min<uint64_t>((uint64_t)std::max(candidates, C1) + 1, count), 2 * M,
+                  g->dpad, lo_bytes));
+    if (g->precision != FV_GPU_PREC_FP32 && tc_supported(g)) {
+        // the tensor-core scans' scratch at its largest batch: growing with
+        // the doubling batches, it was freed and allocated anew ten times
+        // (query tiles x CTAs along the rows are at most the SMs)
+        const uint64_t nq = std::min<uint64_t>(HG_BATCH, count);
+        const uint64_t topb = std::min<uint64_t>((uint64_t)candidates + 1, count);
+        ScanScratch &s = g->scan;
+        const uint64_t tiles = std::min<uint64_t>(
+            g->sm_count, ((nq + TC_BM - 1) / TC_BM) * ((count + TC_BN - 1) / TC_BN));
+        HG_OK(s.part.ensure((size_t)(TC_BM * tiles * 3 * TC_MAX_LIST * 8)));
+        HG_OK(s.part_cnt.ensure(nq * 12 + 512));
+        HG_OK(s.tau.ensure(nq * 8));
+        HG_OK(s.cand.ensure((nq + TC_BM) * ((size_t)g->kpad * 2 + 16) +
+                            nq * (topb * sizeof(FvHit) + 8) + 4096));
+    }
+    if (build_level(g, w, 2 * M, candidates, errbuf, errlen)) return -1;
+    HG_OK(cudaMemcpy(hnsw_l0(h), w.lists.p, (size_t)count * (2 * M + 1) * 4,
+                     cudaMemcpyDeviceToHost));
+    if (ids.size() < 2) return 0;  // a single node has no neighbours
+    HG_OK(cudaMemsetAsync(w.norms.p, 0, ((ids.size() + 127) & ~127ull) * 4, g->stream));
+    const auto vecs = g->d_vecs;
+    const auto vlow = g->d_vlow;
+    const auto norm = g->d_norm;
+    std::vector<uint32_t> lists;
+    int rc = 0;
+    for (int L = 1; L <= top && !rc; L++) {
+        if (L > 1) {
+            ids.erase(std::remove_if(ids.begin(), ids.end(),
+                                     [&](uint32_t i) { return lev[i] < L; }),
+                      ids.end());
+            if (ids.size() < 2) break;
+        }
+        const uint64_t n = ids.size();
+        const uint64_t pieces = n * (g->dpad / 4 + lo_bytes / 16);
+        if (cudaMemcpyAsync(w.ids.p, ids.data(), n * 4, cudaMemcpyHostToDevice, g->stream) !=
+            cudaSuccess) {
+            rc = -1;
+            break;
+        }
+        hg_gather_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, g->stream>>>(
+            vecs, g->dpad, (const unsigned char *)vlow, (int)(lo_bytes / 16), low ? norm : nullptr,
+            w.ids.as<uint32_t>(), n, w.xs.as<float>(), (unsigned char *)w.los.p, w.norms.as<float>());
+        if (cudaGetLastError() != cudaSuccess) rc = -1;
+        // the gathered rows stand in for the table's while the level is built
+        g->d_vecs = w.xs.as<float>();
+        if (low) {
+            g->d_vlow = (decltype(g->d_vlow))w.los.p;
+            g->d_norm = w.norms.as<float>();
+        }
+        g->count = n;
+        g->tmap_x_ok = false;
+        if (!rc) rc = build_level(g, w, M, upper(n), errbuf, errlen);
+        g->d_vecs = vecs;
+        g->d_vlow = vlow;
+        g->d_norm = norm;
+        g->count = count;
+        g->tmap_x_ok = false;
+        if (rc) break;
+        lists.resize(n * (M + 1));
+        if (cudaMemcpy(lists.data(), w.lists.p, lists.size() * 4, cudaMemcpyDeviceToHost) !=
+            cudaSuccess) {
+            rc = -1;
+            break;
+        }
+        for (uint64_t i = 0; i < n; i++) {
+            uint32_t *dst = hnsw_upper_list(h, ids[i], L);
+            const uint32_t *src = &lists[i * (M + 1)];
+            dst[0] = src[0];
+            for (uint32_t j = 0; j < src[0]; j++) dst[1 + j] = ids[src[1 + j]];
+        }
+    }
+    return rc;
 }
 
 }  // namespace
@@ -521,65 +671,14 @@ extern "C" PvHnsw *pv_hnsw_build_gpu(const float *vectors, uint64_t count, int d
         pv_hnsw_free(h);
         return nullptr;
     };
-    // level 0: all rows, R = 2M
-    {
-        FvGpuIndex *g = fv_gpu_index_upload(vectors, nullptr, nullptr, nullptr, 0, count, dim, 0,
-                                            device, precision, errbuf, errlen);
-        if (!g) return fail();
-        int rc = 0;
-        uint32_t *d_lists = nullptr;
-        const int R = 2 * M;
-        {
-            std::lock_guard<std::mutex> lk(g->mu);
-            if (cudaMalloc(&d_lists, (size_t)count * (R + 1) * 4) != cudaSuccess) rc = -1;
-            if (!rc) rc = build_level(g, R, candidates, d_lists, errbuf, errlen);
-            if (!rc && cudaMemcpy(hnsw_l0(h), d_lists, (size_t)count * (R + 1) * 4,
-                                  cudaMemcpyDeviceToHost) != cudaSuccess)
-                rc = -1;
-        }
-        if (d_lists) cudaFree(d_lists);
-        fv_gpu_index_free(g);
-        if (rc) {
-            if (errbuf && errlen && !errbuf[0]) snprintf(errbuf, errlen, "hnsw gpu: level 0 failed");
-            return fail();
-        }
-    }
-    // levels 1..top: the nodes of each level, R = M
-    for (int L = 1; L <= top; L++) {
-        std::vector<uint32_t> ids;
-        for (uint64_t i = 0; i < count; i++)
-            if (lev[i] >= L) ids.push_back((uint32_t)i);
-        const uint64_t n = ids.size();
-        if (n < 2) continue;  // a single node has no neighbours
-        std::vector<float> sub(n * (uint64_t)dim);
-        for (uint64_t i = 0; i < n; i++)
-            memcpy(&sub[i * dim], vectors + (uint64_t)ids[i] * dim, sizeof(float) * dim);
-        FvGpuIndex *g = fv_gpu_index_upload(sub.data(), nullptr, nullptr, nullptr, 0, n, dim, 0,
-                                            device, precision, errbuf, errlen);
-        if (!g) return fail();
-        const int R = M;
-        // upper levels are small: twice the candidates (exact FP32 scans)
-        const int C = (int)std::min<uint64_t>((uint64_t)std::min(2 * candidates + 1, 1023), n - 1);
-        std::vector<uint32_t> lists(n * (R + 1));
-        uint32_t *d_lists = nullptr;
-        int rc = 0;
-        {
-            std::lock_guard<std::mutex> lk(g->mu);
-            if (cudaMalloc(&d_lists, lists.size() * 4) != cudaSuccess) rc = -1;
-            if (!rc) rc = build_level(g, R, C, d_lists, errbuf, errlen);
-            if (!rc && cudaMemcpy(lists.data(), d_lists, lists.size() * 4,
-                                  cudaMemcpyDeviceToHost) != cudaSuccess)
-                rc = -1;
-        }
-        if (d_lists) cudaFree(d_lists);
-        fv_gpu_index_free(g);
-        if (rc) return fail();
-        for (uint64_t i = 0; i < n; i++) {
-            uint32_t *dst = hnsw_upper_list(h, ids[i], L);
-            const uint32_t *src = &lists[i * (R + 1)];
-            dst[0] = src[0];
-            for (uint32_t j = 0; j < src[0]; j++) dst[1 + j] = ids[src[1 + j]];
-        }
+    FvGpuIndex *g = fv_gpu_index_upload(vectors, nullptr, nullptr, nullptr, 0, count, dim, 0,
+                                        device, precision, errbuf, errlen);
+    if (!g) return fail();
+    const int rc = build_levels(h, g, M, candidates, top, errbuf, errlen);
+    fv_gpu_index_free(g);
+    if (rc) {
+        if (errbuf && errlen && !errbuf[0]) snprintf(errbuf, errlen, "hnsw gpu: build failed");
+        return fail();
     }
     hnsw_set_entry(h, entry, top, candidates);
     return h;
