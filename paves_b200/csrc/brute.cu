@@ -376,11 +376,16 @@ int tc_redo_uncertain(FvGpuIndex *g, int nq, const float *queries, const PredBat
     g->last_uncertain = 0;
     if (!g->tc_unc) return 0;
     std::vector<uint8_t> unc((size_t)nq);
-    PV_CUDA_OK(cudaMemcpyAsync(unc.data(), g->tc_unc, (size_t)nq, cudaMemcpyDeviceToHost,
-                               g->stream),
-               errbuf, errlen);
-    PV_CUDA_OK(cudaStreamSynchronize(g->stream), errbuf, errlen);
+    if (g->tc_unc_h) {  // came with the results
+        memcpy(unc.data(), g->tc_unc_h, (size_t)nq);
+    } else {
+        PV_CUDA_OK(cudaMemcpyAsync(unc.data(), g->tc_unc, (size_t)nq, cudaMemcpyDeviceToHost,
+                                   g->stream),
+                   errbuf, errlen);
+        PV_CUDA_OK(cudaStreamSynchronize(g->stream), errbuf, errlen);
+    }
     g->tc_unc = nullptr;
+    g->tc_unc_h = nullptr;
     return redo_flagged(g, nq, queries, pb, topb, unc.data(), out, out_cnt, truncated, errbuf,
                         errlen);
 }
@@ -434,7 +439,7 @@ int brute_run_host(FvGpuIndex *g, int nq, const float *queries, const PredBatch 
     const size_t off_tr = off_cnt + al256((size_t)nq * 4);
     const size_t obytes = off_tr + al256((size_t)nq);
     PV_CUDA_OK(g->scan.out_d.ensure(obytes), errbuf, errlen);
-    PV_CUDA_OK(g->scan.out_h.ensure(obytes + 256), errbuf, errlen);  // + the watchdog word
+    PV_CUDA_OK(g->scan.out_h.ensure(obytes + tc_tail_bytes(nq)), errbuf, errlen);
     char *od = g->scan.out_d.as<char>();
     if (brute_upload(g, db, errbuf, errlen)) return -1;
     cudaEventRecord(g->ev0, g->stream);
@@ -444,7 +449,7 @@ int brute_run_host(FvGpuIndex *g, int nq, const float *queries, const PredBatch 
     cudaEventRecord(g->ev1, g->stream);
     PV_CUDA_OK(cudaMemcpyAsync(g->scan.out_h.p, od, obytes, cudaMemcpyDeviceToHost, g->stream),
                errbuf, errlen);
-    tc_watchdog_enqueue(g, (int *)(g->scan.out_h.as<char>() + obytes));
+    tc_tail_enqueue(g, g->scan.out_h.as<char>() + obytes);
     PV_CUDA_OK(cudaStreamSynchronize(g->stream), errbuf, errlen);
     if (check_tc_watchdog(g, errbuf, errlen)) return -1;
     cudaEventElapsedTime(&g->last_kernel_ms, g->ev0, g->ev1);

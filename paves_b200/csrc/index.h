@@ -134,6 +134,7 @@ struct FvGpuIndex {
     int *tc_err_h = nullptr;  // its copy in pinned memory, queued with the results
     uint8_t *tc_unc = nullptr;  // per query: superset not certified (last TC scan)
     int tc_unc_n = 0;
+    const uint8_t *tc_unc_h = nullptr;  // their copy in pinned memory, like tc_err_h
     int last_uncertain = 0;  // queries of the last call re-run exactly (or flagged)
     // tensor-core scan shape overrides (0 = built-in choice): epilogue warp
     // groups, pipeline stages, CTAs along the rows per query tile

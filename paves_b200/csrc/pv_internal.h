@@ -241,9 +241,12 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
 // Reads and clears the watchdog word of the last tensor-core scan after the
 // stream was synchronized; -1 + errbuf if a bounded wait expired.
 int check_tc_watchdog(FvGpuIndex *g, char *errbuf, size_t errlen);
-// Queues the watchdog word's copy into pinned h_word on g's stream (after
-// the results' copy); the next check_tc_watchdog reads it there.
-void tc_watchdog_enqueue(FvGpuIndex *g, int *h_word);
+// The tail of a tensor-core scan: its watchdog word, then nq uncertain flags.
+constexpr size_t TC_TAIL_UNC = 256;
+inline size_t tc_tail_bytes(int nq) { return TC_TAIL_UNC + (size_t)nq; }
+// Queues its copy into pinned h on g's stream (after the results' copy); the
+// next check_tc_watchdog and the re-run read it there.
+void tc_tail_enqueue(FvGpuIndex *g, char *h);
 
 // ---- HNSW sections (hnsw_build.cpp) for the GPU builder (hnsw_gpu.cu)
 }  // namespace pv

@@ -1084,7 +1084,7 @@ extern "C" int pv_routed_batch(FvGpuIndex *g, PvRouter *r, int nq, const float *
     const size_t pb8 = plan ? 0 : (size_t)nq * r->ncent * 4;  // centroid distances
     const size_t gbytes = have_graph ? graph_out_layout(nq, FV_GPU_MAX_EF).bytes : 0;
     RT_OK(s.out_d.ensure(obytes));
-    RT_OK(s.out_h.ensure(obytes));
+    RT_OK(s.out_h.ensure(obytes + tc_tail_bytes(nq)));
     RT_OK(g->graph.route.ensure(fb + zb + eb + pb8));
     RT_OK(g->graph.route_h.ensure(eb + gbytes));
     if (have_graph) RT_OK(g->graph.gout.ensure(gbytes));
@@ -1133,8 +1133,8 @@ extern "C" int pv_routed_batch(FvGpuIndex *g, PvRouter *r, int nq, const float *
             return -1;
         RT_OK(cudaEventRecord(ev[3], g->stream));
         RT_OK(cudaMemcpyAsync(s.out_h.p, od, obytes, cudaMemcpyDeviceToHost, g->stream));
-        // the watchdog word rides behind the results (the spare tail of out_h)
-        tc_watchdog_enqueue(g, (int *)(s.out_h.as<char>() + obytes - 64));
+        // the watchdog word and the certificates ride behind the results
+        tc_tail_enqueue(g, s.out_h.as<char>() + obytes);
     } else {
         RT_OK(cudaEventRecord(ev[1], g->stream));
     }
@@ -1220,9 +1220,13 @@ extern "C" int pv_routed_batch(FvGpuIndex *g, PvRouter *r, int nq, const float *
         // scan-routed queries whose reduced-precision superset the merge
         // could not certify are re-run exactly
         std::vector<uint8_t> unc(nq), tr(nq);
-        RT_OK(cudaMemcpyAsync(unc.data(), g->tc_unc, (size_t)nq, cudaMemcpyDeviceToHost,
-                              g->stream));
-        RT_OK(cudaStreamSynchronize(g->stream));
+        if (g->tc_unc_h) {
+            memcpy(unc.data(), g->tc_unc_h, (size_t)nq);
+        } else {
+            RT_OK(cudaMemcpyAsync(unc.data(), g->tc_unc, (size_t)nq, cudaMemcpyDeviceToHost,
+                                  g->stream));
+            RT_OK(cudaStreamSynchronize(g->stream));
+        }
         for (int q = 0; q < nq; q++)
             if (hefq[q] > 0) unc[q] = 0;
         if (redo_flagged(g, nq, queries, pb, topb, unc.data(), out, out_cnt, tr.data(), errbuf,
@@ -1232,6 +1236,7 @@ extern "C" int pv_routed_batch(FvGpuIndex *g, PvRouter *r, int nq, const float *
             if (out_cnt[q] > k[q]) out_cnt[q] = k[q];
     }
     g->tc_unc = nullptr;
+    g->tc_unc_h = nullptr;
     if (ngraph > 0) done = ev[4];
     // device time of the batch: the bitmaps, then the search with the
     // routing's tail beside it (t[1]: the routing after the bitmaps; the

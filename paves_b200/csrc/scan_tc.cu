@@ -487,11 +487,12 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const size_t off_qn = (qbytes + 255) & ~(size_t)255;
     const size_t off_qs = off_qn + (((size_t)nqpad * 4 + 255) & ~(size_t)255);
     const size_t off_err = off_qs + (((size_t)nqpad * 4 + 255) & ~(size_t)255);
-    const size_t off_cand = off_err + 256;
+    // (the flags lie behind the watchdog word: one copy brings both)
+    const size_t off_unc = off_err + TC_TAIL_UNC;
+    const size_t off_cand = off_unc + (((size_t)nq + 255) & ~(size_t)255);
     const size_t off_ccnt = off_cand + (((size_t)nq * S * sizeof(FvHit) + 255) & ~(size_t)255);
     const size_t off_ctr = off_ccnt + (((size_t)nq * 4 + 255) & ~(size_t)255);
-    const size_t off_unc = off_ctr + (((size_t)nq + 255) & ~(size_t)255);
-    const size_t cbytes = off_unc + (size_t)nq + 256;
+    const size_t cbytes = off_ctr + (size_t)nq + 256;
     PV_CUDA_OK(s.cand.ensure(cbytes), errbuf, errlen);
     PV_CUDA_OK(s.tau.ensure((size_t)nq * 8), errbuf, errlen);
     const size_t smem = tc_smem(kblocks, NS, KP, EPI);
@@ -706,7 +707,8 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     g->tc_unc_n = nq;
     if (ev) cudaEventRecord(ev[3], g->stream);
     g->tc_err = d_err;
-    g->tc_err_h = nullptr;  // its host copy, if any, is queued by the caller
+    g->tc_err_h = nullptr;  // their host copy, if any, is queued by the caller
+    g->tc_unc_h = nullptr;
     if (tracing && d_trace) {
         uint64_t h[64 * 4];
         cudaStreamSynchronize(g->stream);
@@ -723,15 +725,21 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
 }  // namespace pv
 
 namespace pv {
-// Queues the copy of the watchdog word into pinned host memory behind the
-// batch's own result copy, so reading it costs no extra round trip.
-void tc_watchdog_enqueue(FvGpuIndex *g, int *h_word) {
+// Queues the copy of the watchdog word and, where the scan certifies, its
+// nq flags into pinned host memory (tc_tail_bytes(nq)) behind the batch's own
+// result copy, so reading them costs no extra round trip (two copies into
+// pageable memory with a synchronization each took 15 us of a batch).
+void tc_tail_enqueue(FvGpuIndex *g, char *h) {
     g->tc_err_h = nullptr;
+    g->tc_unc_h = nullptr;
     if (!g->tc_err) return;
-    if (cudaMemcpyAsync(h_word, g->tc_err, 4, cudaMemcpyDeviceToHost, g->stream) == cudaSuccess)
-        g->tc_err_h = h_word;
-    else
+    const size_t bytes = g->tc_unc ? TC_TAIL_UNC + (size_t)g->tc_unc_n : sizeof(int);
+    if (cudaMemcpyAsync(h, g->tc_err, bytes, cudaMemcpyDeviceToHost, g->stream) != cudaSuccess) {
         (void)cudaGetLastError();
+        return;
+    }
+    g->tc_err_h = (int *)h;
+    if (g->tc_unc) g->tc_unc_h = (const uint8_t *)h + TC_TAIL_UNC;
 }
 
 int check_tc_watchdog(FvGpuIndex *g, char *errbuf, size_t errlen) {

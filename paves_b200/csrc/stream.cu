@@ -51,8 +51,10 @@ struct Bucket {
     // tuned plan
     int mode = PV_MODE_EXACT, epi = 0, ns = 0, grow = 0;
     float ms = 0.f;
-    const uint8_t *d_unc = nullptr;  // certificate flags of the TC merge (if any)
-    int *d_err = nullptr;            // watchdog word of the TC scan (if any)
+    int *d_err = nullptr;  // watchdog word of the TC scan (if any)
+    // in out_h, behind the results: its copy, the TC merge's certificate flags
+    int *h_err = nullptr;
+    const uint8_t *h_unc = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
 
@@ -103,7 +105,7 @@ void layout(Bucket &b, const FvGpuIndex *g) {
 int alloc(Bucket &b, char *errbuf, size_t errlen) {
     PV_CUDA_OK(b.stage_h.ensure(b.db.bytes), errbuf, errlen);
     PV_CUDA_OK(b.stage_d.ensure(b.db.bytes), errbuf, errlen);
-    PV_CUDA_OK(b.out_h.ensure(b.obytes), errbuf, errlen);
+    PV_CUDA_OK(b.out_h.ensure(b.obytes + tc_tail_bytes(b.B)), errbuf, errlen);
     PV_CUDA_OK(b.out_d.ensure(b.obytes), errbuf, errlen);
     memset(b.stage_h.p, 0, b.db.bytes);
     return 0;
@@ -165,10 +167,16 @@ int enqueue(PvStream *s, Bucket &b, char *errbuf, size_t errlen) {
     if (brute_launch(v, b.db, b.topb, b.mode, (FvHit *)od, (uint32_t *)(od + b.o_cnt),
                      (uint8_t *)(od + b.o_tr), errbuf, errlen))
         return -1;
-    b.d_unc = v->tc_unc;
     b.d_err = v->tc_err;
     PV_CUDA_OK(cudaMemcpyAsync(b.out_h.p, od, b.obytes, cudaMemcpyDeviceToHost, v->stream),
                errbuf, errlen);
+    tc_tail_enqueue(v, b.out_h.as<char>() + b.obytes);
+    b.h_err = v->tc_err_h;
+    b.h_unc = v->tc_unc_h;
+    if (v->tc_err && (!b.h_err || (v->tc_unc && !b.h_unc))) {
+        snprintf(errbuf, errlen, "stream: result copy failed");
+        return -1;
+    }
     return 0;
 }
 
@@ -434,6 +442,7 @@ extern "C" int pv_stream_run(PvStream *s, int nq, const float *queries, const Fv
     PV_CUDA_OK(cudaEventRecord(s->e1, v->stream), errbuf, errlen);
     PV_CUDA_OK(cudaStreamSynchronize(v->stream), errbuf, errlen);
     v->tc_err = b->d_err;
+    v->tc_err_h = b->h_err;
     if (check_tc_watchdog(v, errbuf, errlen)) return -1;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, s->e0, s->e1);
@@ -446,12 +455,8 @@ extern "C" int pv_stream_run(PvStream *s, int nq, const float *queries, const Fv
                sizeof(FvHit) * c);
         out_cnt[q] = c;
     }
-    if (b->d_unc) {
-        std::vector<uint8_t> unc(b->B);
-        PV_CUDA_OK(cudaMemcpyAsync(unc.data(), b->d_unc, (size_t)b->B, cudaMemcpyDeviceToHost,
-                                   v->stream),
-                   errbuf, errlen);
-        PV_CUDA_OK(cudaStreamSynchronize(v->stream), errbuf, errlen);
+    if (b->h_unc) {
+        const std::vector<uint8_t> unc(b->h_unc, b->h_unc + b->B);
         int n = 0;
         for (int q = 0; q < nq; q++) n += unc[q] ? 1 : 0;
         if (n) {
