@@ -48,14 +48,19 @@ cudaError_t launch_bitmaps_rank(const FvGpuIndex *g, const PredInsn *insns, cons
 // popcnt[qprog[q]] or nrows), tau_out[q] = min(tau_out[q], KO-th key) and
 // unc[q] (a full list's last key, fullmin[q], at or below the answer's end;
 // or, with an estimated bound, fewer than KO keys at or below it).
-// late_counts: the kernel ahead on the stream writes popcnt.
+// late_counts: the kernel ahead on the stream writes popcnt. mode: a caller
+// that needs less than that says so (KO > 32 then takes a shorter way).
+// DM_SET: the answer in any order but the largest key last (a superset to
+// re-rank); DM_BOUND: only tau_out (a seeding sample).
+constexpr int DM_SORTED = 0, DM_SET = 1, DM_BOUND = 2;
 cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *dcnt,
                                bool reset_cnt, const unsigned long long *fullmin,
                                const unsigned long long *tau, int KO, const int32_t *qprog,
                                const unsigned long long *popcnt, uint64_t nrows, int nq,
                                FvHit *out, uint32_t *out_cnt, uint8_t *trunc,
                                unsigned long long *tau_out, uint8_t *unc, cudaStream_t st,
-                               bool estimated = false, bool late_counts = false);
+                               bool estimated = false, bool late_counts = false,
+                               int mode = DM_SORTED);
 
 // ---- exact FP32 scan (scan_f32.cu)
 struct ScanF32Args {

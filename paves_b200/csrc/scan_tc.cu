@@ -117,8 +117,9 @@ __global__ void query_prep_kernel(const float *__restrict__ q, int nq, int dpad,
 // ---------------------------------------------------------------- re-rank
 // Exact FP32 distances (difference form) for each query's merged candidates
 // (up to TC_MAX_SUPERSET, row stride S); keeps the best topb by (dist, id).
-// One CTA (8 warps) per query: 8 lanes per candidate, 32 candidates in
-// flight, then a bitonic sort of the keys in shared memory.
+// One CTA (8 warps) per query: 8 lanes per candidate, 128 candidates in
+// flight (random rows of 512 bytes: latency, then bandwidth), then a bitonic
+// sort of the keys.
 template <int ORDER>
 __global__ void __launch_bounds__(256)
 rerank_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict__ queries,
@@ -140,8 +141,8 @@ rerank_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict_
 // below the grid-wide bound can be in the answer. Keys are unique 64-bit
 // (distance bits, row) values, so the KO-th smallest is found exactly by a
 // radix select, 8 bits per pass (a histogram of the digit among the keys
-// that share the digits chosen so far), and only the at most KO keys at or
-// below it are sorted. Runs up to stage_cap keys are staged in shared
+// that share the digits chosen so far) until few are left, and only the at
+// most KO keys at or below it are sorted, if they need to be. Runs up to stage_cap keys are staged in shared
 // memory; longer ones are read from global memory on every pass (4 loads
 // in flight per lane).
 __global__ void __launch_bounds__(DM_THREADS)
@@ -152,18 +153,16 @@ dense_merge_kernel(const uint64_t *__restrict__ dense, uint64_t dcap, int stage_
                    const unsigned long long *__restrict__ popcnt, uint64_t nrows,
                    FvHit *__restrict__ out, uint32_t *__restrict__ out_cnt,
                    uint8_t *__restrict__ trunc, unsigned long long *tau_out,
-                   uint8_t *__restrict__ unc, int estimated) {
+                   uint8_t *__restrict__ unc, int estimated, int mode) {
     extern __shared__ __align__(16) unsigned char dm_smem[];
     pdl_wait();
     pdl_trigger();
     dense_merge_query(blockIdx.x, (uint64_t *)dm_smem, dense, dcap, stage_cap, dcnt, reset_cnt,
                       fullmin, tau, KO, qprog, popcnt, nrows, out, out_cnt, trunc, tau_out, unc,
-                      estimated != 0);
+                      estimated != 0, mode);
 }
 
-// KO <= 32 W; measured at KO = 64 over 2048 runs of about 500 keys: 0.021 ms
-// against the radix select's 0.107.
-template <int W>
+// KO <= 32
 __global__ void __launch_bounds__(DM_THREADS)
 dense_top32_kernel(const uint64_t *__restrict__ dense, uint64_t dcap, uint32_t *__restrict__ dcnt,
                    int reset_cnt, const unsigned long long *__restrict__ fullmin,
@@ -172,7 +171,7 @@ dense_top32_kernel(const uint64_t *__restrict__ dense, uint64_t dcap, uint32_t *
                    FvHit *__restrict__ out, uint32_t *__restrict__ out_cnt,
                    uint8_t *__restrict__ trunc, unsigned long long *tau_out,
                    uint8_t *__restrict__ unc, int estimated, int late_counts) {
-    __shared__ uint64_t lists[DM_THREADS / 32][32 * W];
+    __shared__ uint64_t lists[DM_THREADS / 32][32];
     // the batch's programs and the bitmap kernel's counts were written two
     // or more kernels back (each kernel of the chain triggers the next only
     // after its own wait): read them while the kernel ahead finishes, unless
@@ -184,7 +183,7 @@ dense_top32_kernel(const uint64_t *__restrict__ dense, uint64_t dcap, uint32_t *
     }
     pdl_wait();
     pdl_trigger();
-    dense_top32_query<W>(blockIdx.x, lists, dense, dcap, dcnt, reset_cnt, fullmin, tau, KO, qprog,
+    dense_top32_query(blockIdx.x, lists, dense, dcap, dcnt, reset_cnt, fullmin, tau, KO, qprog,
                          popcnt, nrows, out, out_cnt, trunc, tau_out, unc, passing,
                          estimated != 0);
 }
@@ -195,14 +194,18 @@ cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *d
                                const unsigned long long *popcnt, uint64_t nrows, int nq,
                                FvHit *out, uint32_t *out_cnt, uint8_t *trunc,
                                unsigned long long *tau_out, uint8_t *unc, cudaStream_t st,
-                               bool estimated, bool late_counts) {
+                               bool estimated, bool late_counts, int mode) {
     if (KO < 1 || KO > DM_OUT) return cudaErrorInvalidValue;
-    if (KO <= 64) {
-        auto *kern = KO <= 32 ? dense_top32_kernel<1> : dense_top32_kernel<2>;
-        return launch_pdl(kern, dim3(nq), dim3(DM_THREADS), 0, st, dense, dcap, dcnt,
+    // The warps' lists where they hold the answer (KO 10 of 2048 runs of 200
+    // and 1,000 keys: 0.0205 and 0.0225 ms, the radix select 0.031 and 0.033),
+    // else the radix select (KO 48 of 1,000 keys: 0.045 ms, lists of 64 0.065;
+    // KO 400 of 512 runs of 1,500 keys with the re-rank: 0.056 ms; with all
+    // eight digits, a sort of 45 barriers and 32 candidates of a query in
+    // flight 0.097).
+    if (KO <= 32)
+        return launch_pdl(dense_top32_kernel, dim3(nq), dim3(DM_THREADS), 0, st, dense, dcap, dcnt,
                           reset_cnt ? 1 : 0, fullmin, tau, KO, qprog, popcnt, nrows, out, out_cnt,
                           trunc, tau_out, unc, estimated ? 1 : 0, late_counts ? 1 : 0);
-    }
     // the stage holds a whole run when it can (runs never exceed dcap)
     const int stage_cap = (int)std::min<uint64_t>(std::max<uint64_t>(dcap, 1), DM_CAP_MAX);
     const size_t smem = (size_t)(stage_cap + DM_OUT) * 8;
@@ -210,7 +213,7 @@ cudaError_t launch_dense_merge(const uint64_t *dense, uint64_t dcap, uint32_t *d
     if (e != cudaSuccess) return e;
     return launch_pdl(dense_merge_kernel, dim3(nq), dim3(DM_THREADS), smem, st, dense, dcap,
                       stage_cap, dcnt, reset_cnt ? 1 : 0, fullmin, tau, KO, qprog, popcnt, nrows,
-                      out, out_cnt, trunc, tau_out, unc, estimated ? 1 : 0);
+                      out, out_cnt, trunc, tau_out, unc, estimated ? 1 : 0, mode);
 }
 
 // ---------------------------------------------------------------- host side
@@ -654,7 +657,8 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         // the merge leaves the counts at zero for the main pass
         PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, true, nullptr, a.tau, rank, d_qprog,
                                       popcnt, g->count, nq, cand, ccnt,
-                                      (uint8_t *)(c + off_ctr), a.tau, nullptr, g->stream),
+                                      (uint8_t *)(c + off_ctr), a.tau, nullptr, g->stream, false,
+                                      false, DM_BOUND),
                    errbuf, errlen);
     }
     // stage boundary: everything before the main pass (bitmaps, query prep,
@@ -681,7 +685,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         PV_CUDA_OK(launch_dense_merge(a.dense, dcap, d_dcnt, false, a.fullmin, a.tau, S,
                                       d_qprog, popcnt, g->count, nq, cand, ccnt,
                                       (uint8_t *)(c + off_ctr), nullptr, d_unc, g->stream,
-                                      seed && estimated),
+                                      seed && estimated, false, DM_SET),
                    errbuf, errlen);
         RerankCert cert;
         if (num_cert) {

@@ -790,6 +790,42 @@ __device__ __forceinline__ void query_prep_row(int qi, int lane, const float *__
     }
 }
 
+// Ascending bitonic sort of n2 (a power of two >= 32) keys in shared memory
+// by a block of whole warps; compare distances below 32 run on a warp's
+// registers, so 512 keys take 15 barriers, not 45. Ends synchronized.
+__device__ __forceinline__ void block_sort(uint64_t *keys, int n2) {
+    const int tid = threadIdx.x, nt = (int)blockDim.x;
+    for (int k = 32; k <= n2; k <<= 1) {
+        for (int j = k >> 1; j >= 32; j >>= 1) {
+            for (int i = tid; i < (n2 >> 1); i += nt) {
+                const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1));
+                const int hi = lo | j;
+                const uint64_t x = keys[lo], y = keys[hi];
+                if ((x > y) == ((lo & k) == 0)) {
+                    keys[lo] = y;
+                    keys[hi] = x;
+                }
+            }
+            __syncthreads();
+        }
+        for (int i = tid; i < n2; i += nt) {
+            uint64_t x = keys[i];
+#pragma unroll
+            for (int kk = 2; kk <= 32; kk <<= 1) {  // the first time all of it
+                if (kk < 32 && k > 32) continue;
+                const int d = kk < 32 ? kk : k;  // direction bit
+#pragma unroll
+                for (int j = kk >> 1; j > 0; j >>= 1) {
+                    const uint64_t o = __shfl_xor_sync(0xffffffffu, x, j);
+                    x = ((i & j) == 0) == ((i & d) == 0) ? (x < o ? x : o) : (x > o ? x : o);
+                }
+            }
+            keys[i] = x;
+        }
+        __syncthreads();
+    }
+}
+
 // The numerical certificate of a re-ranked superset whose scan distances
 // were inexact (f32 rows read as TF32): qnorm = null turns it off.
 //
@@ -906,44 +942,50 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
             }
             keys[j] = make_key(even + odd, row);
         }
-    for (int base = 0; ORDER == RR_LANES8 && base < n; base += NT / 8) {
-        const int j = base + grp;
-        const bool ok = j < n;
-        const uint32_t row = (uint32_t)cand[(size_t)q * S + (ok ? j : 0)].node;
-        const float *x = vecs + (size_t)row * dpad;
-        float acc = 0.f;
-        for (int k = sub * 4; k < dpad; k += 32) {
-            const float4 v = __ldg((const float4 *)(x + k));
-            const float4 w = __ldg((const float4 *)(qv + k));
-            const float d0 = v.x - w.x, d1 = v.y - w.y, d2 = v.z - w.z, d3 = v.w - w.w;
-            acc = fmaf(d0, d0, acc);
-            acc = fmaf(d1, d1, acc);
-            acc = fmaf(d2, d2, acc);
-            acc = fmaf(d3, d3, acc);
+    if (ORDER == RR_LANES8) {
+        constexpr int U = 4;  // candidates of a group in flight
+        for (int base = grp; base < n; base += NT / 8 * U) {
+            uint32_t row[U];
+            float acc[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int j = base + u * (NT / 8);
+                row[u] = (uint32_t)cand[(size_t)q * S + (j < n ? j : base)].node;
+                acc[u] = 0.f;
+            }
+#pragma unroll 2
+            for (int k = sub * 4; k < dpad; k += 32) {
+                const float4 w = __ldg((const float4 *)(qv + k));
+                float4 v[U];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    v[u] = __ldg((const float4 *)(vecs + (size_t)row[u] * dpad + k));
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const float d0 = v[u].x - w.x, d1 = v[u].y - w.y, d2 = v[u].z - w.z,
+                                d3 = v[u].w - w.w;
+                    acc[u] = fmaf(d0, d0, acc[u]);
+                    acc[u] = fmaf(d1, d1, acc[u]);
+                    acc[u] = fmaf(d2, d2, acc[u]);
+                    acc[u] = fmaf(d3, d3, acc[u]);
+                }
+            }
+            const unsigned lanes = 0xffu << (threadIdx.x & 24);  // the group's
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                acc[u] += __shfl_xor_sync(lanes, acc[u], 4);
+                acc[u] += __shfl_xor_sync(lanes, acc[u], 2);
+                acc[u] += __shfl_xor_sync(lanes, acc[u], 1);
+                const int j = base + u * (NT / 8);
+                if (j < n && sub == 0) keys[j] = make_key(acc[u], row[u]);
+            }
         }
-        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-        if (ok && sub == 0) keys[j] = make_key(acc, row);
     }
-    int n2 = 1;
+    int n2 = 32;
     while (n2 < n) n2 <<= 1;
     for (int i = n + tid; i < n2; i += blockDim.x) keys[i] = KEY_MAX;
     __syncthreads();
-    for (int k = 2; k <= n2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = tid; i < (n2 >> 1); i += blockDim.x) {
-                const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1));
-                const int hi = lo | j;
-                const uint64_t x = keys[lo], y = keys[hi];
-                if ((x > y) == ((lo & k) == 0)) {
-                    keys[lo] = y;
-                    keys[hi] = x;
-                }
-            }
-            __syncthreads();
-        }
-    }
+    block_sort(keys, n2);
     const int nout = n < (int)topb ? n : (int)topb;
     for (int i = tid; i < nout; i += blockDim.x) {
         FvHit h;
@@ -975,26 +1017,27 @@ constexpr int DM_THREADS = 512;
 constexpr int DM_CAP_MAX = 24576;   // largest shared-memory stage
 constexpr int DM_OUT = TC_MAX_SUPERSET;
 
-__device__ __forceinline__ void dm_hist_add(unsigned *hist, bool act, unsigned d, int lane) {
-    const int tag = act ? (int)d : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, tag);
-    if (act && lane == __ffs(peers) - 1) atomicAdd(&hist[d], (unsigned)__popc(peers));
-}
-
 // One query's merge (radix select, any KO <= DM_OUT) by all threads of the
 // block; smem_keys: stage_cap + DM_OUT keys of shared memory. Ends with the
-// block synchronized.
+// block synchronized. The keys' common leading bits are skipped (of a float
+// distance the first 9 or so), and once the KO-th key's bucket is down to
+// DM_FEW keys those are ranked by counting: one or two digits of 8 bits
+// instead of eight (measured at launch_dense_merge).
+constexpr int DM_FEW = 128;
+
 static __device__ __noinline__ void dense_merge_query(
     int q, uint64_t *smem_keys, const uint64_t *__restrict__ dense, uint64_t dcap, int stage_cap,
     uint32_t *__restrict__ dcnt, int reset_cnt, const unsigned long long *__restrict__ fullmin,
     const unsigned long long *tau, int KO, const int32_t *__restrict__ qprog,
     const unsigned long long *__restrict__ popcnt, uint64_t nrows, FvHit *__restrict__ out,
     uint32_t *__restrict__ out_cnt, uint8_t *__restrict__ trunc, unsigned long long *tau_out,
-    uint8_t *__restrict__ unc, bool estimated = false) {
+    uint8_t *__restrict__ unc, bool estimated = false, int mode = DM_SORTED) {
     uint64_t *buf = smem_keys;        // [stage_cap] staged keys
-    uint64_t *res = buf + stage_cap;  // [DM_OUT] the answer, sorted
+    uint64_t *res = buf + stage_cap;  // [DM_OUT] the answer
     __shared__ unsigned hist[256];
-    __shared__ int s_m, s_c, s_digit, s_rank, s_tot;
+    __shared__ unsigned long long s_min, s_max, s_kth;
+    uint64_t *s_few = res;  // (before the answer)
+    __shared__ int s_m, s_c, s_digit, s_rank, s_bucket, s_nfew;
     const int NW = blockDim.x >> 5;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned long long bound = tau ? tau[q] : KEY_MAX;
@@ -1004,48 +1047,86 @@ static __device__ __noinline__ void dense_merge_query(
     if (tid == 0) {
         s_m = 0;
         s_c = 0;
+        s_min = KEY_MAX;
+        s_max = 0;
+        s_kth = KEY_MAX;
     }
     __syncthreads();
     if (reset_cnt && tid == 0) dcnt[q] = 0;  // every thread has read it
     const bool staged = n <= (uint64_t)stage_cap;
-    if (staged) {
-        for (uint64_t b = (uint64_t)warp * 32; b < n; b += NW * 32) {
-            const uint64_t i = b + lane;
-            const uint64_t key = i < n ? src[i] : KEY_MAX;
-            const bool keep = i < n && key <= bound;
-            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            int base = 0;
-            if (lane == 0 && bal) base = atomicAdd(&s_m, __popc(bal));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (keep) buf[base + __popc(bal & ((1u << lane) - 1u))] = key;
+    {   // the candidates' number and range; staged: compacted into buf
+        uint64_t mn = KEY_MAX, mx = 0;
+        int cnt = 0;
+        for (uint64_t b = (uint64_t)warp * 128; b < n; b += NW * 128) {
+            uint64_t key[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint64_t i = b + u * 32 + lane;
+                key[u] = i < n ? src[i] : KEY_MAX;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const bool keep = b + u * 32 + lane < n && key[u] <= bound;
+                const unsigned bal = __ballot_sync(0xffffffffu, keep);
+                cnt += __popc(bal);
+                if (keep) {
+                    mn = key[u] < mn ? key[u] : mn;
+                    mx = key[u] > mx ? key[u] : mx;
+                }
+                if (staged && bal) {
+                    int base = 0;
+                    if (lane == 0) base = atomicAdd(&s_m, __popc(bal));
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    if (keep) buf[base + __popc(bal & ((1u << lane) - 1u))] = key[u];
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const uint64_t a = __shfl_xor_sync(0xffffffffu, mn, o),
+                           z = __shfl_xor_sync(0xffffffffu, mx, o);
+            mn = a < mn ? a : mn;
+            mx = z > mx ? z : mx;
+        }
+        if (lane == 0 && cnt) {
+            if (!staged) atomicAdd(&s_m, cnt);
+            atomicMin(&s_min, (unsigned long long)mn);
+            atomicMax(&s_max, (unsigned long long)mx);
         }
     }
     __syncthreads();
     // candidates: buf[0, s_m) if staged, else the keys <= bound of src[0, n)
-    const uint64_t N = staged ? (uint64_t)s_m : n;
-    uint64_t kth = KEY_MAX;  // keep every candidate unless there are more than KO
-    if (!staged || s_m > KO) {
-        uint64_t prefix = 0;
-        int rank = KO;
-        bool selected = true;
-        for (int pass = 0; pass < 8; pass++) {
-            const int shift = 56 - 8 * pass;
+    const int total = s_m;
+    const uint64_t N = staged ? (uint64_t)total : n;
+    const uint64_t *from = staged ? buf : src;
+    // fn(key, whether it is a candidate), warps together, 4 loads in flight
+    auto each = [&](auto fn) {
+        for (uint64_t b = (uint64_t)warp * 128; b < N; b += NW * 128) {
+            uint64_t key[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint64_t i = b + u * 32 + lane;
+                key[u] = i < N ? from[i] : KEY_MAX;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                fn(key[u], b + u * 32 + lane < N && (staged || key[u] <= bound));
+        }
+    };
+    uint64_t kth = s_max;  // every candidate unless there are more than KO
+    if (total > KO) {
+        const int top = 63 - __clzll((long long)(s_min ^ s_max));  // (keys are unique)
+        int shift = max(top - 7, 0);
+        // bits from `fixed` up are decided and equal prefix's
+        int fixed = top + 1, rank = KO;
+        uint64_t prefix = fixed < 64 ? s_max >> fixed << fixed : 0ull;
+        for (;;) {
             for (int i = tid; i < 256; i += (int)blockDim.x) hist[i] = 0;
             __syncthreads();
-            for (uint64_t b = (uint64_t)warp * 128; b < N; b += NW * 128) {
-                uint64_t key[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const uint64_t i = b + u * 32 + lane;
-                    key[u] = i < N ? (staged ? buf[i] : src[i]) : KEY_MAX;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    bool act = b + u * 32 + lane < N && (staged || key[u] <= bound);
-                    if (pass > 0) act = act && (key[u] >> (shift + 8)) == (prefix >> (shift + 8));
-                    dm_hist_add(hist, act, (unsigned)(key[u] >> shift) & 255u, lane);
-                }
-            }
+            each([&](uint64_t key, bool in) {
+                if (in && (fixed >= 64 || (key ^ prefix) >> fixed == 0))
+                    atomicAdd(&hist[(key >> shift) & 255u], 1u);
+            });
             __syncthreads();
             if (warp == 0) {
                 unsigned c[8], sum = 0;
@@ -1060,66 +1141,78 @@ static __device__ __noinline__ void dense_merge_query(
                     if (lane >= o) incl += v;
                 }
                 const unsigned excl = incl - sum;
-                if (pass == 0 && lane == 31) s_tot = (int)incl;
                 if (excl < (unsigned)rank && (unsigned)rank <= incl) {
                     unsigned cum = excl;
-                    int j = 0;
-                    for (; j < 7; j++) {
-                        if (cum + c[j] >= (unsigned)rank) break;
-                        cum += c[j];
+                    int d = lane * 8;
+                    unsigned here = 0;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        if (here == 0) {
+                            if (cum + c[j] >= (unsigned)rank) {
+                                here = c[j];
+                                d += j;
+                            } else {
+                                cum += c[j];
+                            }
+                        }
                     }
-                    s_digit = lane * 8 + j;
+                    s_digit = d;
                     s_rank = rank - (int)cum;
+                    s_bucket = (int)here;
+                    s_nfew = 0;
                 }
             }
             __syncthreads();
-            if (pass == 0 && s_tot <= KO) {  // no more than KO candidates
-                selected = false;
-                break;
-            }
-            prefix |= (uint64_t)s_digit << shift;
+            prefix = (prefix & ~(255ull << shift)) | (uint64_t)s_digit << shift;
+            fixed = shift;
             rank = s_rank;
+            if (s_bucket <= DM_FEW || shift == 0) break;
+            shift = max(shift - 8, 0);
         }
-        if (selected) kth = prefix;
+        if (s_bucket <= DM_FEW) {  // (else one key: no bits are left)
+            const int few = s_bucket;
+            each([&](uint64_t key, bool in) {
+                if (in && (key ^ prefix) >> fixed == 0) s_few[atomicAdd(&s_nfew, 1)] = key;
+            });
+            __syncthreads();
+            if (tid < few) {
+                const uint64_t key = s_few[tid];
+                int less = 0;
+                for (int j = 0; j < few; j++) less += s_few[j] < key;
+                if (less == rank - 1) s_kth = key;
+            }
+            __syncthreads();
+            kth = s_kth;
+        } else {
+            kth = prefix;
+        }
+    }
+    if (mode == DM_BOUND) {
+        // the KO-th key of the sample bounds the KO-th key of all rows
+        if (tid == 0 && total >= KO && kth < tau_out[q]) tau_out[q] = kth;
+        __syncthreads();
+        return;
     }
     // the answer: candidates <= kth (exactly min(count, KO) keys)
-    for (uint64_t b = (uint64_t)warp * 128; b < N; b += NW * 128) {
-        uint64_t key[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint64_t i = b + u * 32 + lane;
-            key[u] = i < N ? (staged ? buf[i] : src[i]) : KEY_MAX;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const bool keep = b + u * 32 + lane < N && key[u] <= bound && key[u] <= kth;
-            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            int base = 0;
-            if (lane == 0 && bal) base = atomicAdd(&s_c, __popc(bal));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            const int pos = base + __popc(bal & ((1u << lane) - 1u));
-            if (keep && pos < DM_OUT) res[pos] = key[u];
-        }
-    }
+    each([&](uint64_t key, bool in) {
+        const bool keep = in && key <= kth;
+        const bool put = keep && (mode != DM_SET || key != kth);
+        const unsigned bal = __ballot_sync(0xffffffffu, put);
+        int base = 0;
+        if (lane == 0 && bal) base = atomicAdd(&s_c, __popc(bal));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const int pos = base + __popc(bal & ((1u << lane) - 1u));
+        if (put && pos < DM_OUT) res[pos] = key;
+        if (keep && !put) res[min(total, KO) - 1] = key;
+    });
     __syncthreads();
-    const int c = min(min(s_c, KO), DM_OUT);
-    int n2 = 1;
-    while (n2 < c) n2 <<= 1;
-    for (int i = c + tid; i < n2; i += (int)blockDim.x) res[i] = KEY_MAX;
-    __syncthreads();
-    for (int k = 2; k <= n2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = tid; i < (n2 >> 1); i += (int)blockDim.x) {
-                const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1));
-                const int hi = lo | j;
-                const uint64_t x = res[lo], y = res[hi];
-                if ((x > y) == ((lo & k) == 0)) {
-                    res[lo] = y;
-                    res[hi] = x;
-                }
-            }
-            __syncthreads();
-        }
+    const int c = min(min(total, KO), DM_OUT);
+    if (mode == DM_SORTED) {
+        int n2 = 32;
+        while (n2 < c) n2 <<= 1;
+        for (int i = c + tid; i < n2; i += (int)blockDim.x) res[i] = KEY_MAX;
+        __syncthreads();
+        block_sort(res, n2);
     }
     for (int i = tid; i < c; i += (int)blockDim.x) {
         FvHit h;
@@ -1149,13 +1242,14 @@ static __device__ __noinline__ void dense_merge_query(
     __syncthreads();
 }
 
-// The same for KO <= 64, without block barriers in the hot loop: each warp
-// keeps its 32 (64) best keys sorted across its lanes (one or two keys per
-// lane) and folds in 32 new keys at a time (a shuffle bitonic sort of the new keys in
-// descending order, an elementwise min with the list, which leaves the 32
-// smallest as a bitonic sequence, and a bitonic clean back to ascending);
-// a batch none of whose keys beats the list's last key is skipped. The
-// warps' lists then fold pairwise into warp 0's.
+// The same for KO <= 32, without block barriers in the hot loop: each warp
+// keeps its 32 best keys sorted across its lanes and folds in 32 new keys at
+// a time (a shuffle bitonic sort of the new keys in descending order, an
+// elementwise min with the list, which leaves the 32 smallest as a bitonic
+// sequence, and a bitonic clean back to ascending); a batch none of whose
+// keys beats the list's last key is skipped. The warps' lists then fold
+// pairwise into warp 0's. (Lists of 64, two keys a lane, lost to the radix
+// select: 64 queries of 500,000 rows, S 40, 0.0717 against 0.0627 ms.)
 __device__ __forceinline__ uint64_t warp_sort32(uint64_t x, int lane, bool descending) {
 #pragma unroll
     for (int k = 2; k <= 32; k <<= 1)
@@ -1178,10 +1272,8 @@ __device__ __forceinline__ uint64_t warp_clean32(uint64_t x, int lane) {
     return x;
 }
 
-// One query's merge for KO <= 32 W (W 1 or 2 keys per lane, the second the
-// larger half of the list) by all threads of the block (any whole number of
-// warps); lists: one slot per warp in shared memory. Ends with the block
-// synchronized.
+// Folds 32 keys into a warp's ascending list of 32 W (W 1 or 2 keys per lane,
+// the second the larger half of the list).
 template <int W>
 __device__ __forceinline__ void warp_fold32(uint64_t (&best)[W], uint64_t d, int lane) {
     // d: 32 keys, descending across the lanes
@@ -1198,9 +1290,11 @@ __device__ __forceinline__ void warp_fold32(uint64_t (&best)[W], uint64_t d, int
     }
 }
 
-template <int W = 1>
+// One query's merge for KO <= 32 by all threads of the block (any whole number
+// of warps); lists: one slot per warp in shared memory. Ends with the block
+// synchronized.
 __device__ __forceinline__ void dense_top32_query(
-    int q, uint64_t (*lists)[32 * W], const uint64_t *__restrict__ dense, uint64_t dcap,
+    int q, uint64_t (*lists)[32], const uint64_t *__restrict__ dense, uint64_t dcap,
     uint32_t *__restrict__ dcnt, int reset_cnt, const unsigned long long *__restrict__ fullmin,
     const unsigned long long *tau, int KO, const int32_t *__restrict__ qprog,
     const unsigned long long *__restrict__ popcnt, uint64_t nrows, FvHit *__restrict__ out,
@@ -1218,20 +1312,15 @@ __device__ __forceinline__ void dense_top32_query(
     const uint64_t *src = dense + (uint64_t)q * dcap;
     __syncthreads();
     if (reset_cnt && tid == 0) dcnt[q] = 0;  // every thread has read it
-    uint64_t best[W];  // ascending across the lanes, half by half
-#pragma unroll
-    for (int h = 0; h < W; h++) best[h] = KEY_MAX;
-    // A long run is cut first: every lane's smallest key (two of them for
-    // W = 2) is a key of the run, so the KO-th smallest of a warp's lane
-    // minima bounds the KO-th key of the run, the smallest such bound leaves
+    uint64_t best[1] = {KEY_MAX};  // ascending across the lanes
+    // A long run is cut first: every lane's smallest key is a key of the run,
+    // so the KO-th smallest of a warp's lane minima bounds the KO-th key of the run, the smallest such bound leaves
     // a few times KO keys, and only those are sorted (folding in all of
     // 10,000 keys, 32 at a time, took 0.026 ms for 64 queries, most groups of
     // 32 holding a key better than the list's last).
     if (n > CUT_MIN) {
         constexpr int U = 4;
-        uint64_t mn[W];
-#pragma unroll
-        for (int h = 0; h < W; h++) mn[h] = KEY_MAX;
+        uint64_t mn = KEY_MAX;
         for (uint64_t b = tid; b < n; b += (uint64_t)blockDim.x * U) {
             uint64_t kk[U];
 #pragma unroll
@@ -1240,16 +1329,9 @@ __device__ __forceinline__ void dense_top32_query(
                 kk[u] = i < n ? src[i] : KEY_MAX;
             }
 #pragma unroll
-            for (int u = 0; u < U; u++) mn[u % W] = kk[u] < mn[u % W] ? kk[u] : mn[u % W];
+            for (int u = 0; u < U; u++) mn = kk[u] < mn ? kk[u] : mn;
         }
-        uint64_t top[W];
-        top[0] = warp_sort32(mn[0], lane, false);
-        if (W > 1) {
-            top[W - 1] = KEY_MAX;
-            warp_fold32<W>(top, warp_sort32(mn[W - 1], lane, true), lane);
-        }
-        const uint64_t lastw = W == 1 || KO <= 32 ? top[0] : top[W - 1];
-        const uint64_t bw = __shfl_sync(0xffffffffu, lastw, (KO - 1) & 31);
+        const uint64_t bw = __shfl_sync(0xffffffffu, warp_sort32(mn, lane, false), KO - 1);
         if (tid == 0) {
             s_cut = bound;
             s_ncut = 0;
@@ -1291,44 +1373,33 @@ __device__ __forceinline__ void dense_top32_query(
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            const uint64_t worst = __shfl_sync(0xffffffffu, best[W - 1], 31);
+            const uint64_t worst = __shfl_sync(0xffffffffu, best[0], 31);
             if (!__any_sync(0xffffffffu, k2[u] < worst)) continue;
-            warp_fold32<W>(best, warp_sort32(k2[u], lane, true), lane);
+            warp_fold32<1>(best, warp_sort32(k2[u], lane, true), lane);
         }
     }
     // the warps' lists fold pairwise, log2(NW) rounds (warp w takes in
     // warp w + step's list, read descending, while w is a multiple of 2 step)
-#pragma unroll
-    for (int h = 0; h < W; h++) lists[warp][h * 32 + lane] = best[h];
+    lists[warp][lane] = best[0];
     for (int step = 1; step < NW; step <<= 1) {
         __syncthreads();
         if ((warp & (2 * step - 1)) == 0 && warp + step < NW) {
-#pragma unroll
-            for (int h = 0; h < W; h++) {
-                const uint64_t d = lists[warp + step][h * 32 + 31 - lane];
-                const uint64_t worst = __shfl_sync(0xffffffffu, best[W - 1], 31);
-                if (__any_sync(0xffffffffu, d < worst)) warp_fold32<W>(best, d, lane);
-            }
-#pragma unroll
-            for (int h = 0; h < W; h++) lists[warp][h * 32 + lane] = best[h];
+            const uint64_t d = lists[warp + step][31 - lane];
+            const uint64_t worst = __shfl_sync(0xffffffffu, best[0], 31);
+            if (__any_sync(0xffffffffu, d < worst)) warp_fold32<1>(best, d, lane);
+            lists[warp][lane] = best[0];
         }
     }
     if (warp == 0) {
-        int c = 0;
-        uint64_t last = 0;
-#pragma unroll
-        for (int h = 0; h < W; h++) {
-            const bool have = h * 32 + lane < KO && best[h] != KEY_MAX;
-            c += __popc(__ballot_sync(0xffffffffu, have));
-            if (have) {
-                FvHit hit;
-                hit.node = (uint64_t)key_row(best[h]);
-                hit.dist = key_dist(best[h]);
-                out[(uint64_t)q * KO + h * 32 + lane] = hit;
-            }
-            const uint64_t l = __shfl_sync(0xffffffffu, best[h], (KO - 1) & 31);
-            if ((KO - 1) >> 5 == h) last = l;
+        const bool have = lane < KO && best[0] != KEY_MAX;
+        const int c = __popc(__ballot_sync(0xffffffffu, have));
+        if (have) {
+            FvHit hit;
+            hit.node = (uint64_t)key_row(best[0]);
+            hit.dist = key_dist(best[0]);
+            out[(uint64_t)q * KO + lane] = hit;
         }
+        const uint64_t last = __shfl_sync(0xffffffffu, best[0], KO - 1);
         if (lane == 0) {
             out_cnt[q] = (uint32_t)c;
             unsigned long long passing = (unsigned long long)passing_pre;
