@@ -504,7 +504,9 @@ extern "C" PvServe *pv_serve_create(FvGpuIndex *g, int max_batch, uint32_t max_k
     // groups would cap the 320 threads' registers below the kernel's
     // needs), as many stages as fit
     s->KPcap = TC_MAX_LIST;
-    const size_t cap = 227 * 1024 - 16 * 1024;  // static shared memory of the bitmap phase
+    // (beside 21 KB of static shared memory: the largest shape below, two
+    // K-blocks and three stages, leaves 0.7 KB)
+    const size_t cap = 227 * 1024 - 16 * 1024;
     s->EPI = 1;
     s->NS = 4;
     while (s->NS > 2 && tc_smem_bytes(kblocks, s->NS, s->KPcap, s->EPI) > cap) s->NS--;
