@@ -348,7 +348,6 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         if ((e = cudaMemcpyAsync(g->d_prows, post_rows, count * (size_t)ncols * 4,
                                  cudaMemcpyHostToDevice, g->stream)) != cudaSuccess)
             return bail("postings copy", e);
-        if ((e = pv::build_rank_cols(g)) != cudaSuccess) return bail("column positions", e);
         pv::build_sorted_cols(g, cols, post_rows);
     }
 
@@ -439,6 +438,8 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return bail("convert", e);
     }
+    // last: what it allocates is left out where there is no room for it
+    if ((e = pv::build_rank_cols(g)) != cudaSuccess) return bail("column positions", e);
     // the caller's arrays may go once this returns
     if ((e = cudaStreamSynchronize(g->stream)) != cudaSuccess) return bail("upload", e);
     return g;

@@ -178,7 +178,10 @@ def concat(preds: Sequence[Optional[Pred]], count: int,
     qd["need_eval"] = 1
     qd["total"] = count
     if entries is not None:
-        qd["entry"] = np.asarray(entries)[:nq]
+        e = entries if isinstance(entries, np.ndarray) else np.asarray(entries, qd["entry"].dtype)
+        if len(e) < nq:
+            raise IndexError(f"{len(e)} entry nodes for {nq} queries")
+        qd["entry"] = e[:nq]
     recs, children, invals = [], [], []
     if nq - sum(p is None for p in preds) <= 8:
         # a few filters: every query's slice in place (the gather below costs

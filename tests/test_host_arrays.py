@@ -29,6 +29,12 @@ def test_concat_places_every_querys_own_slice():
     assert list(bp.qd["entry"]) == list(range(7)) and (bp.qd["total"] == 77).all()
 
 
+@pytest.mark.parametrize("entries", [[3], [1, 2], np.array([4]), [-1, 0, 0]])
+def test_entries_that_are_refused(entries):
+    with pytest.raises((IndexError, OverflowError)):
+        pred.concat([None] * 3, 10, entries=entries)
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 4095, 4096, 4105])
 @pytest.mark.parametrize("odd", [None, 0.5, 257.0, -257.0, np.nan, np.inf, -np.inf, 1e-40])
 def test_integral_amax(n, odd):
