@@ -135,11 +135,123 @@ bitmap_range1_kernel(const double *__restrict__ cols, uint64_t nrows,
     if (threadIdx.x == 0 && s_cnt) atomicAdd(popcnt, (unsigned long long)s_cnt);
 }
 
+// Two to BM_FEW range-form programs (terms checked on the host): the same one
+// wave as bitmap_range1_kernel. The batch's terms are decoded once per block
+// and ordered by column, so a warp reads a column's values for its 4 words
+// once and tests every program's term on them; a lane keeps one bit per
+// program and row. Bound by latency: the constants' three dependent reads,
+// then one wait on HBM per column. Measured on one B200, six filters on two
+// columns of 1M rows: 0.0136 ms (three blocks an SM and 40 registers, which
+// leave the last tenth of the blocks a wave of their own, 0.0150), where the
+// general kernel, which walks its rows in turns of 148 x 2 blocks, took 0.021;
+// 64 real-valued queries 209 -> 200 us, 512 BF16 ones 390 -> 377.
+constexpr int BM_FEW = BM_PCH;
+constexpr int BM_FEW_TERMS = BM_FEW * PV_RANGE_MAX_TERMS;
+constexpr int BM_FEW_THREADS = 512;
+
+__global__ void __launch_bounds__(BM_FEW_THREADS, 4)
+bitmap_few_kernel(const double *__restrict__ cols, uint64_t nrows,
+                  const PredInsn *__restrict__ insns, const PredProg *__restrict__ progs, int P,
+                  const double *__restrict__ consts, int nconsts,
+                  uint32_t *__restrict__ bitmaps, uint64_t bm_words,
+                  unsigned long long *__restrict__ popcnt) {
+    struct Term {
+        double lo, hi;  // or lo's bits: the set
+        int col, prog;  // col | PV_TERM_MASK
+    };
+    __shared__ double s_const[BM_FEW_TERMS * 3];
+    __shared__ Term s_raw[BM_FEW_TERMS], s_term[BM_FEW_TERMS];
+    __shared__ int s_n[BM_FEW];
+    __shared__ unsigned int s_cnt[BM_FEW];
+    pdl_wait();
+    pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int i = tid; i < nconsts; i += BM_FEW_THREADS) s_const[i] = consts[i];
+    PredInsn r = {};
+    if (tid < P) r = insns[progs[tid].insn0];
+    if (tid < BM_FEW) s_cnt[tid] = 0;
+    __syncthreads();
+    if (tid < P) {
+        int ci = r.val0;
+        for (int k = 0; k < r.n; k++) {
+            Term t;
+            t.col = (int)s_const[ci];
+            t.prog = tid;
+            t.lo = s_const[ci + 1];
+            t.hi = t.col & PV_TERM_MASK ? 0.0 : s_const[ci + 2];
+            ci += t.col & PV_TERM_MASK ? 2 : 3;
+            s_raw[tid * PV_RANGE_MAX_TERMS + k] = t;
+        }
+        s_n[tid] = r.n;
+    }
+    __syncthreads();
+    int nt = 0;
+    for (int p = 0; p < P; p++) nt += s_n[p];
+    if (tid < P * PV_RANGE_MAX_TERMS && tid % PV_RANGE_MAX_TERMS < s_n[tid / PV_RANGE_MAX_TERMS]) {
+        const int mine = s_raw[tid].col & 0xFFFF;
+        int at = 0;
+        for (int p = 0; p < P; p++)
+            for (int k = 0; k < s_n[p]; k++) {
+                const int o = p * PV_RANGE_MAX_TERMS + k, c = s_raw[o].col & 0xFFFF;
+                at += c < mine || (c == mine && o < tid);
+            }
+        s_term[at] = s_raw[tid];
+    }
+    __syncthreads();
+    const uint64_t w0 = ((uint64_t)blockIdx.x * (BM_FEW_THREADS / 32) + (tid >> 5)) * 4;
+    unsigned pass[4];  // bit p: program p passes the row
+#pragma unroll
+    for (int j = 0; j < 4; j++) pass[j] = (w0 + j) * 32 + lane < nrows ? 0xFFFFFFFFu : 0u;
+    double v[4] = {};
+    int at = -1;
+    for (int i = 0; i < nt; i++) {
+        const int tc = s_term[i].col, col = tc & 0xFFFF;
+        if (col != at) {
+            const double *c = cols + (uint64_t)col * nrows + w0 * 32 + lane;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                v[j] = (w0 + j) * 32 + lane < nrows ? __ldg(c + j * 32) : 0.0;
+            at = col;
+        }
+        const unsigned bit = 1u << s_term[i].prog;
+        const double lo = s_term[i].lo;
+        if (tc & PV_TERM_MASK) {
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(lo);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const bool in = v[j] >= 0.0 && v[j] < 64.0;
+                const int b = in ? (int)v[j] : 64;
+                const bool ok = in && (double)b == v[j] && ((bits >> (b & 63)) & 1ull);
+                if (!ok) pass[j] &= ~bit;
+            }
+        } else {
+            const double hi = s_term[i].hi;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (!(v[j] >= lo && v[j] <= hi)) pass[j] &= ~bit;
+        }
+    }
+    for (int p = 0; p < P; p++) {
+        uint32_t mine = 0;
+        unsigned cnt = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t wd = __ballot_sync(0xffffffffu, (pass[j] >> p) & 1u);
+            if (lane == j) mine = wd;
+            cnt += __popc(wd);
+        }
+        if (lane < 4 && w0 + lane < bm_words) bitmaps[(uint64_t)p * bm_words + w0 + lane] = mine;
+        if (lane == 0 && cnt) atomicAdd(&s_cnt[p], cnt);
+    }
+    __syncthreads();
+    if (tid < P && s_cnt[tid]) atomicAdd(popcnt + tid, (unsigned long long)s_cnt[tid]);
+}
+
 cudaError_t launch_bitmaps(const double *cols, uint64_t nrows, const PredInsn *insns,
                            const PredProg *progs, const double *consts, int P,
                            uint32_t *bitmaps, uint64_t bm_words,
                            unsigned long long *popcnt, int sm_count, cudaStream_t st,
-                           int ninsns, int nconsts, int ncols, bool one_range) {
+                           int ninsns, int nconsts, int ncols, bool one_range, bool few_range) {
     if (P <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(popcnt, 0, sizeof(unsigned long long) * P, st);
     if (e != cudaSuccess) return e;
@@ -148,6 +260,12 @@ cudaError_t launch_bitmaps(const double *cols, uint64_t nrows, const PredInsn *i
         return launch_pdl(bitmap_range1_kernel, dim3((unsigned)(blocks ? blocks : 1)), dim3(256),
                           0, st, cols, nrows, insns, progs, consts, nconsts, bitmaps, bm_words,
                           popcnt);
+    }
+    if (few_range && P <= BM_FEW && nconsts <= BM_FEW_TERMS * 3) {
+        const uint64_t blocks = (bm_words + BM_FEW_THREADS / 8 - 1) / (BM_FEW_THREADS / 8);
+        return launch_pdl(bitmap_few_kernel, dim3((unsigned)(blocks ? blocks : 1)),
+                          dim3(BM_FEW_THREADS), 0, st, cols, nrows, insns, progs, P, consts,
+                          nconsts, bitmaps, bm_words, popcnt);
     }
     return launch_multi(cols, nrows, insns, progs, consts, P, ninsns, nconsts, nullptr, ncols,
                         bitmaps, bm_words, popcnt, sm_count, st);

@@ -57,12 +57,12 @@ int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &
     if (!pb.insns.empty())
         memcpy(h + db.off_insns, pb.insns.data(), pb.insns.size() * sizeof(PredInsn));
     if (!pb.consts.empty()) memcpy(h + db.off_consts, pb.consts.data(), pb.consts.size() * 8);
-    // one range-form program with well-formed terms: the lean bitmap kernel
-    db.one_range = false;
-    if (P == 1 && pb.progs[0].ninsn == 1 && pb.progs[0].insn0 >= 0 &&
-        pb.progs[0].insn0 < (int)pb.insns.size() &&
-        pb.insns[pb.progs[0].insn0].kind == PV_NODE_RANGE) {
-        const PredInsn &r = pb.insns[pb.progs[0].insn0];
+    // range-form programs with well-formed terms: the lean bitmap kernels
+    auto well_formed = [&](const PredProg &pg) {
+        if (pg.ninsn != 1 || pg.insn0 < 0 || pg.insn0 >= (int)pb.insns.size() ||
+            pb.insns[pg.insn0].kind != PV_NODE_RANGE)
+            return false;
+        const PredInsn &r = pb.insns[pg.insn0];
         bool ok = r.n >= 1 && r.n <= PV_RANGE_MAX_TERMS;
         int ci = r.val0;
         const int nc = (int)pb.consts.size();
@@ -74,10 +74,13 @@ int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &
             ok = (meta & 0xFFFF) < g->ncols && (mask || ci + 3 <= nc);
             ci += mask ? 2 : 3;
         }
-        db.one_range = ok;
-    }
-    // many range-form programs: the position form (up to eight take one turn
-    // of the general kernel, which has no tables to make first)
+        return ok;
+    };
+    db.one_range = P == 1 && well_formed(pb.progs[0]);
+    db.few_range = P > 1 && P < PV_RANK_MIN_PROGS &&
+                   std::all_of(pb.progs.begin(), pb.progs.end(), well_formed);
+    // many range-form programs: the position form (up to eight take
+    // bitmap_few_kernel, which has no tables to make first)
     db.rank_ok = P >= PV_RANK_MIN_PROGS && P <= PV_RANK_MAX_PROGS && rank_batch_ok(g, pb);
     if (db.rank_ok)
         PV_CUDA_OK(g->scan.rank_tab.ensure(rank_tab_bytes(P)), errbuf, errlen);
@@ -150,7 +153,7 @@ int brute_bitmaps(FvGpuIndex *g, const DevBatch &db, char *errbuf, size_t errlen
     g->launches++;
     PV_CUDA_OK(launch_bitmaps(g->d_cols, g->count, d_insns, d_progs, d_consts, P, bm, bm_words,
                               pop, g->sm_count, g->stream, db.ninsns, db.nconsts, g->ncols,
-                              db.one_range),
+                              db.one_range, db.few_range),
                errbuf, errlen);
     return 0;
 }
