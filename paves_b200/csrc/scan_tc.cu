@@ -267,9 +267,12 @@ int tc_superset(const FvGpuIndex *g, uint32_t topb, float q_amax) {
 // (TF32 keeps integers up to 2048 exactly, so the norm-form distances are
 // exact as in the BF16 case), else 4k (at least 16), each query's answer
 // then certified by the re-rank's error bound (RerankCert) and re-run on the
-// CUDA cores when the bound does not separate it. 0 = topb too large.
+// CUDA cores when the bound does not separate it. 0 = topb too large, or
+// rows (one infinite or NaN value is enough) whose norms leave no query
+// certifiable: such a table is scanned on the CUDA cores at once.
 int tf32_superset(const FvGpuIndex *g, uint32_t topb, float q_amax) {
     const bool exact = !g->force_wide_superset && pv_bf16_exact(g->dim, g->row_amax, q_amax);
+    if (!exact && !(g->norm32_max < 0x1p126f)) return 0;
     const int s = exact ? (int)topb : std::max(4 * (int)topb, 16);
     return s <= TC_MAX_SUPERSET ? s : 0;
 }

@@ -850,7 +850,8 @@ __device__ __forceinline__ void block_sort(uint64_t *keys, int n2) {
 // E = 2 (1 + 2^-6) (||x|| ||q - q'|| + ||x - t(x)|| ||q||) + dim 2^-20 ||x|| ||q||
 //     + c2 (xnmax + ||q||^2 + A): the first term's margin covers the f32
 // roundings of the norms themselves, the second is twice what the analysis
-// needs. Queries that fail are flagged in unc[] for an exact re-run.
+// needs. All of this holds while xnmax + ||q||^2 stays inside f32's range.
+// Queries that fail are flagged in unc[] for an exact re-run.
 struct RerankCert {
     const float *qnorm = nullptr;  // [nq] ||q||^2 (f32)
     const float *qres = nullptr;   // [nq] ||q - q'||^2 (f32)
@@ -998,16 +999,23 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
         const int pg = qprog[q];
         const unsigned long long passing = pg >= 0 ? popcnt[pg] : nrows;
         trunc[q] = passing > (unsigned long long)topb ? 1 : 0;
-        // a superset short of S holds every row that can pass: nothing to certify
-        if (cert.qnorm && ncand >= S && nout == (int)topb) {
-            const double A = (double)cand[(size_t)q * S + (S - 1)].dist;
-            const double Dk = (double)key_dist(keys[nout - 1]);
+        if (cert.qnorm) {
             const double qn = (double)cert.qnorm[q], xm = (double)cert.xnmax;
-            const double c2 = (double)(cert.dim + 8) * 0x1p-23;
-            const double qr = (double)cert.qres[q], xr = (double)cert.xrmax;
-            const double E = 2.0 * (1.0 + 0x1p-6) * (sqrt(xm * qr) + sqrt(xr * qn)) +
-                             cert.dim * 0x1p-20 * sqrt(qn * xm) + c2 * (xm + qn + A);
-            if (!((A - E) * (1.0 - c2) > Dk)) cert.unc[q] = 1;
+            // norms whose sum f32 cannot hold put rows at infinity or drop
+            // them; a superset short of S holds every row that passes, unless
+            // the scan lost some (their distances were NaN)
+            bool ok = xm + qn < 0x1p127 &&
+                      (unsigned long long)ncand >= min(passing, (unsigned long long)S);
+            if (ncand >= S && nout == (int)topb) {
+                const double A = (double)cand[(size_t)q * S + (S - 1)].dist;
+                const double Dk = (double)key_dist(keys[nout - 1]);
+                const double c2 = (double)(cert.dim + 8) * 0x1p-23;
+                const double qr = (double)cert.qres[q], xr = (double)cert.xrmax;
+                const double E = 2.0 * (1.0 + 0x1p-6) * (sqrt(xm * qr) + sqrt(xr * qn)) +
+                                 cert.dim * 0x1p-20 * sqrt(qn * xm) + c2 * (xm + qn + A);
+                ok = ok && (A - E) * (1.0 - c2) > Dk;
+            }
+            if (!ok) cert.unc[q] = 1;
         }
     }
     __syncthreads();
