@@ -850,7 +850,9 @@ __device__ __forceinline__ void block_sort(uint64_t *keys, int n2) {
 // E = 2 (1 + 2^-6) (||x|| ||q - q'|| + ||x - t(x)|| ||q||) + dim 2^-20 ||x|| ||q||
 //     + c2 (xnmax + ||q||^2 + A): the first term's margin covers the f32
 // roundings of the norms themselves, the second is twice what the analysis
-// needs. All of this holds while xnmax + ||q||^2 stays inside f32's range.
+// needs. All of this holds while xnmax + ||q||^2 stays inside f32's range;
+// at its lower end, what the squares and products of tiny values lose is
+// added (without it, rows near 1e-20 that TF32 cannot tell apart passed).
 // Queries that fail are flagged in unc[] for an exact re-run.
 struct RerankCert {
     const float *qnorm = nullptr;  // [nq] ||q||^2 (f32)
@@ -1010,9 +1012,14 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
                 const double A = (double)cand[(size_t)q * S + (S - 1)].dist;
                 const double Dk = (double)key_dist(keys[nout - 1]);
                 const double c2 = (double)(cert.dim + 8) * 0x1p-23;
-                const double qr = (double)cert.qres[q], xr = (double)cert.xrmax;
-                const double E = 2.0 * (1.0 + 0x1p-6) * (sqrt(xm * qr) + sqrt(xr * qn)) +
-                                 cert.dim * 0x1p-20 * sqrt(qn * xm) + c2 * (xm + qn + A);
+                // squares below f32's range: at most half its smallest step a
+                // dim in each of the four sums, and products that the MMA may
+                // flush to zero
+                const double lost = cert.dim * 0x1p-149, xu = xm + lost, qu = qn + lost;
+                const double qr = (double)cert.qres[q] + lost, xr = (double)cert.xrmax + lost;
+                const double E = 2.0 * (1.0 + 0x1p-6) * (sqrt(xu * qr) + sqrt(xr * qu)) +
+                                 cert.dim * 0x1p-20 * sqrt(qu * xu) + c2 * (xu + qu + A) +
+                                 cert.dim * 0x1p-124;
                 ok = ok && (A - E) * (1.0 - c2) > Dk;
             }
             if (!ok) cert.unc[q] = 1;
