@@ -129,10 +129,15 @@ rerank_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict_
               FvHit *__restrict__ out, uint32_t *__restrict__ out_cnt,
               uint8_t *__restrict__ trunc, const RerankCert cert) {
     __shared__ uint64_t keys[TC_MAX_SUPERSET];
+    __shared__ int again;
+    if (threadIdx.x == 0) again = 0;
     pdl_wait();
     pdl_trigger();
     rerank_query<256, ORDER>(blockIdx.x, keys, vecs, dpad, queries, cand, cand_cnt, S, topb, qprog, popcnt,
-                      nrows, out, out_cnt, trunc, cert);
+                      nrows, out, out_cnt, trunc, cert, &again);
+    if (ORDER == RR_LANES8 && again)
+        rerank_query<256, RR_WARP>(blockIdx.x, keys, vecs, dpad, queries, cand, cand_cnt, S, topb,
+                                   qprog, popcnt, nrows, out, out_cnt, trunc, cert);
 }
 
 // ---------------------------------------------------------------- merge

@@ -864,7 +864,10 @@ struct RerankCert {
 };
 
 // Orders of the exact distance's sum. Rows up to 128 dims: 8 lanes a
-// candidate (RR_LANES8). Wider rows reach the re-rank only on batches that
+// candidate (RR_LANES8); queries that only this bound separates, and not the
+// one that any values allow (1.25 * 2^-8 ||x|| ||q||), are summed once more
+// in the order of the CUDA-core scan that answered them under that one
+// (RR_WARP, whose shorter chains round less). Wider rows reach the re-rank only on batches that
 // the CUDA-core scans answered before, and keep those kernels' sums bit for
 // bit, so near ties order as they do there: the warp's of scan_f32.cu and of
 // a selective filter's listed rows (RR_WARP), or the thread's of scan_f32t.cu,
@@ -872,7 +875,8 @@ struct RerankCert {
 constexpr int RR_LANES8 = 0, RR_WARP = 1, RR_THREAD = 2;
 
 // One query's re-rank by the block's NT threads (8 lanes per candidate,
-// NT / 8 in flight); keys: TC_MAX_SUPERSET slots of shared memory. Ends
+// NT / 8 in flight); keys: TC_MAX_SUPERSET slots of shared memory; *again
+// (shared memory): whether the answer stands on the closer bound alone. Ends
 // with the block synchronized.
 template <int NT, int ORDER = RR_LANES8>
 __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float *__restrict__ vecs,
@@ -884,7 +888,8 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
                                              uint64_t nrows, FvHit *__restrict__ out,
                                              uint32_t *__restrict__ out_cnt,
                                              uint8_t *__restrict__ trunc,
-                                             const RerankCert cert = RerankCert()) {
+                                             const RerankCert cert = RerankCert(),
+                                             int *again = nullptr) {
     const int tid = threadIdx.x;
     const int grp = tid >> 3, sub = tid & 7;
     const int ncand = (int)cand_cnt[q];
@@ -1021,6 +1026,8 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
                                  cert.dim * 0x1p-20 * sqrt(qu * xu) + c2 * (xu + qu + A) +
                                  cert.dim * 0x1p-124;
                 ok = ok && (A - E) * (1.0 - c2) > Dk;
+                const double E1 = 1.25 * 0x1p-8 * sqrt(qn * xm) * (1.0 + c2) + c2 * (xm + qn + A);
+                if (again) *again = ok && !((A - E1) * (1.0 - c2) > Dk);
             }
             if (!ok) cert.unc[q] = 1;
         }
