@@ -231,6 +231,7 @@ struct TcRowSet {
     uint64_t nrows;
     const uint32_t *rowids;
     const unsigned long long *nrows_dev;  // rows that exist (device), <= nrows
+    bool listed;  // few enough for the sparse route (else the index's scan gives way to it)
 };
 int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
                    const int32_t *d_qprog,

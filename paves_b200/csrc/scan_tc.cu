@@ -707,7 +707,8 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         auto *rerank = rerank_kernel<RR_LANES8>;
         if (tf32 && g->dpad > 128) {
             ScanPlan pl;
-            rerank = !rs && plan_scan_f32t(g->count, g->dpad, nq, (int)topb, g->sm_count, pl)
+            rerank = !(rs && rs->listed) &&
+                             plan_scan_f32t(g->count, g->dpad, nq, (int)topb, g->sm_count, pl)
                          ? rerank_kernel<RR_THREAD> : rerank_kernel<RR_WARP>;
         }
         PV_CUDA_OK(launch_pdl(rerank, dim3(nq), dim3(256), 0, g->stream, g->d_vecs,

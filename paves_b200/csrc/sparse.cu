@@ -550,7 +550,7 @@ int sparse_tc_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, uint64_t bound,
         cap, rows, norms, scales, valid, vwords);
     PV_CUDA_OK(cudaGetLastError(), errbuf, errlen);
     g->launches += 2;  // compaction, gather
-    const TcRowSet rs{rows, norms, scales, cap_pad, ids, d_count};
+    const TcRowSet rs{rows, norms, scales, cap_pad, ids, d_count, db.sparse_bound > 0};
     const double expect = std::min(1.0, db.pass * (double)g->count / (double)cap_pad);
     return launch_scan_tc(g, nq, db.q_amax, d_q, d_qprog, valid, vwords,
                           s.popcnt.as<unsigned long long>(), topb, d_out, d_cnt, d_trunc, ev,

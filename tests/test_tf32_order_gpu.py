@@ -36,3 +36,18 @@ def test_rows_that_only_the_closer_bound_separates(dim, nq, k):
     got, want, (tc, _) = both_routes(x, None, q, [None] * nq, k)
     assert tc == 1
     same(got, want)
+
+
+@pytest.mark.parametrize("dim,nq,k,n", [(200, 32, 10, 400_000), (256, 24, 64, 300_000),
+                                        (160, 100, 1, 500_000), (200, 23, 10, 600_000),
+                                        (300, 130, 10, 200_000), (200, 64, 80, 300_000)])
+def test_gathered_wide_rows(dim, nq, k, n):
+    """A shared filter of 10 % is scanned as a gathered set; the sums are
+    those of the scan of the index."""
+    rng = np.random.default_rng(dim + nq)
+    x = rng.standard_normal((n, dim), dtype=np.float32)
+    q = rng.standard_normal((nq, dim), dtype=np.float32)
+    cols = rng.uniform(0, 1, (1, n))
+    got, want, took = both_routes(x, cols, q, [Cmp(0, "<", 0.1)] * nq, k)
+    assert took == (1, 1)
+    same(got, want)
