@@ -179,6 +179,7 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     // uploads whose rows are too wide for their own scan
     const bool exact_mode = mode == PV_MODE_EXACT || (mode == 1 && !tc_supported(g));
     const bool exact_tc_can = exact_mode && nq >= PV_EXACT_TC_MIN_NQ &&
+                              (db.redo || g->dpad <= 128) &&
                               tf32_supported(g) && tf32_superset(g, topb, db.q_amax) > 0;
     bool sparse_tc = sparse_route && (low_tc_can || exact_tc_can) &&
                      db.sparse_bound >= PV_SPARSE_TC_MIN_ROWS;
@@ -261,7 +262,7 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
         if (launch_scan_tc(g, nq, db.q_amax, d_q, d_qprog, s.bitmaps.as<uint32_t>(), bm_words,
                            s.popcnt.as<unsigned long long>(), topb, d_out, d_cnt, d_trunc, ev,
                            errbuf, errlen, db.counts_on_device ? &lz : nullptr, false, nullptr,
-                           bm_launched, bm_done, db.pass))
+                           bm_launched, bm_done, db.pass, db.redo))
             return -1;
         if (ev) cudaEventRecord(ev[4], g->stream);
         return 0;
@@ -272,7 +273,7 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
         if (launch_scan_tc(g, nq, db.q_amax, d_q, d_qprog, s.bitmaps.as<uint32_t>(), bm_words,
                            s.popcnt.as<unsigned long long>(), topb, d_out, d_cnt, d_trunc, ev,
                            errbuf, errlen, db.counts_on_device ? &lz : nullptr, true, nullptr,
-                           bm_launched, bm_done, db.pass))
+                           bm_launched, bm_done, db.pass, db.redo))
             return -1;
         g->last_exact_tc = 1;
         if (ev) cudaEventRecord(ev[4], g->stream);

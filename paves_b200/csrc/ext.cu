@@ -58,6 +58,7 @@ extern "C" PvBatch *pv_batch_create(FvGpuIndex *g, int nq, const float *queries,
     b->mode = mode;
     b->db.stage_h = &b->stage_h;
     b->db.stage_d = &b->stage_d;
+    b->db.redo = false;  // pv_batch_fetch reports uncertified queries
     auto fail = [&](const char *what, cudaError_t e) -> PvBatch * {
         if (errbuf && errlen && what)
             snprintf(errbuf, errlen, "gpu: %s: %s", what, cudaGetErrorString(e));

@@ -131,6 +131,9 @@ struct DevBatch {
     uint64_t bound = 0;       // one_prog: at most this many rows pass (0: not known)
     double pass = 1.0;        // share of the rows its filter passes, at most or estimated
     bool rows_fused = false;  // scan_rows.cu tests the one filter itself
+    // the caller re-runs queries that the scan could not certify (prepared
+    // batches only report them, and take no route that flags more)
+    bool redo = true;
 };
 
 int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &pb,
@@ -240,11 +243,12 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
                    uint32_t *d_cnt, uint8_t *d_trunc, cudaEvent_t *ev, char *errbuf,
                    size_t errlen, const TcLazy *lz = nullptr, bool tf32 = false,
                    const TcRowSet *rs = nullptr, bool behind_bitmaps = false,
-                   cudaEvent_t prep_done = nullptr, double pass = 1.0);
+                   cudaEvent_t prep_done = nullptr, double pass = 1.0, bool redo = true);
 // behind_bitmaps: the last launch on the stream is this batch's bitmap
 // kernel (query prep then runs beside it); prep_done: recorded behind
 // query prep; pass: the share of the rows that the batch's filters let
-// through, as far as it is known
+// through, as far as it is known; redo: flagged queries are re-run by the
+// caller (else whole lists and certain bounds only)
 // Reads and clears the watchdog word of the last tensor-core scan after the
 // stream was synchronized; -1 + errbuf if a bounded wait expired.
 int check_tc_watchdog(FvGpuIndex *g, char *errbuf, size_t errlen);

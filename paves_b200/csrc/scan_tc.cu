@@ -336,7 +336,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
                    const unsigned long long *popcnt, uint32_t topb, FvHit *d_out,
                    uint32_t *d_cnt, uint8_t *d_trunc, cudaEvent_t *ev, char *errbuf,
                    size_t errlen, const TcLazy *lz, bool tf32, const TcRowSet *rs,
-                   bool behind_bitmaps, cudaEvent_t prep_done, double pass) {
+                   bool behind_bitmaps, cudaEvent_t prep_done, double pass, bool redo) {
     const bool fp8 = !tf32 && g->precision == FV_GPU_PREC_FP8;
     const int kind = tf32 ? TCK_TF32 : fp8 ? TCK_FP8 : TCK_BF16;
     const int esz = tck_esz(kind);
@@ -397,9 +397,11 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         }
     };
     // (three groups' lists hold every nearest row of the query that a list
-    // meets: where rows are stored cluster by cluster, only whole lists do)
+    // meets: where rows are stored cluster by cluster, only whole lists do;
+    // and a run that spills may be full, which flags the query)
     const bool whole3 = S <= tc_list_cap(3, kblocks);
-    shape(kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 && (g->rows_mixed || whole3) ? 3 : 2);
+    const bool three = whole3 || (g->rows_mixed && redo);
+    shape(kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 && three ? 3 : 2);
     bool tuned = false;
     if (g->tune_epi || g->tune_ns) {  // a tuned shape, if it fits
         const int e = g->tune_epi ? g->tune_epi : EPI, n = g->tune_ns ? g->tune_ns : NS;
@@ -440,7 +442,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const double fill = !rs || pass > 0.9 ? 1.0 : std::max(pass, 1.0 / 64);
     const uint64_t region = rs ? tpc : ntiles_all / grow;
     const double best = sqrt((double)S * tpc * fill / grow);
-    const bool may_est = certify && S > TC_MAX_LIST && g->rows_mixed;
+    const bool may_est = certify && S > TC_MAX_LIST && g->rows_mixed && redo;
     const uint64_t least = may_est ? 1 : ((uint64_t)S + grow - 1) / grow;
     const double want_m = std::min<double>(may_est ? 8 : 24, std::max<double>(least, floor(best)));
     uint64_t m = (uint64_t)std::min<double>((double)region, ceil(want_m / fill));

@@ -554,7 +554,7 @@ int sparse_tc_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, uint64_t bound,
     const double expect = std::min(1.0, db.pass * (double)g->count / (double)cap_pad);
     return launch_scan_tc(g, nq, db.q_amax, d_q, d_qprog, valid, vwords,
                           s.popcnt.as<unsigned long long>(), topb, d_out, d_cnt, d_trunc, ev,
-                          errbuf, errlen, nullptr, tf32, &rs, false, nullptr, expect);
+                          errbuf, errlen, nullptr, tf32, &rs, false, nullptr, expect, db.redo);
 }
 
 // The sparse route of brute_launch: every query uses program 0, whose
