@@ -511,6 +511,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
             for (int c = 0; c < nch; c++) {
                 const uint32_t word = c == 0 ? bw[0] : c == 1 ? bw[1] : c == 2 ? bw[2] : bw[3];
                 uint32_t r[32];
+                __syncwarp();  // TMEM is read by the whole warp
                 tmem_ld_32x32b_x32(tbase + c * 32, r);
                 tmem_ld_wait(r);
                 if (WARM && a.seed_group > 0 && !lazy) {
@@ -616,6 +617,7 @@ __device__ __forceinline__ bool tc_pass(const CUtensorMap *tmXp, const CUtensorM
                     const int i = __ffs(rows) - 1;
                     rows &= rows - 1;
                     uint32_t v;
+                    __syncwarp();  // the lanes part below, admitting or not
                     tmem_ld_32x32b_x1(tbase + c * 32 + i, v);
                     tmem_ld_wait(v);
                     if (!((cmask >> i) & 1u)) continue;
