@@ -440,6 +440,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // are a prefix, so the sample's are dealt round robin (every CTA has some
     // of them) and as many more are drawn as `pass` leaves empty.
     const double fill = !rs || pass > 0.9 ? 1.0 : std::max(pass, 1.0 / 64);
+    const bool full = !rs || pass > 0.99;  // (what fills its last tile may be missing)
     const uint64_t region = rs ? tpc : ntiles_all / grow;
     const double best = sqrt((double)S * tpc * fill / grow);
     const bool may_est = certify && S > TC_MAX_LIST && g->rows_mixed && redo;
@@ -458,7 +459,16 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // queries, 500,000 rows, S 40: 0.180 against 0.170 ms).
     int rank_est = S;
     auto enough = [&]() {  // chunk minima for the bound's rank, twice over
-        const double share = std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan);
+        // A compacted set with room to spare: the strides reach past the
+        // prefix of tiles that exist, so the sample holds every step-th of
+        // them and one more, not m of the room (which gave 256 queries of 1M
+        // FP8 rows, k 75, a bound below their superset when half of the room
+        // was used; all were run twice). Right down to half of the expected
+        // tiles.
+        const double share =
+            full ? std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan)
+                 : std::min(1.0, 1.0 / (double)std::max<uint64_t>(1, region / m) +
+                                     2.0 / (fill * (double)region));
         rank_est = may_est ? (int)ceil(S * share + 6.0 * sqrt(S * share) + 8.0) : S;
         return (uint64_t)(m * fill * grow * (TC_BN / 32)) >= 2 * (uint64_t)std::min(S, rank_est);
     };
