@@ -113,6 +113,13 @@ int pv_hnsw_export(const PvHnsw *h, uint32_t *l0, uint8_t *levels, uint64_t *upp
  * bad parameters or a device error. */
 PvHnsw *pv_hnsw_build_gpu(const float *vectors, uint64_t count, int dim, int M, int candidates,
                           int device, int precision, char *errbuf, size_t errlen);
+/* The same with the limit (ns, at most 10 s; 0 = the default) of one
+ * tensor-core scan's waits set: scan number wait_batch of level 0 (from 0, in
+ * batches of up to 2048 rows; -1: none). A scan whose wait runs out fails the
+ * build, whichever it is. */
+PvHnsw *pv_hnsw_build_gpu_wait(const float *vectors, uint64_t count, int dim, int M,
+                               int candidates, int device, int precision, uint64_t wait_ns,
+                               int wait_batch, char *errbuf, size_t errlen);
 /* Level-0 entry point per query by greedy descent through the upper levels
  * (engine_api.h:199 fv_index_graph_entry), parallel over queries. */
 int pv_hnsw_entries(const float *vectors, int dim, const uint64_t *upper_offs,

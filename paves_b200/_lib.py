@@ -207,6 +207,9 @@ _EXT_SIGS["pv_exact_tc"] = (C.c_int, [P, C.c_int])
 _EXT_SIGS["pv_last_exact_tc"] = (C.c_int, [P])
 _EXT_SIGS["pv_hnsw_build_gpu"] = (P, [P, C.c_uint64, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
                                         C.c_char_p, C.c_size_t])
+_EXT_SIGS["pv_hnsw_build_gpu_wait"] = (P, [P, C.c_uint64, C.c_int, C.c_int, C.c_int, C.c_int,
+                                             C.c_int, C.c_uint64, C.c_int, C.c_char_p,
+                                             C.c_size_t])
 PV_SERVE_MAX_K = 256
 _EXT_SIGS.update({
     "pv_serve_create": (P, [P, C.c_int, C.c_uint32, C.c_uint32, C.c_char_p, C.c_size_t]),

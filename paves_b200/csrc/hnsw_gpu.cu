@@ -324,11 +324,13 @@ void launch_final(uint64_t *fwd, uint32_t *fwd_cnt, const uint64_t *rev, const u
 // Exact nearest neighbours of rows [r0, r0 + nq) of g among all rows of g:
 // the tensor-core scan when its BF16 distances are certified exact for
 // these rows, else the exact FP32 scan (queries read in place from g's f32
-// rows). out [nq][topb] ascending, cnt [nq]; unc [nq]: nonzero where short
-// lists may have dropped a neighbour (the batch is then run again, `exact`).
+// rows). out [nq][topb] ascending, cnt [nq]; tail (zeroed by the caller): the
+// scan's watchdog word and flags as tc_tail_bytes lays them out, a query's
+// flag nonzero where short lists may have dropped a neighbour (the batch is
+// then run again, `exact`).
 int knn_batch(FvGpuIndex *g, uint64_t r0, int nq, uint32_t topb, const int32_t *d_qprog,
               const unsigned long long *d_popcnt, FvHit *d_out, uint32_t *d_cnt, uint8_t *d_tr,
-              uint8_t *d_unc, bool exact, char *errbuf, size_t errlen) {
+              uint8_t *d_tail, bool exact, char *errbuf, size_t errlen) {
     const float *d_q = g->d_vecs + r0 * (uint64_t)g->dpad;
     const uint64_t bm_words = (g->count + 31) / 32;
     g->tc_unc = nullptr;
@@ -337,10 +339,13 @@ int knn_batch(FvGpuIndex *g, uint64_t r0, int nq, uint32_t topb, const int32_t *
         if (launch_scan_tc(g, nq, g->row_amax, d_q, d_qprog, nullptr, bm_words, d_popcnt, topb,
                            d_out, d_cnt, d_tr, nullptr, errbuf, errlen))
             return -1;
-        if (g->tc_unc)
-            PV_CUDA_OK(cudaMemcpyAsync(d_unc, g->tc_unc, (size_t)nq, cudaMemcpyDeviceToDevice,
-                                       g->stream),
-                       errbuf, errlen);
+        // (each batch's own: the next one's query prep clears the word, and
+        // may have it elsewhere)
+        PV_CUDA_OK(cudaMemcpyAsync(d_tail, g->tc_err,
+                                   g->tc_unc ? tc_tail_bytes(nq) : sizeof(int),
+                                   cudaMemcpyDeviceToDevice, g->stream),
+                   errbuf, errlen);
+        g->tc_err = nullptr;
         g->tc_unc = nullptr;
         return 0;
     }
@@ -382,6 +387,15 @@ int knn_batch(FvGpuIndex *g, uint64_t r0, int nq, uint32_t topb, const int32_t *
 }
 
 constexpr int HG_BATCH = 2048;  // scan batch (queries per call)
+constexpr size_t HG_TAIL = TC_TAIL_UNC + HG_BATCH;
+// scan batches of an insertion step at most (the first 64 rows, then as many
+// as are in)
+uint64_t hg_step_batches(uint64_t n) { return 1 + n / 2 / HG_BATCH; }
+// A limit for the waits of one scan of level 0 (its number), for tests.
+struct HgWait {
+    uint64_t ns = 0;
+    int batch = -1;
+};
 
 // Workspace of the levels, sized for the largest (level 0 has the most rows
 // and the longest lists, an upper level may have the longest answers), and
@@ -389,7 +403,7 @@ constexpr int HG_BATCH = 2048;  // scan batch (queries per call)
 // 3 of a build's 30 ms and at times ten times that).
 struct HgWork {
     void *base = nullptr;
-    DevArr qprog, popcnt, out, cnt, tr, unc, lst, lcnt, in_cnt, in_off, cursor, rev, lists;
+    DevArr qprog, popcnt, out, cnt, tr, tails, lst, lcnt, in_cnt, in_off, cursor, rev, lists;
     DevArr ids, xs, los, norms;  // of n1 rows
     ~HgWork() {
         if (base) cudaFree(base);
@@ -403,7 +417,7 @@ struct HgWork {
                      {&out, (size_t)HG_BATCH * topb * sizeof(FvHit)},
                      {&cnt, (size_t)HG_BATCH * 4},
                      {&tr, (size_t)HG_BATCH},
-                     {&unc, (size_t)n},
+                     {&tails, (size_t)hg_step_batches(n) * HG_TAIL},
                      {&lst, (size_t)n * R * 8},
                      {&lcnt, (size_t)n * 4},
                      {&in_cnt, (size_t)n * 4},
@@ -431,7 +445,8 @@ struct HgWork {
 
 // One level over the rows of g by batched insertion: w.lists [count][R + 1]
 // of local ids.
-int build_level(FvGpuIndex *g, HgWork &w, int R, int C, char *errbuf, size_t errlen) {
+int build_level(FvGpuIndex *g, HgWork &w, int R, int C, const HgWait &wait, char *errbuf,
+                size_t errlen) {
     const uint64_t n = g->count;
     const int dpad = g->dpad;
     const int NVn = (dpad + 127) / 128;
@@ -453,24 +468,29 @@ int build_level(FvGpuIndex *g, HgWork &w, int R, int C, char *errbuf, size_t err
         g->tmap_x_ok = true;
     }
     DevArr &qprog = w.qprog, &popcnt = w.popcnt, &out = w.out, &cnt = w.cnt, &tr = w.tr,
-           &unc = w.unc, &lst = w.lst, &lcnt = w.lcnt, &in_cnt = w.in_cnt, &in_off = w.in_off,
+           &tails = w.tails, &lst = w.lst, &lcnt = w.lcnt, &in_cnt = w.in_cnt, &in_off = w.in_off,
            &cursor = w.cursor, &rev = w.rev;
     HG_OK(cudaMemsetAsync(qprog.p, 0xFF, (size_t)B * 4, st));  // no filter
     HG_OK(cudaMemsetAsync(lcnt.p, 0, (size_t)n * 4, st));
-    std::vector<uint8_t> h_unc;
-    int rc = 0;
+    std::vector<uint8_t> h_tails;
+    int rc = 0, nbatch = 0;
     for (uint64_t lo = 0; lo < n && rc == 0;) {
         const uint64_t hi = lo == 0 ? std::min(n, first) : std::min(n, 2 * lo);
         // 1-2: candidates among the inserted prefix [0, hi), forward selection
         g->count = hi;
         const int topb = (int)std::min<uint64_t>((uint64_t)C + 1, hi);
-        HG_OK(cudaMemsetAsync(unc.p, 0, (size_t)(hi - lo), st));
+        const size_t steps = (hi - lo + B - 1) / B;
+        HG_OK(cudaMemsetAsync(tails.p, 0, steps * HG_TAIL, st));
         auto batch = [&](uint64_t r0, bool exact) {
             const int nq = (int)std::min<uint64_t>(B, hi - r0);
-            if (knn_batch(g, r0, nq, (uint32_t)topb, qprog.as<int32_t>(),
-                          popcnt.as<unsigned long long>(), out.as<FvHit>(), cnt.as<uint32_t>(),
-                          tr.as<uint8_t>(), unc.as<uint8_t>() + (r0 - lo), exact, errbuf, errlen))
-                return -1;
+            const uint64_t limit = g->tc_timeout_ns;
+            if (nbatch++ == wait.batch) g->tc_timeout_ns = wait.ns;
+            const int bad = knn_batch(
+                g, r0, nq, (uint32_t)topb, qprog.as<int32_t>(), popcnt.as<unsigned long long>(),
+                out.as<FvHit>(), cnt.as<uint32_t>(), tr.as<uint8_t>(),
+                tails.as<uint8_t>() + (r0 - lo) / B * HG_TAIL, exact, errbuf, errlen);
+            g->tc_timeout_ns = limit;
+            if (bad) return -1;
             if (NVn <= 1)
                 launch_forward<1>(out.as<FvHit>(), cnt.as<uint32_t>(), topb, r0, nq, R, g->d_vecs,
                                   dpad, lst.as<uint64_t>(), lcnt.as<uint32_t>(), st);
@@ -483,18 +503,24 @@ int build_level(FvGpuIndex *g, HgWork &w, int R, int C, char *errbuf, size_t err
             return cudaGetLastError() == cudaSuccess ? 0 : -1;
         };
         for (uint64_t r0 = lo; r0 < hi && rc == 0; r0 += B) rc = batch(r0, false);
-        if (!rc) rc = check_tc_watchdog(g, errbuf, errlen);
         if (!rc) {
-            h_unc.resize(hi - lo);
-            if (cudaMemcpyAsync(h_unc.data(), unc.p, (size_t)(hi - lo), cudaMemcpyDeviceToHost, st) !=
-                    cudaSuccess ||
+            h_tails.resize(steps * HG_TAIL);
+            if (cudaMemcpyAsync(h_tails.data(), tails.p, h_tails.size(), cudaMemcpyDeviceToHost,
+                                st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess)
                 rc = -1;
         }
+        for (size_t i = 0; i < steps && rc == 0; i++) {
+            int e;
+            memcpy(&e, &h_tails[i * HG_TAIL], sizeof(e));
+            if (e) {
+                snprintf(errbuf, errlen, "hnsw gpu: tensor-core scan wait expired (role %d)", e);
+                rc = -1;
+            }
+        }
         for (uint64_t r0 = lo; r0 < hi && rc == 0; r0 += B) {
-            const uint64_t r1 = std::min<uint64_t>(r0 + B, hi);
-            if (std::any_of(h_unc.begin() + (r0 - lo), h_unc.begin() + (r1 - lo),
-                            [](uint8_t u) { return u != 0; }))
+            const auto f = h_tails.begin() + (r0 - lo) / B * HG_TAIL + TC_TAIL_UNC;
+            if (std::any_of(f, f + std::min<uint64_t>(B, hi - r0), [](uint8_t u) { return u != 0; }))
                 rc = batch(r0, true);
         }
         g->count = n;
@@ -547,8 +573,8 @@ int build_level(FvGpuIndex *g, HgWork &w, int R, int C, char *errbuf, size_t err
 // 2M; levels 1..top the rows of each level, R = M, gathered on the device
 // into one set of buffers that stands in for the table's (an upload of its
 // own per level took 8 of a build's 50 ms, 60,000 rows).
-int build_levels(PvHnsw *h, FvGpuIndex *g, int M, int candidates, int top, char *errbuf,
-                 size_t errlen) {
+int build_levels(PvHnsw *h, FvGpuIndex *g, int M, int candidates, int top, const HgWait &wait,
+                 char *errbuf, size_t errlen) {
     std::lock_guard<std::mutex> lk(g->mu);
     const uint64_t count = g->count;
     const uint8_t *lev = hnsw_levels(h);
@@ -581,7 +607,7 @@ int build_levels(PvHnsw *h, FvGpuIndex *g, int M, int candidates, int top, char 
         HG_OK(s.cand.ensure((nq + TC_BM) * ((size_t)g->kpad * 2 + 16) +
                             nq * (topb * sizeof(FvHit) + 8) + 4096));
     }
-    if (build_level(g, w, 2 * M, candidates, errbuf, errlen)) return -1;
+    if (build_level(g, w, 2 * M, candidates, wait, errbuf, errlen)) return -1;
     HG_OK(cudaMemcpy(hnsw_l0(h), w.lists.p, (size_t)count * (2 * M + 1) * 4,
                      cudaMemcpyDeviceToHost));
     if (ids.size() < 2) return 0;  // a single node has no neighbours
@@ -617,7 +643,7 @@ int build_levels(PvHnsw *h, FvGpuIndex *g, int M, int candidates, int top, char 
         }
         g->count = n;
         g->tmap_x_ok = false;
-        if (!rc) rc = build_level(g, w, M, upper(n), errbuf, errlen);
+        if (!rc) rc = build_level(g, w, M, upper(n), HgWait(), errbuf, errlen);
         g->d_vecs = vecs;
         g->d_vlow = vlow;
         g->d_norm = norm;
@@ -648,8 +674,16 @@ using namespace pv;
 extern "C" PvHnsw *pv_hnsw_build_gpu(const float *vectors, uint64_t count, int dim, int M,
                                      int candidates, int device, int precision, char *errbuf,
                                      size_t errlen) {
+    return pv_hnsw_build_gpu_wait(vectors, count, dim, M, candidates, device, precision, 0, -1,
+                                  errbuf, errlen);
+}
+
+extern "C" PvHnsw *pv_hnsw_build_gpu_wait(const float *vectors, uint64_t count, int dim, int M,
+                                          int candidates, int device, int precision,
+                                          uint64_t wait_ns, int wait_batch, char *errbuf,
+                                          size_t errlen) {
     if (!vectors || count == 0 || dim <= 0 || dim > 512 || M < 2 || M > HG_RMAX / 2 ||
-        candidates < 2 * M || candidates > 1023 ||
+        candidates < 2 * M || candidates > 1023 || wait_ns > 10000000000ull ||
         (precision != FV_GPU_PREC_FP32 && precision != FV_GPU_PREC_BF16)) {
         if (errbuf && errlen) snprintf(errbuf, errlen, "hnsw gpu: bad build parameters");
         return nullptr;
@@ -674,7 +708,7 @@ extern "C" PvHnsw *pv_hnsw_build_gpu(const float *vectors, uint64_t count, int d
     FvGpuIndex *g = fv_gpu_index_upload(vectors, nullptr, nullptr, nullptr, 0, count, dim, 0,
                                         device, precision, errbuf, errlen);
     if (!g) return fail();
-    const int rc = build_levels(h, g, M, candidates, top, errbuf, errlen);
+    const int rc = build_levels(h, g, M, candidates, top, HgWait{wait_ns, wait_batch}, errbuf, errlen);
     fv_gpu_index_free(g);
     if (rc) {
         if (errbuf && errlen && !errbuf[0]) snprintf(errbuf, errlen, "hnsw gpu: build failed");
