@@ -35,6 +35,13 @@ int pv_pred_check(int nq, const FvGpuQueryDesc *qd, const FvGpuPredNode *nodes, 
  * most 256 (rows whose BF16 distances can be certified exact), else -1. */
 float pv_rows_integral_amax(const float *v, uint64_t n);
 
+/* Whether an upload of count rows and ncols attribute columns, with free_bytes
+ * of the device's total_bytes left, also makes the arrays that speed up
+ * batches of many filters (13 bytes per row and column, 1 to 4 columns): 1
+ * when the scratch of the largest calls and a quarter of the device stay
+ * free beside them. */
+int pv_rank_tables_fit(uint64_t free_bytes, uint64_t total_bytes, uint64_t count, int ncols);
+
 typedef struct PvBatch PvBatch;
 
 /* Compiles the batch's predicates and copies queries + predicate programs

@@ -83,6 +83,7 @@ def exported_symbols():
 
 
 _EXT_SIGS = {
+    "pv_rank_tables_fit": (C.c_int, [C.c_uint64, C.c_uint64, C.c_uint64, C.c_int]),
     "pv_rows_integral_amax": (C.c_float, [P, C.c_uint64]),
     "pv_pred_check": (C.c_int, [C.c_int, P, P, C.c_int, P, C.c_int, P, C.c_int, C.c_int, P,
                                 C.c_char_p, C.c_size_t]),

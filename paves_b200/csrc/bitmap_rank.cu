@@ -120,13 +120,30 @@ __global__ void rank_check_kernel(const double *__restrict__ col,
     }
 }
 
+// Whether the arrays below may be made: only batches of many filters are
+// faster with them, so they leave the calls' own scratch its room (bitmaps
+// and visited sets of the largest batch, a gathered set, lists and runs) and
+// another index or process a quarter of the device.
+bool rank_tables_fit(uint64_t free_bytes, uint64_t total_bytes, uint64_t count, int ncols) {
+    if (ncols < 1 || ncols > PV_RANK_COLS) return false;
+    const uint64_t tables = (uint64_t)ncols * count * 13 + PV_RANK_COLS * 16;
+    const uint64_t calls = (2ull << 30) + 2ull * FV_GPU_MAX_BATCH * ((count + 31) / 32) * 4;
+    return free_bytes >= tables + std::max(calls, total_bytes / 4);
+}
+
 // Positions, sorted values and codes of every column (tables of at most
 // PV_RANK_COLS columns); a column whose posting rows are no ordering of its
 // values is left out. Runs on g's stream and waits for it.
 cudaError_t build_rank_cols(FvGpuIndex *g) {
     g->rank_cols = g->code_cols = 0;
-    if (g->ncols < 1 || g->ncols > PV_RANK_COLS) return cudaSuccess;
     const uint64_t n = g->count;
+    size_t room = 0, total = 0;
+    if (g->ncols < 1 || g->ncols > PV_RANK_COLS) return cudaSuccess;
+    if (cudaMemGetInfo(&room, &total) != cudaSuccess ||
+        !rank_tables_fit(room, total, n, g->ncols)) {
+        (void)cudaGetLastError();
+        return cudaSuccess;
+    }
     const size_t words = (size_t)g->ncols * n;
     cudaError_t e = cudaMalloc(&g->d_rank, words * 4 + PV_RANK_COLS * 16);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_sorted, words * 8);
@@ -557,3 +574,8 @@ cudaError_t launch_bitmaps_rank(const FvGpuIndex *g, const PredInsn *insns, cons
 }
 
 }  // namespace pv
+
+extern "C" int pv_rank_tables_fit(uint64_t free_bytes, uint64_t total_bytes, uint64_t count,
+                                  int ncols) {
+    return pv::rank_tables_fit(free_bytes, total_bytes, count, ncols) ? 1 : 0;
+}
