@@ -400,6 +400,8 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         g->rows_mixed = (int)h_max[2] <= std::max(samples / 10, (int)(6.0 * sqrt((double)samples)));
     }
 
+    if ((e = pv::tf32_look(g)) != cudaSuccess) return bail("row sample", e);
+
     if (precision != FV_GPU_PREC_FP32) {
         const bool f8 = precision == FV_GPU_PREC_FP8;
         const size_t esz = f8 ? 1 : 2;
@@ -547,6 +549,7 @@ FvGpuIndex *index_view(const FvGpuIndex *g) {
     v->norm32_max = g->norm32_max;
     v->res32_max = g->res32_max;
     v->rows_mixed = g->rows_mixed;
+    v->tf32_blind = g->tf32_blind;
     v->exact_tc = g->exact_tc;
     v->row_amax = g->row_amax;
     v->sorted_cols = g->sorted_cols;

@@ -115,6 +115,7 @@ struct FvGpuIndex {
     float *d_norm32 = nullptr;  // [rows padded to 128] ||x||^2 of the f32 rows
     float norm32_max = 0.f;     // largest of them
     float res32_max = 0.f;      // largest squared part of a row that TF32 drops
+    bool tf32_blind = false;    // rows beyond 128 dims that TF32 does not tell apart (tf32_look)
     // rows in an order unrelated to where they lie (order_kernel): a query's
     // nearest spread over the table, so short lists and samples of tiles serve
     bool rows_mixed = false;

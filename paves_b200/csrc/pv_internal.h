@@ -203,6 +203,7 @@ bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns);
 int tc_superset(const FvGpuIndex *g, uint32_t topb, float q_amax);
 bool tc_supported(const FvGpuIndex *g);
 int tf32_superset(const FvGpuIndex *g, uint32_t topb, float q_amax);
+cudaError_t tf32_look(FvGpuIndex *g);
 bool tf32_supported(const FvGpuIndex *g);
 // Exact-mode batches of at least this many queries scan on the tensor cores
 // (f32 rows read as TF32 + certified exact re-rank); smaller ones stream

@@ -856,6 +856,17 @@ __device__ __forceinline__ void block_sort(uint64_t *keys, int n2) {
 // at its lower end, what the squares and products of tiny values lose is
 // added (without it, rows near 1e-20 that TF32 cannot tell apart passed).
 // Queries that fail are flagged in unc[] for an exact re-run.
+__host__ __device__ inline double tf32_scan_error(int dim, double xm, double xr, double qn,
+                                                  double qr, double A) {
+    const double c2 = (dim + 8) * 0x1p-23;
+    // squares below f32's range: at most half its smallest step a dim in each
+    // of the four sums, and products that the MMA may flush to zero
+    const double lost = dim * 0x1p-149;
+    xm += lost, xr += lost, qn += lost, qr += lost;
+    return 2.0 * (1.0 + 0x1p-6) * (sqrt(xm * qr) + sqrt(xr * qn)) + dim * 0x1p-20 * sqrt(qn * xm) +
+           c2 * (xm + qn + A) + dim * 0x1p-124;
+}
+
 struct RerankCert {
     const float *qnorm = nullptr;  // [nq] ||q||^2 (f32)
     const float *qres = nullptr;   // [nq] ||q - q'||^2 (f32)
@@ -1019,14 +1030,8 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
                 const double A = (double)cand[(size_t)q * S + (S - 1)].dist;
                 const double Dk = (double)key_dist(keys[nout - 1]);
                 const double c2 = (double)(cert.dim + 8) * 0x1p-23;
-                // squares below f32's range: at most half its smallest step a
-                // dim in each of the four sums, and products that the MMA may
-                // flush to zero
-                const double lost = cert.dim * 0x1p-149, xu = xm + lost, qu = qn + lost;
-                const double qr = (double)cert.qres[q] + lost, xr = (double)cert.xrmax + lost;
-                const double E = 2.0 * (1.0 + 0x1p-6) * (sqrt(xu * qr) + sqrt(xr * qu)) +
-                                 cert.dim * 0x1p-20 * sqrt(qu * xu) + c2 * (xu + qu + A) +
-                                 cert.dim * 0x1p-124;
+                const double qr = (double)cert.qres[q], xr = (double)cert.xrmax;
+                const double E = tf32_scan_error(cert.dim, xm, xr, qn, qr, A);
                 ok = ok && (A - E) * (1.0 - c2) > Dk;
                 const double E1 = 1.25 * 0x1p-8 * sqrt(qn * xm) * (1.0 + c2) + c2 * (xm + qn + A);
                 if (again) *again = ok && !((A - E1) * (1.0 - c2) > Dk);
