@@ -379,11 +379,18 @@ static size_t tc_smem(int kblocks, int NS, int KP, int EPI) {
     return tc_smem_bytes(kblocks, NS, KP, EPI, tc_qstream(kblocks));
 }
 
+// Three groups' lists hold every nearest row of the query that a list meets:
+// where rows are stored cluster by cluster, only whole lists do.
+static bool tc_three_groups(const FvGpuIndex *g, int S, int kblocks) {
+    return g->rows_mixed || S <= tc_list_cap(3, kblocks);
+}
+
 bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns) {
     if (!tc_supported(g) || epi < 1 || epi > 3 || ns < 2 || ns > TC_MAX_STAGES) return false;
     const int S = tc_superset(g, topb, -1.f);
     if (!S) return false;
     const int kblocks = g->kpad * (g->precision == FV_GPU_PREC_FP8 ? 1 : 2) / TC_KB_BYTES;
+    if (epi == 3 && !tc_three_groups(g, S, kblocks)) return false;
     const int KP = std::min(S, tc_list_cap(epi, kblocks));
     return tc_smem(kblocks, ns, KP, epi) <= 227 * 1024;
 }
@@ -475,20 +482,16 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
             NS = 2;
         }
     };
-    // (three groups' lists hold every nearest row of the query that a list
-    // meets: where rows are stored cluster by cluster, only whole lists do;
-    // and a run that spills may be full, which flags the query)
-    const bool whole3 = S <= tc_list_cap(3, kblocks);
-    const bool three = whole3 || (g->rows_mixed && redo);
+    // (and a run that spills may be full, which flags the query)
+    const bool three = S <= tc_list_cap(3, kblocks) || (redo && tc_three_groups(g, S, kblocks));
     shape(kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 && three ? 3 : 2);
-    bool tuned = false;
     if (g->tune_epi || g->tune_ns) {  // a tuned shape, if it fits
-        const int e = g->tune_epi ? g->tune_epi : EPI, n = g->tune_ns ? g->tune_ns : NS;
-        if (e >= 1 && e <= 3 && n >= 2 && n <= TC_MAX_STAGES &&
+        const int e = std::min(g->tune_epi ? g->tune_epi : EPI, three ? 3 : 2);
+        const int n = g->tune_ns ? g->tune_ns : NS;
+        if (e >= 1 && n >= 2 && n <= TC_MAX_STAGES &&
             tc_smem(kblocks, n, std::min(S, tc_list_cap(e, kblocks)), e) <= smem_cap) {
             EPI = e;
             NS = n;
-            tuned = true;
         }
     }
     int KP = std::min(S, tc_list_cap(EPI, kblocks));
@@ -575,7 +578,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
                         admits * std::min(32, qtiles > 1 ? 32 : nq) <= 150.0;
     const bool seed = g->tune_seed != 2 && !little && enough();
     if (!seed) {
-        if (EPI == 3 && !tuned) {  // without a bound: lists that keep the best
+        if (EPI == 3) {  // without a bound: lists that keep the best
             shape(2);
             KP = std::min(S, tc_list_cap(EPI, kblocks));
             certify = KP < S;
