@@ -214,6 +214,10 @@ __device__ __forceinline__ void graph_dists(const GraphArgs &a, const float *sq,
 // filter at ef 64 (403 steps, a frontier of thousands) 3.3 ms against 5.4,
 // 0.15 % (8 queries, 2294 steps) 17.6 ms against 43.7; 60,000 rows, 10 %:
 // 0.16 ms, 3.1 us a step with every read in L2, against 0.24.
+//
+// WIDE: rows of so many dims that the query has no room beside the search's
+// arrays; it is read where it lies.
+template <bool WIDE>
 __global__ void __launch_bounds__(G_THREADS) graph_kernel(GraphArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t *const fm0 = (uint64_t *)smem_raw;  // [2][G_FC] frontier: the rest
@@ -224,7 +228,7 @@ __global__ void __launch_bounds__(G_THREADS) graph_kernel(GraphArgs a) {
     uint32_t *nid = hash + G_HC;                 // [G_NB] gathered neighbours
     int *rpos = (int *)(nid + G_NB);             // [G_NB] new results' places
     int *fpos = rpos + G_NB;                     // [G_NB] new frontier keys' places
-    float *sq = (float *)(fpos + G_NB);          // [dpad] query
+    float *s_q = (float *)(fpos + G_NB);         // [dpad] query
 
     // a step's counts: fresh neighbours, admitted keys, passing ones (two
     // sets: the next step's are cleared while this one's are read)
@@ -251,7 +255,9 @@ __global__ void __launch_bounds__(G_THREADS) graph_kernel(GraphArgs a) {
     uint32_t *vb = a.visited_bits + (uint64_t)q * a.bm_words;
     const float *qv = a.queries + (uint64_t)q * a.dpad;
 
-    for (int i = tid; i < a.dpad; i += blockDim.x) sq[i] = qv[i];
+    const float *sq = WIDE ? qv : s_q;
+    if (!WIDE)
+        for (int i = tid; i < a.dpad; i += blockDim.x) s_q[i] = qv[i];
     for (int i = tid; i < G_HC; i += blockDim.x) hash[i] = G_EMPTY;
     if (tid < 6) s_cnt[tid / 3][tid % 3] = 0;
     if (tid == 0) s_hcount = 1;
@@ -584,16 +590,20 @@ __global__ void __launch_bounds__(G_THREADS) graph_kernel(GraphArgs a) {
     }
 }
 
-size_t graph_smem_bytes(int dpad) {
+constexpr int G_DIMS = 11460;  // dims at most
+size_t graph_smem_bytes(int dpad) {  // without the query: 0 dims
     return (size_t)(2 * G_FC + 2 * G_BC + 2 * G_RC + G_NB + 2) * 8 +
            (size_t)(G_HC + 3 * G_NB) * 4 + (size_t)dpad * 4;
 }
 
 cudaError_t launch_graph(const GraphArgs &a, int nq, cudaStream_t st) {
-    const size_t smem = graph_smem_bytes(a.dpad);
-    cudaError_t e = raise_smem_limit((const void *)graph_kernel, smem);
+    if (a.dpad > G_DIMS) return cudaErrorInvalidValue;
+    const bool wide = graph_smem_bytes(a.dpad) > 227 * 1024 - 256;  // (28 bytes static)
+    const size_t smem = graph_smem_bytes(wide ? 0 : a.dpad);
+    auto *kernel = wide ? graph_kernel<true> : graph_kernel<false>;
+    cudaError_t e = raise_smem_limit((const void *)kernel, smem);
     if (e != cudaSuccess) return e;
-    graph_kernel<<<nq, G_THREADS, smem, st>>>(a);
+    kernel<<<nq, G_THREADS, smem, st>>>(a);
     return cudaGetLastError();
 }
 
