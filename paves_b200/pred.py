@@ -124,7 +124,11 @@ _KIND = {And: FV_NODE_AND, Or: FV_NODE_OR, Not: FV_NODE_NOT}
 
 
 def _i32(v) -> int:
-    return v if type(v) is int else int(np.int32(v))
+    if type(v) is int and -2 ** 31 <= v < 2 ** 31:
+        return v
+    cell = np.zeros(1, np.int32)
+    cell[0] = v  # refuses and converts as an assignment to a record does
+    return int(cell[0])
 
 
 def _flat(n: Pred, recs: list, children: list, invals: list, at=(0, 0, 0)) -> int:
@@ -140,8 +144,8 @@ def _flat(n: Pred, recs: list, children: list, invals: list, at=(0, 0, 0)) -> in
         recs.append(_record(FV_NODE_IN, _i32(n.col), 0, 0, c0, len(n.values), v0, 0, 0.0))
         invals.extend(n.values)
     else:
-        kids = n.children
-        recs.append(_record(_KIND[type(n)], 0, 0, len(kids), c0, 0, v0, 0, 0.0))
+        kind, kids = _KIND[type(n)], n.children
+        recs.append(_record(kind, 0, 0, len(kids), c0, 0, v0, 0, 0.0))
         j = len(children)
         children.extend(kids)  # their places, once they have them
         for k in kids:
@@ -178,10 +182,16 @@ def concat(preds: Sequence[Optional[Pred]], count: int,
     qd["need_eval"] = 1
     qd["total"] = count
     if entries is not None:
-        e = entries if isinstance(entries, np.ndarray) else np.asarray(entries, qd["entry"].dtype)
-        if len(e) < nq:
-            raise IndexError(f"{len(e)} entry nodes for {nq} queries")
-        qd["entry"] = e[:nq]
+        e = entries
+        if isinstance(e, (list, tuple, range)):
+            e = np.asarray(e, qd["entry"].dtype)
+        if isinstance(e, np.ndarray) and e.ndim == 1:
+            if len(e) < nq:
+                raise IndexError(f"{len(e)} entry nodes for {nq} queries")
+            qd["entry"] = e[:nq]
+        else:  # whatever takes an index
+            for q in range(nq):
+                qd[q]["entry"] = entries[q]
     recs, children, invals = [], [], []
     if nq - sum(p is None for p in preds) <= 8:
         # a few filters: every query's slice in place (the gather below costs
