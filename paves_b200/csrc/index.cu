@@ -132,8 +132,7 @@ __global__ void to_fp8_kernel(const float *__restrict__ src, int dpad, int dim,
 // [cnt, n0, n1, ...] rows of stride l0_stride -> fixed-width adjacency.
 // Out-of-range neighbour ids are dropped (they would otherwise be followed).
 __global__ void adj_kernel(const uint32_t *__restrict__ l0, uint32_t l0_stride,
-                           uint64_t nrows, int deg_cap, uint32_t *__restrict__ adj,
-                           uint16_t *__restrict__ deg) {
+                           uint64_t nrows, int deg_cap, uint32_t *__restrict__ adj) {
     uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= nrows) return;
     const uint32_t *src = l0 + row * l0_stride;
@@ -144,7 +143,6 @@ __global__ void adj_kernel(const uint32_t *__restrict__ l0, uint32_t l0_stride,
         uint32_t v = src[1 + i];
         if (v < nrows) adj[row * deg_cap + n++] = v;
     }
-    deg[row] = (uint16_t)n;
     for (int i = n; i < deg_cap; i++) adj[row * deg_cap + i] = 0xFFFFFFFFu;
 }
 
@@ -235,7 +233,6 @@ extern "C" void fv_gpu_index_free(FvGpuIndex *g) {
         cudaFree(g->d_code);
         cudaFree(g->d_sorted);
         cudaFree(g->d_adj);
-        cudaFree(g->d_deg);
         cudaFree(g->d_vlow);
         cudaFree(g->d_vscale);
         cudaFree(g->d_norm);
@@ -293,7 +290,7 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
     const int kpad = precision == FV_GPU_PREC_FP8 ? (dim + 127) & ~127 : (dim + 63) & ~63;
     const uint64_t rows_pad = (count + 127) & ~127ull;  // norms/scales per 128-row tile
     size_t need = count * (size_t)dpad * 4 + count * (size_t)ncols * 12;
-    if (l0) need += count * (size_t)(l0_stride - 1) * 4 + count * 2;
+    if (l0) need += count * (size_t)(l0_stride - 1) * 4;
     if (precision != FV_GPU_PREC_FP32) need += count * (size_t)kpad * 2 + count * 8;
     if (device < 0) device = pick_device(need);
     if (device < 0) return fail("no CUDA device with enough free memory", cudaSuccess);
@@ -359,10 +356,9 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         e = cudaMemcpyAsync(d_l0, l0, count * (size_t)l0_stride * 4, cudaMemcpyHostToDevice,
                             g->stream);
         if (e == cudaSuccess) e = cudaMalloc(&g->d_adj, count * (size_t)g->deg_cap * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&g->d_deg, count * 2);
         if (e == cudaSuccess) {
             adj_kernel<<<(unsigned)((count + 255) / 256), 256, 0, g->stream>>>(
-                d_l0, l0_stride, count, g->deg_cap, g->d_adj, g->d_deg);
+                d_l0, l0_stride, count, g->deg_cap, g->d_adj);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
@@ -539,7 +535,6 @@ FvGpuIndex *index_view(const FvGpuIndex *g) {
     v->rank_cols = g->rank_cols;
     v->code_cols = g->code_cols;
     v->d_adj = g->d_adj;
-    v->d_deg = g->d_deg;
     v->deg_cap = g->deg_cap;
     v->kpad = g->kpad;
     v->d_vlow = g->d_vlow;

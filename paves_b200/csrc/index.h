@@ -100,9 +100,8 @@ struct FvGpuIndex {
     int rank_cols = 0, code_cols = 0;
 
     // level-0 graph as fixed-degree device adjacency ("device CSR"):
-    // d_adj[node*deg_cap + i], padded with UINT32_MAX; d_deg[node]
+    // d_adj[node*deg_cap + i], padded with UINT32_MAX
     uint32_t *d_adj = nullptr;
-    uint16_t *d_deg = nullptr;
     int deg_cap = 0;
 
     // reduced-precision copies (precision != FP32)
