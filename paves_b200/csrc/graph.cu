@@ -294,6 +294,9 @@ __global__ void __launch_bounds__(G_THREADS) graph_kernel(GraphArgs a) {
     unsigned long long visited = 1;
     unsigned int probes = 0, steps = 0;
     int exh = 0;
+    // the step's nodes; t0 > 0: the rest of a list longer than G_NB is next
+    uint32_t selnode = 0;
+    int nsel = 0, t0 = 0;
 
     for (;;) {
         // ---- selection (by every warp): the best W entries, cut at the
@@ -329,49 +332,51 @@ __global__ void __launch_bounds__(G_THREADS) graph_kernel(GraphArgs a) {
             me -= e - lo;
             dropped = true;
         }
-        const int nb = be - bh, nm = me - mh, avail = nb + nm;
-        // an empty frontier is exhaustion unless entries were dropped (they
-        // would still sit in an unbounded candidate queue)
-        if (avail <= 0) {
-            exh = dropped ? 0 : 1;
-            break;
-        }
-        if (visited >= a.max_visited) {
-            exh = 1;
-            break;
-        }
-        const int w = min(avail, a.wmax);
-        const uint64_t own = lane < G_WMAX ? (lane < nb ? FB[bh + lane] : KEY_MAX)
-                                           : (lane - G_WMAX < nm ? FM[mh + lane - G_WMAX] : KEY_MAX);
-        uint64_t k = own;
-        if (nm > 0) {
-#pragma unroll
-            for (int s = 16; s; s >>= 1) {  // two ascending halves: reverse one, then clean
-                const uint64_t o = s == 16 ? __shfl_sync(0xffffffffu, k, 31 - lane)
-                                           : __shfl_xor_sync(0xffffffffu, k, s);
-                const bool low = (lane & s) == 0;
-                k = low ? (k < o ? k : o) : (k > o ? k : o);
+        if (t0 == 0) {
+            const int nb = be - bh, nm = me - mh, avail = nb + nm;
+            // an empty frontier is exhaustion unless entries were dropped (they
+            // would still sit in an unbounded candidate queue)
+            if (avail <= 0) {
+                exh = dropped ? 0 : 1;
+                break;
             }
+            if (visited >= a.max_visited) {
+                exh = 1;
+                break;
+            }
+            const int w = min(avail, a.wmax);
+            const uint64_t own = lane < G_WMAX ? (lane < nb ? FB[bh + lane] : KEY_MAX)
+                                               : (lane - G_WMAX < nm ? FM[mh + lane - G_WMAX] : KEY_MAX);
+            uint64_t k = own;
+            if (nm > 0) {
+#pragma unroll
+                for (int s = 16; s; s >>= 1) {  // two ascending halves: reverse one, then clean
+                    const uint64_t o = s == 16 ? __shfl_sync(0xffffffffu, k, 31 - lane)
+                                               : __shfl_xor_sync(0xffffffffu, k, s);
+                    const bool low = (lane & s) == 0;
+                    k = low ? (k < o ? k : o) : (k > o ? k : o);
+                }
+            }
+            const bool okl = lane < w && (lane == 0 || !full || !(key_dist(k) > worst));
+            const unsigned okm = __ballot_sync(0xffffffffu, okl);
+            nsel = okm == 0xffffffffu ? 32 : __ffs(~okm) - 1;  // leading run
+            if (full && key_dist(__shfl_sync(0xffffffffu, k, 0)) > worst) break;
+            selnode = grow_of(k);
+            const uint64_t klast = __shfl_sync(0xffffffffu, k, nsel - 1);
+            const int fromb =
+                __popc(__ballot_sync(0xffffffffu, lane < G_WMAX && lane < nb && own <= klast));
+            bh += fromb;
+            mh += nsel - fromb;
         }
-        const bool okl = lane < w && (lane == 0 || !full || !(key_dist(k) > worst));
-        const unsigned okm = __ballot_sync(0xffffffffu, okl);
-        const int nsel = okm == 0xffffffffu ? 32 : __ffs(~okm) - 1;  // leading run
-        if (full && key_dist(__shfl_sync(0xffffffffu, k, 0)) > worst) break;
-        const uint32_t selnode = grow_of(k);
-        const uint64_t klast = __shfl_sync(0xffffffffu, k, nsel - 1);
-        const int fromb =
-            __popc(__ballot_sync(0xffffffffu, lane < G_WMAX && lane < nb && own <= klast));
-        bh += fromb;
-        mh += nsel - fromb;
         int *cnt = s_cnt[steps & 1];
         steps++;
 
         // ---- gather neighbours of the selected nodes, visited test-and-set
-        // (lists are padded to deg_cap with ids no row has; one round unless
-        // a single list is longer than G_NB)
+        // (lists are padded to deg_cap with ids no row has; G_NB of them at a
+        // time, which is all unless a single list is longer)
         const int dc = a.deg_cap;
         const int total = nsel * dc;
-        for (int t0 = 0; t0 < total; t0 += G_NB) {
+        {
             constexpr int SL = G_NB / G_THREADS;
             uint32_t nv[SL];
             bool fresh[SL];
@@ -425,6 +430,7 @@ __global__ void __launch_bounds__(G_THREADS) graph_kernel(GraphArgs a) {
                 wb += __popc(fmask[u]);
             }
         }
+        t0 = t0 + G_NB < total ? t0 + G_NB : 0;
         if (tid < 3) s_cnt[steps & 1][tid] = 0;  // the next step's
         __syncthreads();
         const int nnew = min(cnt[0], G_NB);
