@@ -397,18 +397,21 @@ struct HgWait {
     int batch = -1;
 };
 
-// Workspace of the levels, sized for the largest (level 0 has the most rows
-// and the longest lists, an upper level may have the longest answers), and
-// the upper levels' rows: one allocation (17 of them, and their frees, took
-// 3 of a build's 30 ms and at times ten times that).
+// Workspace of a level: one allocation (17 of them, and their frees, took 3 of
+// a build's 30 ms and at times ten times that), laid out for level 0 and then
+// for the upper levels, whose rows take what level 0 no longer needs.
 struct HgWork {
     void *base = nullptr;
     DevArr qprog, popcnt, out, cnt, tr, tails, lst, lcnt, in_cnt, in_off, cursor, rev, lists;
-    DevArr ids, xs, los, norms;  // of n1 rows
+    DevArr ids, xs, los, norms;  // upper levels: the rows gathered
     ~HgWork() {
         if (base) cudaFree(base);
     }
-    cudaError_t alloc(uint64_t n, uint64_t n1, int topb, int R, int dpad, size_t lo_bytes) {
+    // A level of n rows with lists of R and answers of topb, the rows gathered
+    // or not (dpad f32 and lo_bytes of low-precision row each). The bytes it
+    // takes from base on.
+    size_t layout(uint64_t n, int topb, int R, int dpad, size_t lo_bytes, bool gathered) {
+        const uint64_t n1 = gathered ? n : 0;
         const struct {
             DevArr *a;
             size_t bytes;
@@ -430,16 +433,12 @@ struct HgWork {
                      {&xs, (size_t)n1 * dpad * 4},
                      {&los, (size_t)n1 * lo_bytes},
                      {&norms, (size_t)((n1 + 127) & ~127ull) * 4}};  // whole tiles
-        size_t bytes = 0;
-        for (const auto &p : parts) bytes += (p.bytes + 255) & ~(size_t)255;
-        const cudaError_t e = cudaMalloc(&base, bytes);
-        if (e != cudaSuccess) return e;
         char *at = (char *)base;
         for (const auto &p : parts) {
             p.a->p = at;
             at += (p.bytes + 255) & ~(size_t)255;
         }
-        return cudaSuccess;
+        return (size_t)(at - (char *)base);
     }
 };
 
@@ -585,13 +584,18 @@ int build_levels(PvHnsw *h, FvGpuIndex *g, int M, int candidates, int top, const
     auto upper = [&](uint64_t n) {
         return (int)std::min<uint64_t>((uint64_t)std::min(2 * candidates + 1, 1023), n - 1);
     };
-    const int C1 = ids.size() >= 2 ? upper(ids.size()) : 0;
     HgWork w;
     const bool low = g->d_vlow != nullptr;
     const size_t lo_bytes = low ? (size_t)g->kpad * (g->precision == FV_GPU_PREC_FP8 ? 1 : 2) : 0;
-    HG_OK(w.alloc(count, ids.size(),
-                  (int)std::min<uint64_t>((uint64_t)std::max(candidates, C1) + 1, count), 2 * M,
-                  g->dpad, lo_bytes));
+    auto lay_upper = [&]() {
+        return w.layout(ids.size(), upper(ids.size()) + 1, M, g->dpad, lo_bytes, true);
+    };
+    auto lay_level0 = [&]() {
+        return w.layout(count, (int)std::min<uint64_t>((uint64_t)candidates + 1, count), 2 * M,
+                        g->dpad, lo_bytes, false);
+    };
+    HG_OK(cudaMalloc(&w.base, std::max(ids.size() >= 2 ? lay_upper() : 0, lay_level0())));
+    lay_level0();
     if (g->precision != FV_GPU_PREC_FP32 && tc_supported(g)) {
         // the tensor-core scans' scratch at its largest batch: growing with
         // the doubling batches, it was freed and allocated anew ten times
@@ -611,6 +615,7 @@ int build_levels(PvHnsw *h, FvGpuIndex *g, int M, int candidates, int top, const
     HG_OK(cudaMemcpy(hnsw_l0(h), w.lists.p, (size_t)count * (2 * M + 1) * 4,
                      cudaMemcpyDeviceToHost));
     if (ids.size() < 2) return 0;  // a single node has no neighbours
+    lay_upper();
     HG_OK(cudaMemsetAsync(w.norms.p, 0, ((ids.size() + 127) & ~127ull) * 4, g->stream));
     const auto vecs = g->d_vecs;
     const auto vlow = g->d_vlow;
