@@ -24,7 +24,7 @@
 // general kernel 2.80 ms, one position test per filter 0.55 ms; writing the
 // words alone, 128 MB, takes 0.02 ms), 29 filters 0.022 ms (0.037; general
 // kernel 0.157 ms). Six filters over 1M rows take these three 0.022 ms,
-// bitmap_few_kernel 0.014.
+// bitmap_few_kernel 0.014. Where they pay: rank_pays.
 #include <string.h>
 
 #include <algorithm>
@@ -179,6 +179,18 @@ cudaError_t build_rank_cols(FvGpuIndex *g) {
         if (h[c * 4 + 2] == 0) g->code_cols |= 1 << c;
     }
     return cudaSuccess;
+}
+
+// Whether the three kernels are faster than the general one for P programs:
+// that takes 2.3 ps a row and program beyond its first wave, these take 5 us
+// of launches and 0.04 us a program (ends, tables and their loads) whatever
+// the rows are. Measured, in us with the batch's query prep, general kernel
+// against these: 9 programs over 200,000 rows 20 and 22, over 400,000 26 and
+// 22; 32 over 60,000 27 and 29, 100,000 33 and 31; 128 over 20,000 31 and
+// 39, 60,000 42 and 40; 1000 over 20,000 75 and 77, 2,000 31 and 71.
+bool rank_pays(uint64_t rows, int P) {
+    return P >= PV_RANK_MIN_PROGS && P <= PV_RANK_MAX_PROGS &&
+           rows * (uint64_t)P >= 2400000ull + 25000ull * (uint64_t)P;
 }
 
 // Whether every program of a batch has the form these kernels take.

@@ -81,7 +81,7 @@ int brute_prepare(FvGpuIndex *g, int nq, const float *queries, const PredBatch &
                    std::all_of(pb.progs.begin(), pb.progs.end(), well_formed);
     // many range-form programs: the position form (up to eight take
     // bitmap_few_kernel, which has no tables to make first)
-    db.rank_ok = P >= PV_RANK_MIN_PROGS && P <= PV_RANK_MAX_PROGS && rank_batch_ok(g, pb);
+    db.rank_ok = rank_pays(g->count, P) && rank_batch_ok(g, pb);
     if (db.rank_ok)
         PV_CUDA_OK(g->scan.rank_tab.ensure(rank_tab_bytes(P)), errbuf, errlen);
     // sparse route: one filter shared by the whole batch whose matches are
@@ -134,7 +134,7 @@ int brute_bitmaps(FvGpuIndex *g, const DevBatch &db, char *errbuf, size_t errlen
                                          d_counts, P, db.ninsns, db.nconsts, bm, bm_words, pop,
                                          g->sm_count, g->stream, g->ncols),
                    errbuf, errlen);
-        if (!g->rank_cols || P > PV_RANK_MAX_PROGS) return 0;
+        if (!g->rank_cols || !rank_pays(g->count, P)) return 0;  // (nor for fewer)
         PV_CUDA_OK(s.rank_tab.ensure(rank_tab_bytes(P)), errbuf, errlen);
         g->launches += 3;
         PV_CUDA_OK(launch_bitmaps_rank(g, d_insns, d_progs, d_consts, P, d_counts + 4,

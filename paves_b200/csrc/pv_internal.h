@@ -36,6 +36,7 @@ constexpr int PV_RANK_MIN_PROGS = 9;
 constexpr int PV_RANK_MAX_PROGS = 1024;  // its tables of four columns fit a block
 size_t rank_tab_bytes(int P);
 cudaError_t build_rank_cols(FvGpuIndex *g);
+bool rank_pays(uint64_t rows, int P);
 bool rank_batch_ok(const FvGpuIndex *g, const PredBatch &pb);
 cudaError_t launch_bitmaps_rank(const FvGpuIndex *g, const PredInsn *insns, const PredProg *progs,
                                 const double *consts, int P, const int *dP, void *tab,

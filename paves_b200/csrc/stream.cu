@@ -145,7 +145,8 @@ int stage(Bucket &b, const FvGpuIndex *g, int nq, const float *queries, const Pr
     int32_t *cnt = (int32_t *)(h + b.db.off_counts);
     // all programs in the position form: the rank kernels take them (cnt[4]),
     // else the general one does (cnt[0])
-    const bool rank = !lazy && P >= PV_RANK_MIN_PROGS && b.db.P <= PV_RANK_MAX_PROGS && rank_batch_ok(g, pb);
+    const bool rank = !lazy && rank_pays(g->count, P) && rank_pays(g->count, b.db.P) &&
+                      rank_batch_ok(g, pb);
     cnt[0] = lazy || rank ? 0 : P;
     cnt[4] = rank ? P : 0;
     cnt[1] = (int)pb.insns.size();
