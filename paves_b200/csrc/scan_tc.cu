@@ -567,15 +567,19 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // Nor does it pay when lists fill little without a bound: few kept keys
     // for the merge and few admissions per warp (one tile per CTA, a list's
     // passing rows p; it keeps min(S, p) and admits about S (1 + ln(p / S))).
-    // The sample and its merge take 15 to 20 us; 1 to 7 queries of 50,000 to
+    // The sample and its merge take 8 to 20 us; 1 to 7 queries of 50,000 to
     // 100,000 rows with k of 1 or 2, or 1.6 % of the rows passing, took 10 to
-    // 20 us more with them.
+    // 20 us more with them. (The lines, over 6,000 batches of 1 to 300
+    // queries: the merge takes what the sample saves from 5,000 kept keys on,
+    // from 4,400 with 100 admissions a warp; the pass does from 150
+    // admissions on. Below, unseeded is 1 to 10 us faster; a little beyond, 2
+    // to 10 slower.)
     const uint64_t ugrow = std::min<uint64_t>(std::max(1, g->sm_count / qtiles), ntiles_all);
     const double p = pass * (double)nrows_scan / (double)(ugrow * EPI * R);
     const double kept = std::min<double>(KP, p);
     const double admits = p <= KP ? p : KP * (1.0 + log(p / KP));
-    const bool little = kept * ugrow * EPI * R <= 3000.0 &&
-                        admits * std::min(32, qtiles > 1 ? 32 : nq) <= 150.0;
+    const double per_warp = admits * std::min(32, qtiles > 1 ? 32 : nq);
+    const bool little = per_warp <= 150.0 && kept * ugrow * EPI * R + 8.0 * per_warp <= 5200.0;
     const bool seed = g->tune_seed != 2 && !little && enough();
     if (!seed) {
         if (EPI == 3) {  // without a bound: lists that keep the best
