@@ -204,7 +204,8 @@ int brute_launch(FvGpuIndex *g, DevBatch &db, uint32_t topb, int mode, FvHit *d_
     const bool exact_mode = mode == PV_MODE_EXACT || (mode == 1 && !tc_supported(g));
     const bool exact_tc_can = exact_mode && nq >= PV_EXACT_TC_MIN_NQ &&
                               (db.redo || g->dpad <= 128) &&
-                              tf32_supported(g) && tf32_superset(g, topb, db.q_amax) > 0;
+                              tf32_supported(g) && tf32_superset(g, topb, db.q_amax) > 0 &&
+                              tf32_pays(g, topb, tf32_superset(g, topb, db.q_amax), db.pass);
     bool sparse_tc = sparse_route && (low_tc_can || exact_tc_can) &&
                      db.sparse_bound >= PV_SPARSE_TC_MIN_ROWS;
     uint64_t list_bound = db.sparse_bound;

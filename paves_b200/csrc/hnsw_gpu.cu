@@ -710,8 +710,7 @@ extern "C" PvHnsw *pv_hnsw_build_gpu_wait(const float *vectors, uint64_t count, 
         pv_hnsw_free(h);
         return nullptr;
     };
-    FvGpuIndex *g = fv_gpu_index_upload(vectors, nullptr, nullptr, nullptr, 0, count, dim, 0,
-                                        device, precision, errbuf, errlen);
+    FvGpuIndex *g = upload_rows(vectors, count, dim, device, precision, errbuf, errlen);
     if (!g) return fail();
     const int rc = build_levels(h, g, M, candidates, top, HgWait{wait_ns, wait_batch}, errbuf, errlen);
     fv_gpu_index_free(g);

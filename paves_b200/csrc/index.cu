@@ -267,7 +267,7 @@ struct Prepared {
 FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t *post_rows,
                         const uint32_t *l0, uint32_t l0_stride, uint64_t count, int dim,
                         int ncols, int device, int precision, const Prepared *prep,
-                        char *errbuf, size_t errlen) {
+                        char *errbuf, size_t errlen, bool look = true) {
     auto fail = [&](const char *what, cudaError_t e) -> FvGpuIndex * {
         if (errbuf && errlen)
             snprintf(errbuf, errlen, "gpu: index upload: %s%s%s", what, e ? ": " : "",
@@ -396,8 +396,6 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         g->rows_mixed = (int)h_max[2] <= std::max(samples / 10, (int)(6.0 * sqrt((double)samples)));
     }
 
-    if ((e = pv::tf32_look(g)) != cudaSuccess) return bail("row sample", e);
-
     if (precision != FV_GPU_PREC_FP32) {
         const bool f8 = precision == FV_GPU_PREC_FP8;
         const size_t esz = f8 ? 1 : 2;
@@ -436,6 +434,7 @@ FvGpuIndex *upload_impl(const float *vectors, const double *cols, const uint32_t
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return bail("convert", e);
     }
+    if (look) pv::tf32_look(g, vectors);
     // last: what it allocates is left out where there is no room for it
     if ((e = pv::build_rank_cols(g)) != cudaSuccess) return bail("column positions", e);
     // the caller's arrays may go once this returns
@@ -452,6 +451,13 @@ extern "C" FvGpuIndex *fv_gpu_index_upload(const float *vectors, const double *c
                                            char *errbuf, size_t errlen) {
     return upload_impl(vectors, cols, post_rows, l0, l0_stride, count, dim, ncols, device,
                        precision, nullptr, errbuf, errlen);
+}
+
+// The rows alone, for scans that do not choose their route (the graph builder).
+FvGpuIndex *pv::upload_rows(const float *vectors, uint64_t count, int dim, int device,
+                            int precision, char *errbuf, size_t errlen) {
+    return upload_impl(vectors, nullptr, nullptr, nullptr, 0, count, dim, 0, device, precision,
+                       nullptr, errbuf, errlen, false);
 }
 
 extern "C" FvGpuIndex *pv_index_upload_prepared(const float *vectors, const double *cols,
@@ -544,7 +550,7 @@ FvGpuIndex *index_view(const FvGpuIndex *g) {
     v->norm32_max = g->norm32_max;
     v->res32_max = g->res32_max;
     v->rows_mixed = g->rows_mixed;
-    v->tf32_blind = g->tf32_blind;
+    memcpy(v->tf32_share, g->tf32_share, sizeof(v->tf32_share));
     v->exact_tc = g->exact_tc;
     v->row_amax = g->row_amax;
     v->sorted_cols = g->sorted_cols;

@@ -204,7 +204,8 @@ bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns);
 int tc_superset(const FvGpuIndex *g, uint32_t topb, float q_amax);
 bool tc_supported(const FvGpuIndex *g);
 int tf32_superset(const FvGpuIndex *g, uint32_t topb, float q_amax);
-cudaError_t tf32_look(FvGpuIndex *g);
+void tf32_look(FvGpuIndex *g, const float *vectors);
+bool tf32_pays(const FvGpuIndex *g, uint32_t topb, int S, double pass);
 bool tf32_supported(const FvGpuIndex *g);
 // Exact-mode batches of at least this many queries scan on the tensor cores
 // (f32 rows read as TF32 + certified exact re-rank); smaller ones stream
@@ -260,6 +261,9 @@ inline size_t tc_tail_bytes(int nq) { return TC_TAIL_UNC + (size_t)nq; }
 // Queues its copy into pinned h on g's stream (after the results' copy); the
 // next check_tc_watchdog and the re-run read it there.
 void tc_tail_enqueue(FvGpuIndex *g, char *h);
+
+FvGpuIndex *upload_rows(const float *vectors, uint64_t count, int dim, int device, int precision,
+                        char *errbuf, size_t errlen);  // index.cu
 
 // ---- HNSW sections (hnsw_build.cpp) for the GPU builder (hnsw_gpu.cu)
 }  // namespace pv

@@ -278,87 +278,86 @@ int tc_superset(const FvGpuIndex *g, uint32_t topb, float q_amax) {
 // certifiable: such a table is scanned on the CUDA cores at once.
 int tf32_superset(const FvGpuIndex *g, uint32_t topb, float q_amax) {
     const bool exact = !g->force_wide_superset && pv_bf16_exact(g->dim, g->row_amax, q_amax);
-    if (!exact && (g->tf32_blind || !(g->norm32_max < 0x1p126f))) return 0;
+    if (!exact && !(g->norm32_max < 0x1p126f)) return 0;
     const int s = exact ? (int)topb : std::max(4 * (int)topb, 16);
     return s <= TC_MAX_SUPERSET ? s : 0;
 }
 
-// Of 32 rows as queries: squared distances to `samples` rows spread over the
-// table, their own norm and what TF32 rounds off them (query_prep_row).
-constexpr int TS_Q = 32;
-__global__ void __launch_bounds__(256)
-tf32_sample_kernel(const float *__restrict__ vecs, int dpad, uint64_t nrows, int samples,
-                   float *__restrict__ dist, float *__restrict__ qn, float *__restrict__ qr) {
-    const int p = blockIdx.y, lane = threadIdx.x & 31;
-    const int t = (int)(blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5));
-    if (t >= samples) return;
-    const uint64_t i = p * nrows / TS_Q, j = t * nrows / samples;
-    float d = 0.f, n = 0.f, r = 0.f;
-    for (int k = lane; k < dpad; k += 32) {
-        const float v = vecs[i * dpad + k], w = v - vecs[j * dpad + k];
-        const uint32_t u = __float_as_uint(v);
-        const float e = v - __uint_as_float((u + 0xFFFu + ((u >> 13) & 1u)) & 0xFFFFE000u);
-        d = fmaf(w, w, d);
-        n = fmaf(v, v, n);
-        r = fmaf(e, e, r);
+// For which k a table of rows beyond 128 dims goes through TF32 at all. Below
+// that width every batch of 16+ queries does; wider rows were the CUDA-core
+// scan's alone, and where the certificate then sends most queries there after
+// all, the call takes half as long again: 64 real-valued queries of 60,000 x
+// 512 rows in clusters of 200, k 10 0.48 ms instead of 0.37, 0.37 through
+// TF32 alone for k 100. So 16 rows are looked up at upload by the exact scan,
+// and for k of 1, 2, 4 .. the share of them is kept whose gap between the
+// k-th and the superset's last distance the certificate's bound would leave
+// open (about a millisecond beside 31 for 300 MB of rows).
+constexpr int TL_Q = 16, TL_K = 512;
+void tf32_look(FvGpuIndex *g, const float *vectors) {
+    memset(g->tf32_share, 0, sizeof(g->tf32_share));
+    if (g->dpad <= 128 || !tf32_supported(g) || !(g->norm32_max < 0x1p126f) ||
+        tc_supported(g))  // (the low-precision rows are scanned)
+        return;
+    std::vector<float> q((size_t)TL_Q * g->dim);
+    PredBatch none;
+    none.qprog.assign(TL_Q, -1);
+    for (int p = 0; p < TL_Q; p++)
+        memcpy(&q[(size_t)p * g->dim], vectors + (p * g->count / TL_Q) * (uint64_t)g->dim,
+               sizeof(float) * g->dim);
+    std::vector<FvHit> hits((size_t)TL_Q * TL_K);
+    std::vector<uint32_t> cnt(TL_Q);
+    std::vector<uint8_t> tr(TL_Q);
+    char err[256];
+    const int bad = brute_run_host(g, TL_Q, q.data(), none, TL_K, PV_MODE_SIMT, hits.data(),
+                                   cnt.data(), tr.data(), err, sizeof(err));
+    g->launches = 0;
+    g->last_kernel_ms = 0.f;
+    if (bad) {  // (no room, say: the CUDA-core scan it is)
+        (void)cudaGetLastError();
+        return;
     }
-    for (int o = 16; o; o >>= 1) {
-        d += __shfl_xor_sync(0xffffffffu, d, o);
-        n += __shfl_xor_sync(0xffffffffu, n, o);
-        r += __shfl_xor_sync(0xffffffffu, r, o);
-    }
-    if (lane == 0) {
-        dist[p * samples + t] = i == j ? __int_as_float(0x7f800000) : d;
-        if (t == 0) {
-            qn[p] = n;
-            qr[p] = r;
+    const double c2 = (g->dpad + 8) * 0x1p-23;
+    for (int p = 0; p < TL_Q; p++) {
+        double qn = 0.0, qr = 0.0;
+        for (int j = 0; j < g->dim; j++) {
+            const float v = q[(size_t)p * g->dim + j];
+            uint32_t u;
+            memcpy(&u, &v, 4);
+            u = (u + 0xFFFu + ((u >> 13) & 1u)) & 0xFFFFE000u;  // (query_prep_row)
+            float t;
+            memcpy(&t, &u, 4);
+            qn += (double)v * v;
+            qr += ((double)v - t) * ((double)v - t);
+        }
+        double d[TL_K];  // distances, the row itself left out
+        int n = 0;
+        for (uint32_t i = 0; i < cnt[p]; i++)
+            if (hits[(size_t)p * TL_K + i].node != p * g->count / TL_Q)
+                d[n++] = hits[(size_t)p * TL_K + i].dist;
+        for (int i = 0; i < FvGpuIndex::TF32_KS; i++) {
+            const int k = 1 << i, S = std::min(std::max(4 * k, 16), n);
+            if (k > n) break;
+            const double A = d[S - 1];
+            const double E = tf32_scan_error(g->dpad, g->norm32_max, g->res32_max, qn, qr, A);
+            g->tf32_share[i] += (A - E) * (1.0 - c2) > d[k - 1] ? 1 : 0;
         }
     }
 }
 
-// Whether TF32 tells a table's rows apart at all: among a sample of rows, the
-// gap between the 4th and the 16th nearest (a superset holds 4k) against the
-// certificate's bound, for rows as queries. In the whole table the gap is
-// smaller, so where it does not do for half of them here (an offset far
-// larger than the spread), the certificate would send the batches to the
-// CUDA-core scan after a scan in vain: 1.79 ms instead of 1.62 for 100 such
-// queries of 400,000 x 200 rows, 0.70 instead of 0.56 for 33 of 200,000 x
-// 384. Only for rows beyond 128 dims, whose batches then go there at once; an
-// upload of 300 MB takes 31 ms with the look and without.
-cudaError_t tf32_look(FvGpuIndex *g) {
-    g->tf32_blind = false;
-    if (g->dpad <= 128 || g->row_amax >= 0.f || !tf32_supported(g)) return cudaSuccess;
-    const int m = (int)std::min<uint64_t>(g->count, 4096);
-    float *d = nullptr;
-    std::vector<float> h((size_t)TS_Q * (m + 2));
-    cudaError_t e = cudaMalloc(&d, h.size() * 4);
-    if (e != cudaSuccess) {  // no room to look
-        (void)cudaGetLastError();
-        return cudaSuccess;
-    }
-    tf32_sample_kernel<<<dim3((m + 7) / 8, TS_Q), 256, 0, g->stream>>>(
-        g->d_vecs, g->dpad, g->count, m, d, d + TS_Q * m, d + TS_Q * m + TS_Q);
-    e = cudaGetLastError();
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(h.data(), d, h.size() * 4, cudaMemcpyDeviceToHost, g->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    cudaFree(d);
-    if (e != cudaSuccess) return e;
-    int apart = 0;
-    for (int p = 0; p < TS_Q; p++) {
-        float *v = &h[(size_t)p * m];
-        // (NaN would break the ordering; such tables are refused by their norms)
-        for (int i = 0; i < m; i++)
-            if (!(v[i] == v[i])) v[i] = INFINITY;
-        std::nth_element(v, v + 15, v + m);
-        const double A = v[15];
-        std::nth_element(v, v + 3, v + 15);
-        const double E = tf32_scan_error(g->dpad, g->norm32_max, g->res32_max,
-                                         h[(size_t)TS_Q * m + p], h[(size_t)TS_Q * m + TS_Q + p], A);
-        apart += (A - E) * (1.0 - (g->dpad + 8) * 0x1p-23) > (double)v[3];
-    }
-    g->tf32_blind = apart < TS_Q / 2;
-    return cudaSuccess;
+// Whether an exact batch that can take the TF32 scan (superset S) should:
+// pass, the share of the rows its filters let through, thins the neighbours
+// out. Three of four queries looked up must come through, for the k's on
+// either side; and lists shorter than the superset lose its rows where they
+// are stored cluster by cluster (250,000 x 200 such rows, 40 queries, k 100:
+// all run again, 1.3 ms instead of 0.49).
+bool tf32_pays(const FvGpuIndex *g, uint32_t topb, int S, double pass) {
+    if (g->dpad <= 128) return true;
+    if (S > TC_MAX_LIST && !g->rows_mixed) return false;
+    if (S == (int)topb) return true;  // (distances are exact)
+    const double k = log2((double)topb / std::max(pass, 1e-9));
+    const int lo = std::min((int)k, FvGpuIndex::TF32_KS - 1);
+    const int hi = std::min(lo + (k > lo ? 1 : 0), FvGpuIndex::TF32_KS - 1);
+    return std::min(g->tf32_share[lo], g->tf32_share[hi]) >= TL_Q * 3 / 4;
 }
 
 // Rows of at most 512 f32 (beyond 128 the query tile streams with the rows),
