@@ -556,6 +556,15 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // (a table of few tiles is sampled more of: 60,000 rows, 512 queries,
     // S 800 took 1.08 ms without a bound, 0.36 seeded)
     while (!enough() && m < region) m++;
+    // Rows stored cluster by cluster: a query's nearest lie in a few chunks of
+    // a few tiles, of which the sample keeps one row a chunk, so its bound is
+    // loose and the pass admits cluster after cluster. Four times the tiles,
+    // then, and every chunk's best row kept (k 100, 200 queries of 300,000 x
+    // 32 BF16 rows: 1229 us a call without either, 490 with both; 715 behind
+    // heaps of a smaller sample's best keys. 2,160 batches over such tables:
+    // 1.36 times as fast as behind those heaps, 1.05 without either). Three
+    // times as many are 1 % slower, eight times as many the same.
+    if (!g->rows_mixed) m = std::min<uint64_t>(region, 4 * m);
     const bool estimated = rank_est < S;
     const int rank = std::min(S, rank_est);
     // Seeding pays from two tiles per CTA on, as long as the sample's chunk
@@ -746,13 +755,14 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         // the rank-th of 4 rank chunk minima lies about 1.15 times as deep as
         // the sample's own rank-th key. Lazy batches, which cannot tell a
         // chunk's best passing row, keep their share of the best keys; a
-        // full list's last key then bounds the S-th key if it holds S.
+        // full list's last key then bounds the S-th key if it holds S. Rows in
+        // clusters: as many chunks' best as a list takes.
         const int epiw = std::min(EPI, 2);
         const int chunks = (int)((m + epiw - 1) / epiw) * (TC_BN / R / 32);  // of a list
         const int lists = grow * (int)std::min<uint64_t>(m, epiw) * R;
         const int want = std::max(1, (4 * rank + lists - 1) / lists);
-        sa.KP = std::min(KP * EPI / epiw, (int)ceil(want / fill));
-        sa.seed_group = std::max(1, std::max((int)(chunks * fill) / want,
+        sa.KP = std::min(KP * EPI / epiw, g->rows_mixed ? (int)ceil(want / fill) : chunks);
+        sa.seed_group = std::max(1, std::max(g->rows_mixed ? (int)(chunks * fill) / want : 1,
                                              (chunks + sa.KP - 1) / sa.KP));
         sa.push_tau = sa.KP == S ? 1 : 0;
         sa.spill = 0;
