@@ -119,7 +119,9 @@ class Serialized:
 
 
 _record = struct.Struct("<8id").pack  # one NODE_DTYPE record
+_query = struct.Struct("<5iIQ").pack  # one QD_DTYPE record
 assert struct.calcsize("<8id") == NODE_DTYPE.itemsize
+assert struct.calcsize("<5iIQ") == QD_DTYPE.itemsize
 _KIND = {And: FV_NODE_AND, Or: FV_NODE_OR, Not: FV_NODE_NOT}
 
 
@@ -178,9 +180,13 @@ class BatchPred:
 def concat(preds: Sequence[Optional[Pred]], count: int,
            entries: Optional[Sequence[int]] = None) -> BatchPred:
     nq = len(preds)
-    qd = np.zeros(nq, QD_DTYPE)
-    qd["need_eval"] = 1
-    qd["total"] = count
+    if type(count) is int and 0 <= count < 2 ** 64:
+        qd = np.frombuffer(bytearray(_query(-1, 1, 0, 0, 0, 0, count) * nq), QD_DTYPE)
+    else:
+        qd = np.zeros(nq, QD_DTYPE)
+        qd["proot"] = -1
+        qd["need_eval"] = 1
+        qd["total"] = count
     if entries is not None:
         e = entries
         if isinstance(e, (list, tuple, range)):
@@ -197,8 +203,9 @@ def concat(preds: Sequence[Optional[Pred]], count: int,
         # a few filters: every query's slice in place (the gather below costs
         # 45 us whatever the batch)
         roots = [-1 if p is None else _flat(p, recs, children, invals) for p in preds]
-        qd["proot"] = roots
-        return BatchPred(qd, np.frombuffer(b"".join(recs), NODE_DTYPE).copy(),
+        if recs:
+            qd["proot"] = roots
+        return BatchPred(qd, np.frombuffer(bytearray(b"".join(recs)), NODE_DTYPE),
                          np.array(children, np.int32), np.array(invals, np.float64),
                          np.zeros(0, SPAN_DTYPE), np.zeros(0, np.uint64), np.zeros(nq, np.uint8),
                          np.array(roots, np.int32))
@@ -225,7 +232,6 @@ def concat(preds: Sequence[Optional[Pred]], count: int,
     end = np.asarray(size, np.int64)
     start, length = end[:-1][w], np.diff(end, axis=0)[w]
     base = np.cumsum(length, axis=0) - length  # where each query's slices begin
-    qd["proot"] = -1
     qd["proot"][has] = base[:, 0]
 
     def gather(a, k):
