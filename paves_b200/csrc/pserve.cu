@@ -682,8 +682,14 @@ bool sv_plan(PvServe *s, int nq, uint32_t topb, float q_amax, SvPlan &pl) {
     const uint64_t ntiles_all = (g->count + TC_BN - 1) / TC_BN;
     int grow = s->grid / pl.qtiles;
     if (grow < 1) grow = 1;
-    const uint64_t maxg = (ntiles_all + 3) / 4;
-    if ((uint64_t)grow > maxg) grow = (int)maxg;
+    // Seeded as the one-shot scan is; else a tile per CTA as far as they go,
+    // since lists fill without a bound (60 queries of 3,000 rows, k 16: 146 us
+    // on 6 CTAs of four tiles, 53 on 24 of one).
+    const uint64_t most = std::min<uint64_t>((uint64_t)grow, ntiles_all);
+    pl.seed = ntiles_all >= 2 * most &&
+              !tc_fills_little(KP, most * s->EPI * R, (double)g->count, nq, pl.qtiles);
+    if (pl.seed) grow = (int)std::min<uint64_t>((uint64_t)grow, (ntiles_all + 1) / 2);
+    else grow = (int)most;
     const uint64_t tpc = (ntiles_all + grow - 1) / grow;
     grow = (int)((ntiles_all + tpc - 1) / tpc);
     pl.grow = grow;
@@ -695,7 +701,6 @@ bool sv_plan(PvServe *s, int nq, uint32_t topb, float q_amax, SvPlan &pl) {
     pl.topb = (int)topb;
     const int nlists = grow * s->EPI * R;
     pl.dcap = (uint64_t)nlists * KP;
-    pl.seed = ntiles_all >= 8 * (uint64_t)grow;
     if (pl.seed) {
         const uint64_t region = ntiles_all / grow;
         const uint64_t m = std::min<uint64_t>(std::min<uint64_t>(8, region),

@@ -201,6 +201,7 @@ int brute_run_host(FvGpuIndex *g, int nq, const float *queries, const PredBatch 
 
 // ---- tensor-core scan (scan_tc.cu)
 bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns);
+bool tc_fills_little(int KP, uint64_t lists, double rows, int nq, int qtiles);
 int tc_superset(const FvGpuIndex *g, uint32_t topb, float q_amax);
 bool tc_supported(const FvGpuIndex *g);
 int tf32_superset(const FvGpuIndex *g, uint32_t topb, float q_amax);

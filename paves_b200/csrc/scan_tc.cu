@@ -411,6 +411,23 @@ static cudaError_t tc_launch(int kind, int grid, size_t smem, cudaStream_t st,
     return tc_launch_kind<TCK_BF16, EPI, WARM>(grid, smem, st, tmX, tmQ, a);
 }
 
+// Whether a query's `lists` of KP keys, one tile each of the `rows` that pass,
+// fill little without a bound: few kept keys for the merge and few admissions
+// per warp (of a list's p passing rows it keeps min(KP, p) and admits about
+// KP (1 + ln(p / KP))). The sample and its merge take 8 to 20 us; 1 to 7
+// queries of 50,000 to 100,000 rows with k of 1 or 2, or 1.6 % of the rows
+// passing, took 10 to 20 us more with them. (The lines, over 6,000 batches of
+// 1 to 300 queries: the merge takes what the sample saves from 5,000 kept keys
+// on, from 4,400 with 100 admissions a warp; the pass does from 150 admissions
+// on. Below, unseeded is 1 to 10 us faster; a little beyond, 2 to 10 slower.)
+bool tc_fills_little(int KP, uint64_t lists, double rows, int nq, int qtiles) {
+    const double p = rows / (double)lists;
+    const double kept = std::min<double>(KP, p);
+    const double admits = p <= KP ? p : KP * (1.0 + log(p / KP));
+    const double per_warp = admits * std::min(32, qtiles > 1 ? 32 : nq);
+    return per_warp <= 150.0 && kept * (double)lists + 8.0 * per_warp <= 5200.0;
+}
+
 // Launches query prep, the tensor-core scan, the per-query merge and the
 // exact re-rank. Inputs: f32 queries [nq][dpad] on the device, predicate
 // programs/bitmaps already built. tf32: scan the f32 rows themselves (the
@@ -572,22 +589,9 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // 2 to 4 times as long filling their lists behind no bound (100,000 BF16
     // rows, 73 queries: k 2, 25, 100 in 0.106, 0.158, 0.343 ms, seeded 0.043,
     // 0.044, 0.079). Without it every tile gets its own CTA.
-    // Nor does it pay when lists fill little without a bound: few kept keys
-    // for the merge and few admissions per warp (one tile per CTA, a list's
-    // passing rows p; it keeps min(S, p) and admits about S (1 + ln(p / S))).
-    // The sample and its merge take 8 to 20 us; 1 to 7 queries of 50,000 to
-    // 100,000 rows with k of 1 or 2, or 1.6 % of the rows passing, took 10 to
-    // 20 us more with them. (The lines, over 6,000 batches of 1 to 300
-    // queries: the merge takes what the sample saves from 5,000 kept keys on,
-    // from 4,400 with 100 admissions a warp; the pass does from 150
-    // admissions on. Below, unseeded is 1 to 10 us faster; a little beyond, 2
-    // to 10 slower.)
+    // Nor does it pay when lists fill little without a bound (tc_fills_little).
     const uint64_t ugrow = std::min<uint64_t>(std::max(1, g->sm_count / qtiles), ntiles_all);
-    const double p = pass * (double)nrows_scan / (double)(ugrow * EPI * R);
-    const double kept = std::min<double>(KP, p);
-    const double admits = p <= KP ? p : KP * (1.0 + log(p / KP));
-    const double per_warp = admits * std::min(32, qtiles > 1 ? 32 : nq);
-    const bool little = per_warp <= 150.0 && kept * ugrow * EPI * R + 8.0 * per_warp <= 5200.0;
+    const bool little = tc_fills_little(KP, ugrow * EPI * R, pass * (double)nrows_scan, nq, qtiles);
     const bool seed = g->tune_seed != 2 && !little && enough();
     if (!seed) {
         if (EPI == 3) {  // without a bound: lists that keep the best
