@@ -115,8 +115,8 @@ struct FvGpuIndex {
     float norm32_max = 0.f;     // largest of them
     float res32_max = 0.f;      // largest squared part of a row that TF32 drops
     // rows beyond 128 dims: of 16 rows looked up, how many TF32 would answer
-    // for k = 1, 2, 4 .. 128 (tf32_look)
-    static constexpr int TF32_KS = 8;
+    // for k = 1, 2, 4 .. 64 (tf32_look)
+    static constexpr int TF32_KS = 7;
     uint8_t tf32_share[TF32_KS] = {};
     // rows in an order unrelated to where they lie (order_kernel): a query's
     // nearest spread over the table, so short lists and samples of tiles serve

@@ -291,28 +291,68 @@ int tf32_superset(const FvGpuIndex *g, uint32_t topb, float q_amax) {
 // TF32 alone for k 100. So 16 rows are looked up at upload by the exact scan,
 // and for k of 1, 2, 4 .. the share of them is kept whose gap between the
 // k-th and the superset's last distance the certificate's bound would leave
-// open (about a millisecond beside 31 for 300 MB of rows).
-constexpr int TL_Q = 16, TL_K = 512;
+// open.
+constexpr int TL_Q = 16, TL_K = 257;  // (a row finds itself too)
 void tf32_look(FvGpuIndex *g, const float *vectors) {
     memset(g->tf32_share, 0, sizeof(g->tf32_share));
     if (g->dpad <= 128 || !tf32_supported(g) || !(g->norm32_max < 0x1p126f) ||
         tc_supported(g))  // (the low-precision rows are scanned)
         return;
-    std::vector<float> q((size_t)TL_Q * g->dim);
-    PredBatch none;
-    none.qprog.assign(TL_Q, -1);
-    for (int p = 0; p < TL_Q; p++)
-        memcpy(&q[(size_t)p * g->dim], vectors + (p * g->count / TL_Q) * (uint64_t)g->dim,
-               sizeof(float) * g->dim);
+    const uint64_t stride = g->count / TL_Q;  // row p * stride is query p
     std::vector<FvHit> hits((size_t)TL_Q * TL_K);
     std::vector<uint32_t> cnt(TL_Q);
-    std::vector<uint8_t> tr(TL_Q);
-    char err[256];
-    const int bad = brute_run_host(g, TL_Q, q.data(), none, TL_K, PV_MODE_SIMT, hits.data(),
-                                   cnt.data(), tr.data(), err, sizeof(err));
-    g->launches = 0;
-    g->last_kernel_ms = 0.f;
-    if (bad) {  // (no room, say: the CUDA-core scan it is)
+    // the exact scan on scratch of its own: [queries][bounds][keys][counts]
+    // [no program][filter count][hits][counts][flags]
+    ScanPlan pl;
+    if (!plan_scan_f32(g->count, g->dpad, TL_Q, TL_K, g->sm_count, pl)) return;
+    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t row = (size_t)g->dpad * 4;
+    const size_t o_tau = al(TL_Q * row), o_part = o_tau + al(TL_Q * 8);
+    const size_t o_pcnt = o_part + al((size_t)TL_Q * pl.grow * TL_K * 8);
+    const size_t o_prog = o_pcnt + al((size_t)TL_Q * pl.grow * 4), o_pop = o_prog + al(TL_Q * 4);
+    const size_t o_hit = o_pop + 256, o_cnt = o_hit + al(hits.size() * sizeof(FvHit));
+    const size_t o_tr = o_cnt + al(TL_Q * 4);
+    char *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, o_tr + al(TL_Q));
+    for (int p = 0; p < TL_Q && e == cudaSuccess; p++)
+        e = cudaMemcpyAsync(d + p * row, g->d_vecs + p * stride * (uint64_t)g->dpad, row,
+                            cudaMemcpyDeviceToDevice, g->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d + o_tau, 0xFF, TL_Q * 8, g->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d + o_prog, 0xFF, TL_Q * 4, g->stream);
+    if (e == cudaSuccess) {
+        ScanF32Args a;
+        a.vecs = g->d_vecs;
+        a.nrows = g->count;
+        a.dpad = g->dpad;
+        a.queries = (const float *)d;
+        a.nq = TL_Q;
+        a.bitmaps = nullptr;
+        a.bm_words = (g->count + 31) / 32;
+        a.qprog = (const int32_t *)(d + o_prog);
+        a.K = TL_K;
+        a.S = pl.S;
+        a.CB = pl.CB;
+        a.rows_per_cta = pl.rows_per_cta;
+        a.grow = pl.grow;
+        a.qtiles = pl.qtiles;
+        a.tau = (unsigned long long *)(d + o_tau);
+        a.part = (uint64_t *)(d + o_part);
+        a.part_cnt = (uint32_t *)(d + o_pcnt);
+        e = launch_scan_f32(a, pl, g->stream);
+        if (e == cudaSuccess)
+            e = launch_merge(a.part, a.part_cnt, pl.grow, TL_K, pl, a.tau, a.qprog,
+                             (const unsigned long long *)(d + o_pop), g->count, TL_Q,
+                             (FvHit *)(d + o_hit), (uint32_t *)(d + o_cnt), (uint8_t *)(d + o_tr),
+                             g->stream);
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(hits.data(), d + o_hit, hits.size() * sizeof(FvHit),
+                            cudaMemcpyDeviceToHost, g->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(cnt.data(), d + o_cnt, TL_Q * 4, cudaMemcpyDeviceToHost, g->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    cudaFree(d);
+    if (e != cudaSuccess) {  // (no room, say: the CUDA-core scan it is)
         (void)cudaGetLastError();
         return;
     }
@@ -320,7 +360,7 @@ void tf32_look(FvGpuIndex *g, const float *vectors) {
     for (int p = 0; p < TL_Q; p++) {
         double qn = 0.0, qr = 0.0;
         for (int j = 0; j < g->dim; j++) {
-            const float v = q[(size_t)p * g->dim + j];
+            const float v = vectors[p * stride * (uint64_t)g->dim + j];
             uint32_t u;
             memcpy(&u, &v, 4);
             u = (u + 0xFFFu + ((u >> 13) & 1u)) & 0xFFFFE000u;  // (query_prep_row)
@@ -331,8 +371,8 @@ void tf32_look(FvGpuIndex *g, const float *vectors) {
         }
         double d[TL_K];  // distances, the row itself left out
         int n = 0;
-        for (uint32_t i = 0; i < cnt[p]; i++)
-            if (hits[(size_t)p * TL_K + i].node != p * g->count / TL_Q)
+        for (uint32_t i = 0; i < std::min<uint32_t>(cnt[p], TL_K); i++)
+            if (hits[(size_t)p * TL_K + i].node != p * stride)
                 d[n++] = hits[(size_t)p * TL_K + i].dist;
         for (int i = 0; i < FvGpuIndex::TF32_KS; i++) {
             const int k = 1 << i, S = std::min(std::max(4 * k, 16), n);
