@@ -126,11 +126,19 @@ _KIND = {And: FV_NODE_AND, Or: FV_NODE_OR, Not: FV_NODE_NOT}
 
 
 def _i32(v) -> int:
-    if type(v) is int and -2 ** 31 <= v < 2 ** 31:
+    if type(v) is int:  # (packing refuses what is beyond 32 bits)
         return v
     cell = np.zeros(1, np.int32)
     cell[0] = v  # refuses and converts as an assignment to a record does
     return int(cell[0])
+
+
+def _flat_all(trees, recs: list, children: list, invals: list) -> list:
+    """_flat of each tree (None: -1), refusing what a record cannot hold."""
+    try:
+        return [-1 if p is None else _flat(p, recs, children, invals) for p in trees]
+    except struct.error as e:
+        raise OverflowError(str(e)) from None
 
 
 def _flat(n: Pred, recs: list, children: list, invals: list, at=(0, 0, 0)) -> int:
@@ -159,7 +167,7 @@ def _flat(n: Pred, recs: list, children: list, invals: list, at=(0, 0, 0)) -> in
 def serialize(p: Pred) -> Serialized:
     """One tree -> flat arrays, node 0 = root (pre-order)."""
     recs, children, invals = [], [], []
-    _flat(p, recs, children, invals)
+    _flat_all([p], recs, children, invals)
     return Serialized(np.frombuffer(b"".join(recs), NODE_DTYPE).copy(),
                       np.asarray(children, np.int32), np.asarray(invals, np.float64))
 
@@ -202,7 +210,7 @@ def concat(preds: Sequence[Optional[Pred]], count: int,
     if nq - sum(p is None for p in preds) <= 8:
         # a few filters: every query's slice in place (the gather below costs
         # 45 us whatever the batch)
-        roots = [-1 if p is None else _flat(p, recs, children, invals) for p in preds]
+        roots = _flat_all(preds, recs, children, invals)
         if recs:
             qd["proot"] = roots
         return BatchPred(qd, np.frombuffer(bytearray(b"".join(recs)), NODE_DTYPE),
@@ -213,16 +221,19 @@ def concat(preds: Sequence[Optional[Pred]], count: int,
     # its indexes moved to the slice's place
     place, size = {}, [(0, 0, 0)]  # tree -> its number; running ends of the three arrays
     which = []
-    for p in preds:
-        if p is None:
-            which.append(-1)
-            continue
-        i = place.get(id(p))
-        if i is None:
-            i = place[id(p)] = len(place)
-            _flat(p, recs, children, invals, size[-1])
-            size.append((len(recs), len(children), len(invals)))
-        which.append(i)
+    try:
+        for p in preds:
+            if p is None:
+                which.append(-1)
+                continue
+            i = place.get(id(p))
+            if i is None:
+                i = place[id(p)] = len(place)
+                _flat(p, recs, children, invals, size[-1])
+                size.append((len(recs), len(children), len(invals)))
+            which.append(i)
+    except struct.error as e:
+        raise OverflowError(str(e)) from None
     which = np.asarray(which, np.int64)
     has = which >= 0
     w = which[has]
