@@ -363,7 +363,7 @@ void tf32_look(FvGpuIndex *g, const float *vectors) {
             const float v = vectors[p * stride * (uint64_t)g->dim + j];
             uint32_t u;
             memcpy(&u, &v, 4);
-            u = (u + 0xFFFu + ((u >> 13) & 1u)) & 0xFFFFE000u;  // (query_prep_row)
+            u &= 0xFFFFE000u;
             float t;
             memcpy(&t, &u, 4);
             qn += (double)v * v;

@@ -766,12 +766,9 @@ __device__ __forceinline__ void query_prep_row(int qi, int lane, const float *__
             out[(size_t)qi * kelems + j] = *(unsigned char *)&b;
             r = float(b) * s;
         } else if (kind == TCK_TF32) {
-            // the nearest TF32 value (the MMA would drop the low bits, twice
-            // as far off); the norm is the exact row's
-            const uint32_t u = __float_as_uint(v);
-            float t = __uint_as_float((u + 0xFFFu + ((u >> 13) & 1u)) & 0xFFFFE000u);
-            if (!(fabsf(v) < 3e38f)) t = v;  // infinities and NaN as they are
-            ((float *)out)[(size_t)qi * kelems + j] = t;
+            // as it is: the MMA drops the low 13 mantissa bits, as the rows'
+            const float t = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
+            ((float *)out)[(size_t)qi * kelems + j] = v;
             r = v;
             res = fmaf(v - t, v - t, res);
         } else {
@@ -787,7 +784,7 @@ __device__ __forceinline__ void query_prep_row(int qi, int lane, const float *__
     }
     if (lane == 0) {
         qnorm[qi] = acc;
-        // fp8: the scale; TF32: what the rounding left of the query, squared
+        // fp8: the scale; TF32: what the MMA drops of the query, squared
         if (qscale) qscale[qi] = kind == TCK_TF32 ? res : s;
     }
 }
@@ -837,11 +834,11 @@ __device__ __forceinline__ void block_sort(uint64_t *keys, int n2) {
 //     (A - E) * (1 - c2) > Dk,
 // E bounding |scan distance - true distance| and c2 the relative error of
 // the f32 difference-form sum (the exact distance) against the true one:
-//   * the MMA sees t(x), the row without its low 13 mantissa bits, and q',
-//     the query rounded to TF32: x.q - t(x).q' = t(x).(q - q') + (x - t(x)).q,
-//     at most ||x|| ||q - q'|| + ||x - t(x)|| ||q|| (Cauchy-Schwarz, and
+//   * the MMA sees t(x) and t(q), row and query without their low 13
+//     mantissa bits: x.q - t(x).t(q) = t(x).(q - t(q)) + (x - t(x)).q, at
+//     most ||x|| ||q - t(q)|| + ||x - t(x)|| ||q|| (Cauchy-Schwarz, and
 //     ||t(x)|| <= ||x||), with ||x||^2 at most xnmax and ||x - t(x)||^2 at
-//     most xrmax over all rows: about 1.2 * 2^-10 ||x|| ||q|| on ordinary
+//     most xrmax over all rows: about 0.8 * 2^-10 ||x|| ||q|| on ordinary
 //     values, where 2^-9 per product is what any values allow (that bound
 //     left 3 of 64 queries of 1M real-valued rows uncertified, whose exact
 //     re-run took two thirds of the call);
@@ -849,7 +846,7 @@ __device__ __forceinline__ void block_sort(uint64_t *keys, int n2) {
 //     dim * 2^-22 of sum |x_i q_i| <= ||x|| ||q||;
 //   * the f32 norms (dim terms) and the two roundings of ||x||^2 + ||q||^2
 //     - 2 q.x stay within c2 = (dim + 8) * 2^-23 of the values they round.
-// E = 2 (1 + 2^-6) (||x|| ||q - q'|| + ||x - t(x)|| ||q||) + dim 2^-20 ||x|| ||q||
+// E = 2 (1 + 2^-6) (||x|| ||q - t(q)|| + ||x - t(x)|| ||q||) + dim 2^-20 ||x|| ||q||
 //     + c2 (xnmax + ||q||^2 + A): the first term's margin covers the f32
 // roundings of the norms themselves, the second is twice what the analysis
 // needs. All of this holds while xnmax + ||q||^2 stays inside f32's range;
@@ -869,7 +866,7 @@ __host__ __device__ inline double tf32_scan_error(int dim, double xm, double xr,
 
 struct RerankCert {
     const float *qnorm = nullptr;  // [nq] ||q||^2 (f32)
-    const float *qres = nullptr;   // [nq] ||q - q'||^2 (f32)
+    const float *qres = nullptr;   // [nq] ||q - t(q)||^2 (f32)
     float xnmax = 0.f;             // max ||x||^2 over the rows (f32 norms)
     float xrmax = 0.f;             // max ||x - t(x)||^2 over the rows
     int dim = 0;
