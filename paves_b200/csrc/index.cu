@@ -71,8 +71,11 @@ __global__ void norm32_kernel(const float *__restrict__ src, int dpad, uint64_t 
     }
     if (lane == 0) {
         norm[row] = acc;
-        atomicMax(nmax, __float_as_uint(acc));
-        atomicMax(nmax + 1, __float_as_uint(res));
+        // (a maximum once reached is only read: an atomic per row and word took
+        // 1.33 ms for 1M x 128 rows, 0.69 with one word, this 0.55)
+        const unsigned a = __float_as_uint(acc), r = __float_as_uint(res);
+        if (a > *(volatile unsigned *)nmax) atomicMax(nmax, a);
+        if (r > *(volatile unsigned *)(nmax + 1)) atomicMax(nmax + 1, r);
     }
 }
 
