@@ -418,18 +418,11 @@ static size_t tc_smem(int kblocks, int NS, int KP, int EPI) {
     return tc_smem_bytes(kblocks, NS, KP, EPI, tc_qstream(kblocks));
 }
 
-// Three groups' lists hold every nearest row of the query that a list meets:
-// where rows are stored cluster by cluster, only whole lists do.
-static bool tc_three_groups(const FvGpuIndex *g, int S, int kblocks) {
-    return g->rows_mixed || S <= tc_list_cap(3, kblocks);
-}
-
 bool tc_shape_fits(const FvGpuIndex *g, uint32_t topb, int epi, int ns) {
     if (!tc_supported(g) || epi < 1 || epi > 3 || ns < 2 || ns > TC_MAX_STAGES) return false;
     const int S = tc_superset(g, topb, -1.f);
     if (!S) return false;
     const int kblocks = g->kpad * (g->precision == FV_GPU_PREC_FP8 ? 1 : 2) / TC_KB_BYTES;
-    if (epi == 3 && !tc_three_groups(g, S, kblocks)) return false;
     const int KP = std::min(S, tc_list_cap(epi, kblocks));
     return tc_smem(kblocks, ns, KP, epi) <= 227 * 1024;
 }
@@ -538,11 +531,14 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
             NS = 2;
         }
     };
-    // (and a run that spills may be full, which flags the query)
-    const bool three = S <= tc_list_cap(3, kblocks) || (redo && tc_three_groups(g, S, kblocks));
+    // (three groups' lists hold every nearest row of the query that a list
+    // meets: where rows are stored cluster by cluster, only whole lists do;
+    // and a run that spills may be full, which flags the query)
+    const bool whole3 = S <= tc_list_cap(3, kblocks);
+    const bool three = whole3 || (g->rows_mixed && redo);
     shape(kblocks * TC_KB_BYTES * R >= 1024 ? 1 : R == 1 && three ? 3 : 2);
     if (g->tune_epi || g->tune_ns) {  // a tuned shape, if it fits
-        const int e = std::min(g->tune_epi ? g->tune_epi : EPI, three ? 3 : 2);
+        const int e = std::min(g->tune_epi ? g->tune_epi : EPI, whole3 || redo ? 3 : 2);
         const int n = g->tune_ns ? g->tune_ns : NS;
         if (e >= 1 && n >= 2 && n <= TC_MAX_STAGES &&
             tc_smem(kblocks, n, std::min(S, tc_list_cap(e, kblocks)), e) <= smem_cap) {
@@ -621,7 +617,10 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // heaps of a smaller sample's best keys. 2,160 batches over such tables:
     // 1.36 times as fast as behind those heaps, 1.05 without either). Three
     // times as many are 1 % slower, eight times as many the same.
-    if (!g->rows_mixed) m = std::min<uint64_t>(region, 4 * m);
+    // (Batches that may test their filters lazily cannot tell a chunk's best
+    // passing row: twice their share of the best keys.)
+    const bool clusters = !g->rows_mixed && !lz;
+    if (clusters) m = std::min<uint64_t>(region, 4 * m);
     const bool estimated = rank_est < S;
     const int rank = std::min(S, rank_est);
     // Seeding pays from two tiles per CTA on, as long as the sample's chunk
@@ -805,8 +804,9 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         const int chunks = (int)((m + epiw - 1) / epiw) * (TC_BN / R / 32);  // of a list
         const int lists = grow * (int)std::min<uint64_t>(m, epiw) * R;
         const int want = std::max(1, (4 * rank + lists - 1) / lists);
-        sa.KP = std::min(KP * EPI / epiw, g->rows_mixed ? (int)ceil(want / fill) : chunks);
-        sa.seed_group = std::max(1, std::max(g->rows_mixed ? (int)(chunks * fill) / want : 1,
+        sa.KP = std::min(KP * EPI / epiw, clusters ? chunks
+                                          : (int)ceil(want / fill) * (g->rows_mixed ? 1 : 2));
+        sa.seed_group = std::max(1, std::max(clusters ? 1 : (int)(chunks * fill) / want,
                                              (chunks + sa.KP - 1) / sa.KP));
         sa.push_tau = sa.KP == S ? 1 : 0;
         sa.spill = 0;
