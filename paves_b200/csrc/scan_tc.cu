@@ -137,8 +137,8 @@ rerank_kernel(const float *__restrict__ vecs, int dpad, const float *__restrict_
     rerank_query<256, ORDER>(blockIdx.x, keys, vecs, dpad, queries, cand, cand_cnt, S, topb, qprog, popcnt,
                       nrows, out, out_cnt, trunc, cert, &again);
     if (ORDER == RR_LANES8 && again)
-        rerank_query<256, RR_WARP>(blockIdx.x, keys, vecs, dpad, queries, cand, cand_cnt, S, topb,
-                                   qprog, popcnt, nrows, out, out_cnt, trunc, cert);
+        rerank_again<256>(blockIdx.x, keys, vecs, dpad, queries, (int)min(cand_cnt[blockIdx.x], (uint32_t)S),
+                          (int)topb, out);
 }
 
 // ---------------------------------------------------------------- merge

@@ -877,11 +877,11 @@ struct RerankCert {
 // candidate (RR_LANES8); queries that only this bound separates, and not the
 // one that any values allow (1.25 * 2^-8 ||x|| ||q||), are summed once more
 // in the order of the CUDA-core scan that answered them under that one
-// (RR_WARP, whose shorter chains round less). Wider rows reach the re-rank only on batches that
-// the CUDA-core scans answered before, and keep those kernels' sums bit for
-// bit, so near ties order as they do there: the warp's of scan_f32.cu and of
-// a selective filter's listed rows (RR_WARP), or the thread's of scan_f32t.cu,
-// even and odd dims apart (RR_THREAD).
+// (RR_WARP). Wider rows reach the re-rank only on batches that the CUDA-core
+// scans answered before, and keep those kernels' sums bit for bit, so near
+// ties order as they do there: the warp's of scan_f32.cu and of a selective
+// filter's listed rows (RR_WARP), or the thread's of scan_f32t.cu, even and
+// odd dims apart (RR_THREAD).
 constexpr int RR_LANES8 = 0, RR_WARP = 1, RR_THREAD = 2;
 
 // One query's re-rank by the block's NT threads (8 lanes per candidate,
@@ -1031,12 +1031,80 @@ __device__ __forceinline__ void rerank_query(int q, uint64_t *keys, const float 
                 const double E = tf32_scan_error(cert.dim, xm, xr, qn, qr, A);
                 ok = ok && (A - E) * (1.0 - c2) > Dk;
                 const double E1 = 1.25 * 0x1p-8 * sqrt(qn * xm) * (1.0 + c2) + c2 * (xm + qn + A);
-                if (again) *again = ok && !((A - E1) * (1.0 - c2) > Dk);
+                // (its last distance in the other order is within 4 c2 of Dk)
+                if (again && ok && !((A - E1) * (1.0 - c2) > Dk)) {
+                    ok = (A - E) * (1.0 - c2) > Dk * (1.0 + 4.0 * c2);
+                    *again = ok;
+                }
             }
             if (!ok) cert.unc[q] = 1;
         }
     }
     __syncthreads();
+}
+
+// A full answer once more in the warp's order (RR_WARP). keys: what
+// rerank_query left, n candidates ascending. Each sum is within (dim + 8)
+// 2^-23 of the distance, so the topb rows of this order are among those whose
+// first sum is at most four such steps (six are taken) beyond the topb-th:
+// little more than topb rows are summed, and sorted, again.
+template <int NT>
+__device__ __forceinline__ void rerank_again(int q, uint64_t *keys, const float *__restrict__ vecs,
+                                             int dpad, const float *__restrict__ queries, int n,
+                                             int topb, FvHit *__restrict__ out) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float *qv = queries + (size_t)q * dpad;
+    const float last = key_dist(keys[topb - 1]);
+    const float lim = last * (1.f + 6.f * (float)(dpad + 8) * 0x1p-23f);
+    int m = topb;
+    while (m < n && key_dist(keys[m]) <= lim) m++;
+    __syncthreads();  // every thread has read the keys
+    constexpr int U = 4;
+    for (int base = warp * U; base < m; base += NT / 32 * U) {
+        float s[U];
+        uint32_t row[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            row[u] = key_row(keys[min(base + u, m - 1)]);
+            s[u] = 0.f;
+        }
+        for (int k = lane * 4; k < dpad; k += 128) {
+            const float4 w = __ldg((const float4 *)(qv + k));
+            float4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                v[u] = __ldg((const float4 *)(vecs + (size_t)row[u] * dpad + k));
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const float d0 = v[u].x - w.x, d1 = v[u].y - w.y, d2 = v[u].z - w.z,
+                            d3 = v[u].w - w.w;
+                s[u] = fmaf(d0, d0, s[u]);
+                s[u] = fmaf(d1, d1, s[u]);
+                s[u] = fmaf(d2, d2, s[u]);
+                s[u] = fmaf(d3, d3, s[u]);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < U; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+        __syncwarp();  // (places past m re-read this warp's own last row)
+        if (lane == 0)
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (base + u < m) keys[base + u] = make_key(s[u], row[u]);
+    }
+    int n2 = 32;
+    while (n2 < m) n2 <<= 1;
+    for (int i = m + tid; i < n2; i += NT) keys[i] = KEY_MAX;
+    __syncthreads();
+    block_sort(keys, n2);
+    for (int i = tid; i < topb; i += NT) {
+        FvHit h;
+        h.node = key_row(keys[i]);
+        h.dist = key_dist(keys[i]);
+        out[(size_t)q * topb + i] = h;
+    }
 }
 
 constexpr int DM_THREADS = 512;
