@@ -449,7 +449,10 @@ int pv_tc_timeout(FvGpuIndex *g, uint64_t ns);
  * topb itself on integer rows, where the distances are exact) re-ranked in
  * FP32, and each query's answer certified by an error bound of the scan
  * distances; a query the bound cannot separate is re-run on the CUDA-core
- * scan. on = 0 keeps every exact batch on the CUDA cores. -1: bad value.
+ * scan. Tables with a value whose square leaves f32 stay on the CUDA cores,
+ * and so do rows beyond 128 dims where a look at upload says that the bound
+ * would not do for this topb, and in prepared batches (which do not re-run).
+ * on = 0 keeps every exact batch on the CUDA cores. -1: bad value.
  * pv_last_exact_tc: 1 if the last brute batch on g took the tensor cores. */
 int pv_exact_tc(FvGpuIndex *g, int on);
 int pv_last_exact_tc(const FvGpuIndex *g);
