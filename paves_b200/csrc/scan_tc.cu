@@ -592,6 +592,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     // and not for up to 64 keys, which a certain bound costs little (512
     // queries, 500,000 rows, S 40: 0.180 against 0.170 ms).
     int rank_est = S;
+    double share = 1.0;
     auto enough = [&]() {  // chunk minima for the bound's rank, twice over
         // A compacted set with room to spare: the strides reach past the
         // prefix of tiles that exist, so the sample holds every step-th of
@@ -599,7 +600,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         // FP8 rows, k 75, a bound below their superset when half of the room
         // was used; all were run twice). Right down to half of the expected
         // tiles.
-        const double share =
+        share =
             full ? std::min(1.0, (double)m * grow * TC_BN / (double)nrows_scan)
                  : std::min(1.0, 1.0 / (double)std::max<uint64_t>(1, region / m) +
                                      2.0 / (fill * (double)region));
@@ -642,6 +643,26 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
         tpc = split(ntiles_all);
     }
 
+    // A run that spills has to hold what its query's bound lets through, and
+    // the sample of a large table leaves that far above S: room for 2.5 times
+    // rank / share (chunk minima lie 1.15 times as deep, and six deviations of
+    // 64 keys are another 1.75), or whole lists where that is more than 1 GB.
+    // With 64 keys a list and no more, every query of large batches over large
+    // tables was run again: 1024 queries of 4M x 64 rows, k 40 61 ms (whole
+    // lists 5.0 before there were short ones, now 2.1), of 10M FP8 rows, k 10
+    // 150 ms (12.5, now 5.5), graphs of 1M rows 11.7 s (3.2, now 1.0). Whole
+    // lists from 3,000 keys on instead take 1.1 to 2.1 times as long.
+    uint64_t run_keys = (uint64_t)grow * EPI * R * std::min(S, TC_MAX_LIST);
+    if (seed && certify && EPI == 3) {
+        run_keys = std::max(run_keys, (uint64_t)(2.5 * rank / share) +
+                                          (uint64_t)grow * EPI * R * KP);
+        if ((uint64_t)nq * run_keys * 8 > 1ull << 30) {
+            shape(2);
+            KP = std::min(S, tc_list_cap(EPI, kblocks));
+            certify = KP < S;
+        }
+    }
+
     ScanScratch &s = g->scan;
     const size_t qbytes = (size_t)nqpad * kelems * esz;
     const size_t off_qn = (qbytes + 255) & ~(size_t)255;
@@ -659,7 +680,7 @@ int launch_scan_tc(FvGpuIndex *g, int nq, float q_amax, const float *d_q,
     const int nlists = grow * EPI * R;  // lists per query
     const bool spill = seed && certify && EPI == 3;
     // a query's dense run at most
-    const uint64_t dcap = (uint64_t)nlists * (spill ? std::min(S, TC_MAX_LIST) : KP);
+    const uint64_t dcap = spill ? run_keys : (uint64_t)nlists * KP;
     PV_CUDA_OK(s.part.ensure((size_t)nq * dcap * 8), errbuf, errlen);
     // [dcnt u32 x nq][fullmin u64 x nq]
     const size_t off_fm = ((size_t)nq * 4 + 255) & ~(size_t)255;
